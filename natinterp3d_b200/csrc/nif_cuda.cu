@@ -57,7 +57,14 @@ constexpr int LARGE_G = 32;
 using LargeWS = Workspace<16384, 4096, 8192, 2048, 8192, LARGE_G, uint16_t, int16_t>;
 constexpr int ROW_STAGE = 24;         // get_weights: entries staged per row (mean about 15.5)
 using CavWS = CavWorkspace<256, 96, FAST_G, uint8_t, int8_t>;
-using VolWS = VolWorkspace<REC_CAV, 128, 64, 128, FAST_G>;
+#ifndef NIF_VOL_BF
+#define NIF_VOL_BF 42
+#endif
+using VolWS = VolWorkspace<REC_CAV, NIF_VOL_BF, 64, FAST_G>;
+// the rows VolWS does not hold: a record's tets have at most 2 * 48 + 2
+// boundary faces (each joins the others through a face)
+using GenWS = VolWorkspace<REC_CAV, 98, 64, FAST_G>;
+constexpr int GEN_OCC = 3;
 // rows a record buffer holds: calls run in chunks of these (measured: 256k-
 // and 64k-row chunks, whose records stay in L2, ran 6 % and 25 % slower on
 // 10M queries -- the launches' tails cost more than the DRAM round trip)
@@ -67,8 +74,10 @@ using VolWS = VolWorkspace<REC_CAV, 128, 64, 128, FAST_G>;
 constexpr int REC_CHUNK = NIF_REC_CHUNK;
 // resident blocks per SM of the split kernels (0: the mesh's blocks_per_sm).
 // The cavity kernel is issue-bound and fits 10 blocks in 48 registers (1-2 %
-// faster than 8 on 10M queries); the volume kernel spills at 10 (16 % slower)
-// and follows the mesh's setting.
+// faster than 8 on 10M queries).  The volume kernel takes 6 or, for the
+// setting of 8, 7: with 72 registers a thread it barely spills, and a warp's
+// workspace holds 42 boundary faces (2M queries, 200k keys: 7.1 ms at 7
+// blocks, 7.4 ms at 6, 10.1 ms at 8 with 64 registers and 34 faces).
 #ifndef NIF_CAV_OCC
 #define NIF_CAV_OCC 10
 #endif
@@ -96,6 +105,8 @@ struct DevSummary {
     int large_count;  // rows queued for the large kernel
     int refill_count; // get_weights: fast-kernel rows longer than ROW_STAGE
     int wide_count;   // split rows whose cavity exceeds a record (the fused kernel takes them)
+    int general_count; // rows of the current chunk for k_rows_general
+    int reserved;
     // predicate evaluations the filter could not certify / whose decision the
     // exact sign changes (PRED_AUDIT and PRED_EXACT meshes)
     unsigned long long orient_unc, orient_flip, insphere_unc, insphere_flip;
@@ -178,6 +189,19 @@ __global__ void k_prep_geometry(MeshView M, uint32_t *__restrict__ tinfo, d4 *__
         fcc[4 * (size_t)t + 1] = d4{f1.x, f1.y, f1.z, 0.0};
         fcc[4 * (size_t)t + 2] = d4{f2.x, f2.y, f2.z, 0.0};
         fcc[4 * (size_t)t + 3] = d4{f3.x, f3.y, f3.z, 0.0};
+    }
+}
+
+// every corner term of every tet, one thread a (tet, mask): 32 bytes each,
+// 512 a tet in one piece
+__global__ void k_prep_corner(MeshView M, d4 *__restrict__ corner) {
+    const int64_t n = 16 * (int64_t)M.nt;
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
+         i += (int64_t)gridDim.x * blockDim.x) {
+        const int t = (int)(i >> 4);
+        const unsigned m = (unsigned)i & 15u;
+        corner[i] = d4{corner_term(M, t, m, 0), corner_term(M, t, m, 1), corner_term(M, t, m, 2),
+                       corner_term(M, t, m, 3)};
     }
 }
 
@@ -548,6 +572,28 @@ struct StageSink {
             if (!large && !stage) refill[atomicAdd(&sum->refill_count, 1)] = (int)i;
         }
     }
+    // the same from a split row's lanes
+    template <int G, class W, int IDS>
+    __device__ __forceinline__ void emit_lanes(int64_t i, W &ws, const Grp<G> &g, RowInfo &r,
+                                               RowLanes<IDS> &L) {
+        split_weights<G>(ws, g, r, L);
+        const bool stage = r.nnb <= ROW_STAGE;
+        if (stage) {
+            const int64_t o = i * ROW_STAGE;
+#pragma unroll
+            for (int k = 0; k < IDS; k++)
+                if (L.col[k] < r.nnb) {
+                    cols[o + L.col[k]] = L.vid[k];
+                    vals[o + L.col[k]] = L.a[k];
+                }
+        }
+        if (g.lane == 0) {
+            total[i] = (r.nnb > 0) ? r.total : 0.0;
+            cnt[i] = r.nnb;
+            staged[i] = stage ? 1 : 0;
+            if (!stage) refill[atomicAdd(&sum->refill_count, 1)] = (int)i;
+        }
+    }
     __device__ __forceinline__ void empty(int64_t i, int lane) {
         if (lane == 0) {
             cnt[i] = 0;
@@ -606,6 +652,8 @@ struct InterpSink {
     int D;
     static constexpr bool FULL = true;
     static constexpr bool SORTED = sizeof(WT) == 4;
+    static constexpr int STAGED_D = 8;  // columns summed from staged products
+    static constexpr int LANE_D = 4;    // of these, the columns a lane reads ahead
 
     template <int G, class W>
     __device__ __forceinline__ void emit(int64_t i, int nnb, W &ws, const Grp<G> &g, bool,
@@ -615,37 +663,132 @@ struct InterpSink {
             for (int d = g.lane; d < D; d += G) o[d] = (CT)0;
             return;
         }
-        // the cavity-search scratch is free now: stage the products there
-        double *buf = reinterpret_cast<double *>(&ws.u);
-        constexpr int BUFN = (int)(sizeof(ws.u) / sizeof(double));
         if (SORTED) {
-            // position of each neighbour in ascending column order (columns are distinct)
+            // the neighbours in ascending column order (columns are distinct)
             for (int s = g.lane; s < nnb; s += G) {
                 const int v = ws.nbr_vid[s];
                 int r = 0;
                 for (int t = 0; t < nnb; t++) r += ws.nbr_vid[t] < v;
-                ws.vh_first[s] = r;
+                ws.vh_first[r] = s;
             }
         }
-        const int dc = max(1, min(D, BUFN / nnb));
-        for (int d0 = 0; d0 < D; d0 += dc) {
-            const int nd = min(dc, D - d0);
-            g.sync();
-            for (int k = g.lane; k < nnb * nd; k += G) {
-                const int s = k / nd, d = k - s * nd;
+        // the cavity-search scratch is free now: stage the products there
+        double *buf = reinterpret_cast<double *>(&ws.u);
+        constexpr int BUFN = (int)(sizeof(ws.u) / sizeof(double));
+        if (D <= STAGED_D && nnb * D <= BUFN) {
+            // few columns: a lane per neighbour forms its products, then a lane
+            // per column adds them in order
+            for (int s = g.lane; s < nnb; s += G) {
                 const CT w = (CT)(WT)ws.acc[s];
-                const CT x = (CT)values[(int64_t)ws.nbr_vid[s] * D + d0 + d];
-                const int row = SORTED ? ws.vh_first[s] : s;
-                buf[row * nd + d] = (double)Arith<CT>::mul(w, x);
+                const VT *x = values + (int64_t)ws.nbr_vid[s] * D;
+#pragma unroll 1
+                for (int d = 0; d < D; d++) buf[s * D + d] = (double)Arith<CT>::mul(w, (CT)x[d]);
             }
             g.sync();
-            for (int d = g.lane; d < nd; d += G) {
+            if (g.lane < D) {
                 CT acc = (CT)0;
-                for (int s = 0; s < nnb; s++) acc = Arith<CT>::add(acc, (CT)buf[s * nd + d]);
-                o[d0 + d] = acc;
+                for (int s = 0; s < nnb; s++)
+                    acc = Arith<CT>::add(acc, (CT)buf[(SORTED ? ws.vh_first[s] : s) * D + g.lane]);
+                o[g.lane] = acc;
+            }
+        } else {
+            // a lane per column: the values of one neighbour are one coalesced read
+            if (SORTED) g.sync();
+            for (int d = g.lane; d < D; d += G) {
+                CT acc = (CT)0;
+#pragma unroll 4
+                for (int s = 0; s < nnb; s++) {
+                    const int t = SORTED ? ws.vh_first[s] : s;
+                    const CT w = (CT)(WT)ws.acc[t];
+                    acc = Arith<CT>::add(acc, Arith<CT>::mul(w, (CT)values[(int64_t)ws.nbr_vid[t] * D + d]));
+                }
+                o[d] = acc;
             }
         }
         g.sync();
+    }
+
+    // The same from a split row's lanes: lane l's neighbour, whose values are
+    // read before the normalisation's chain of additions.
+    template <int G, class W, int IDS>
+    __device__ __forceinline__ void emit_lanes(int64_t i, W &ws, const Grp<G> &g, RowInfo &r,
+                                               RowLanes<IDS> &L) {
+        CT *o = out + i * (int64_t)D;
+        const bool few = D <= STAGED_D;
+        VT x[IDS][LANE_D];
+#pragma unroll
+        for (int k = 0; k < IDS; k++)
+#pragma unroll
+            for (int d = 0; d < LANE_D; d++)
+                if (d < D && few && L.col[k] < r.nnb) x[k][d] = values[(int64_t)L.vid[k] * D + d];
+        split_weights<G>(ws, g, r, L);
+        const int nnb = r.nnb;
+        if (nnb == 0) {
+            for (int d = g.lane; d < D; d += G) o[d] = (CT)0;
+            return;
+        }
+        // a neighbour's place in the sum: its column, or the number of smaller vertices
+        int at[IDS];
+#pragma unroll
+        for (int k = 0; k < IDS; k++) {
+            at[k] = L.col[k];
+            if (SORTED && L.col[k] < nnb) at[k] = 0;
+        }
+        if (SORTED) {
+            // neighbour 32 k + l is lane l's k-th, except in a coincident row
+#pragma unroll
+            for (int k = 0; k < IDS; k++) {
+                unsigned m = g.ballot(L.col[k] < nnb);
+                while (m) {
+                    const int v = g.shfl(L.vid[k], __ffs(m) - 1);
+                    m &= m - 1u;
+#pragma unroll
+                    for (int j = 0; j < IDS; j++)
+                        if (v < L.vid[j]) at[j]++;
+                }
+            }
+        }
+        if (few) {
+            double *buf = reinterpret_cast<double *>(&ws.u);
+            static_assert(W::NBR * STAGED_D * sizeof(double) <= sizeof(ws.u), "the products of a row");
+#pragma unroll
+            for (int k = 0; k < IDS; k++)
+                if (L.col[k] < nnb) {
+                    const CT w = (CT)(WT)L.a[k];
+#pragma unroll
+                    for (int d = 0; d < LANE_D; d++)
+                        if (d < D) buf[at[k] * D + d] = (double)Arith<CT>::mul(w, (CT)x[k][d]);
+#pragma unroll 1
+                    for (int d = LANE_D; d < D; d++)
+                        buf[at[k] * D + d] =
+                            (double)Arith<CT>::mul(w, (CT)values[(int64_t)L.vid[k] * D + d]);
+                }
+            g.sync();
+            if (g.lane < D) {
+                CT acc = (CT)0;
+#pragma unroll 4
+                for (int s = 0; s < nnb; s++) acc = Arith<CT>::add(acc, (CT)buf[s * D + g.lane]);
+                o[g.lane] = acc;
+            }
+        } else {
+            g.sync();
+#pragma unroll
+            for (int k = 0; k < IDS; k++)
+                if (L.col[k] < nnb) {
+                    ws.acc[at[k]] = L.a[k];
+                    ws.nbr_vid[at[k]] = L.vid[k];
+                }
+            g.sync();
+#pragma unroll 1
+            for (int d = g.lane; d < D; d += G) {
+                CT acc = (CT)0;
+#pragma unroll 4
+                for (int s = 0; s < nnb; s++)
+                    acc = Arith<CT>::add(acc, Arith<CT>::mul((CT)(WT)ws.acc[s],
+                                                             (CT)values[(int64_t)ws.nbr_vid[s] * D + d]));
+                o[d] = acc;
+            }
+        }
     }
     __device__ __forceinline__ void empty(int64_t i, int lane) {
         CT *o = out + i * (int64_t)D;
@@ -678,6 +821,12 @@ struct GradSink {
     QT *__restrict__ gq;             // [M][3]
     int D;
 
+    template <int G, class W, int IDS>
+    __device__ __forceinline__ void emit_lanes(int64_t i, W &ws, const Grp<G> &g, RowInfo &r,
+                                               RowLanes<IDS> &, const MeshView &M, dv3 q) {
+        emit<G>(i, r.nnb, ws, g, false, M, q, r);
+    }
+
     template <int G, class W>
     __device__ __forceinline__ void emit(int64_t i, int nnb, W &ws, const Grp<G> &g, bool,
                                          const MeshView &M, dv3 q, const RowInfo &r) {
@@ -702,23 +851,35 @@ struct GradSink {
             for (int s = g.lane; s < nnb; s += G) ck[s] = (ck[s] - gbar) * inv_total;
             g.sync();
             for (int b = g.lane; b < r.nbf; b += G) {
-                const int cf = ws.bface[b];
-                const int f = cf & 3;
-                const int tt = ws.cav_tet[cf >> 2];
-                const int4 p = M.tv[tt];
-                const int va = comp(p, face_vslot(f, 0));
-                const int vb = comp(p, face_vslot(f, 1));
-                const int vc = comp(p, face_vslot(f, 2));
-                const int sa = va < M.n ? neighbour_slot(ws, va) : -1;
-                const int sb = vb < M.n ? neighbour_slot(ws, vb) : -1;
-                const int sc = vc < M.n ? neighbour_slot(ws, vc) : -1;
+                dv3 pa, pb, pc;
+                int sa, sb, sc, ffi;
+                if constexpr (W::SPLIT) {
+                    const unsigned ids = ws.fid[b];
+                    sa = ids & 0xff, sb = (ids >> 8) & 0xff, sc = ids >> 16;
+                    pa = sload(ws.pos[sa]), pb = sload(ws.pos[sb]), pc = sload(ws.pos[sc]);
+                    sa = sa < nnb ? ws.start[sa] : -1, sb = sb < nnb ? ws.start[sb] : -1,
+                    sc = sc < nnb ? ws.start[sc] : -1;
+                    ffi = ws.bff[b];
+                } else {
+                    const int cf = ws.bface[b];
+                    const int f = cf & 3;
+                    const int tt = ws.cav_tet[cf >> 2];
+                    const int4 p = M.tv[tt];
+                    const int va = comp(p, face_vslot(f, 0));
+                    const int vb = comp(p, face_vslot(f, 1));
+                    const int vc = comp(p, face_vslot(f, 2));
+                    sa = va < M.n ? neighbour_slot(ws, va) : -1;
+                    sb = vb < M.n ? neighbour_slot(ws, vb) : -1;
+                    sc = vc < M.n ? neighbour_slot(ws, vc) : -1;
+                    pa = vload(M, va), pb = vload(M, vb), pc = vload(M, vc);
+                    ffi = 4 * tt + (3 - f);
+                }
                 // virtual terms enter the stolen volumes with a minus sign
                 const double c0 = sa >= 0 ? -ck[sa] : 0.0;
                 const double c1 = sb >= 0 ? -ck[sb] : 0.0;
                 const double c2 = sc >= 0 ? -ck[sc] : 0.0;
                 if (c0 == 0.0 && c1 == 0.0 && c2 == 0.0) continue;
-                const dv3 gf = virtual_face_grad(q, vload(M, va), vload(M, vb), vload(M, vc),
-                                                 cload(&M.fcc[4 * (size_t)tt + (3 - f)]), c0, c1, c2);
+                const dv3 gf = virtual_face_grad(q, pa, pb, pc, cload(&M.fcc[ffi]), c0, c1, c2);
                 gx += gf.x;
                 gy += gf.y;
                 gz += gf.z;
@@ -1192,12 +1353,15 @@ __global__ void __launch_bounds__(FAST_BLOCK, OCC)
 // natinterp3d's LIFO visiting order (natural_insertionfree.c:486-551,
 // replayed on the cavity; its non-cavity tets are leaves and do not change
 // the order) and which of its faces take a neighbour's face-cache copy;
-// k_rows_volume derives the fcc[] indices from these.  One warp takes 32
-// consecutive rows: the lanes load the rows' neighbour bytes into shared
-// memory entry by entry, each lane replays one row there, and the lanes
-// write the positions back entry by entry.  Rows without a cavity record
-// are left alone.
+// k_rows_volume picks its corner terms by these.  One warp takes `per`
+// consecutive rows (a power of two up to 32): the lanes load the rows'
+// neighbour bytes into shared memory entry by entry, each lane replays one row
+// there, and the lanes write the positions back entry by entry.  Rows without
+// a cavity record are left alone.  A warp's replays diverge from one another: a
+// call with fewer rows than 32 for each resident warp spreads them (5,000 rows:
+// 31 us with 32 rows a warp, 17 us with 4).
 constexpr int ORD_WARPS = 2;
+constexpr int ORD_RESIDENT = 16;  // warps a SM holds
 constexpr int ORD_PAD = REC_CAV + 1;  // row stride of the shared tables (banks)
 struct OrderWS {
     int nbr[32][ORD_PAD];
@@ -1206,19 +1370,20 @@ struct OrderWS {
     int start[33];
 };
 
-__global__ void __launch_bounds__(32 * ORD_WARPS) k_rows_order(int64_t nrows, const RowHead *__restrict__ heads,
-                                                               RowEntry *__restrict__ ents) {
+__global__ void __launch_bounds__(32 * ORD_WARPS) k_rows_order(int64_t nrows, int per, const RowHead *__restrict__ heads,
+                                                               RowEntry *__restrict__ ents, DevSummary *sum) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) sum->general_count = 0;  // k_rows_volume's queue, per chunk
     extern __shared__ __align__(16) unsigned char smem[];
     OrderWS &w = reinterpret_cast<OrderWS *>(smem)[threadIdx.x >> 5];
     const int lane = threadIdx.x & 31;
     const unsigned full = 0xffffffffu;
-    const int64_t ngroups = (nrows + 31) / 32;
+    const int64_t ngroups = (nrows + per - 1) / per;
     for (int64_t gi = (int64_t)blockIdx.x * ORD_WARPS + (threadIdx.x >> 5); gi < ngroups;
          gi += (int64_t)gridDim.x * ORD_WARPS) {
-        const int64_t s0 = gi * 32;
+        const int64_t s0 = gi * per;
         const int64_t s = s0 + lane;
         int nc = 0;
-        if (s < nrows) {
+        if (lane < per && s < nrows) {
             const RowHead h = heads[s];
             if (h.state == RS_OK && h.ncav > 0 && h.ncav <= REC_CAV) nc = h.ncav;
         }
@@ -1235,7 +1400,7 @@ __global__ void __launch_bounds__(32 * ORD_WARPS) k_rows_order(int64_t nrows, co
         const int total = w.start[32];
         // row of flattened entry k: the last row whose start is <= k
         auto row_of = [&](int k) {
-            int lo = 0, hi = 32;  // start[lo] <= k < start[hi]
+            int lo = 0, hi = per;  // start[lo] <= k < start[hi]
             while (hi - lo > 1) {
                 const int mid = (lo + hi) >> 1;
                 if (w.start[mid] <= k) lo = mid; else hi = mid;
@@ -1305,12 +1470,37 @@ __global__ void __launch_bounds__(32 * ORD_WARPS) k_rows_order(int64_t nrows, co
     }
 }
 
+// what the split row kernels do with a finished row i
+template <class W, class Sink, int IDS>
+__device__ __forceinline__ void finish_row(int64_t i, RowInfo &r, RowLanes<IDS> &L, const MeshView &M,
+                                           const dv3 q, W &ws, const Grp<FAST_G> &g, Sink &sink,
+                                           const LargeQueue &lq, DevSummary *sum) {
+    if (r.status == ST_CAPACITY) {
+        if (g.lane == 0) lq.list[atomicAdd(&sum->large_count, 1)] = (int)i;
+        return;
+    }
+    if (r.status != ST_OK) {
+        r.nnb = 0;
+        if (g.lane == 0) {
+            atomicAdd(&sum->rows_failed, 1ull);
+            atomicCAS(&sum->first_status, 0, NIF_ERR_WALK);
+        }
+    }
+    record<FAST_G>(sum, r, g.lane);
+    if constexpr (Sink::FULL)
+        sink.template emit_lanes<FAST_G>(i, ws, g, r, L);
+    else
+        sink.template emit_lanes<FAST_G>(i, ws, g, r, L, M, q);
+}
+
+// Rows that split_row_body gives up on (ST_GENERAL) are queued in `gen`, by
+// position, for k_rows_general.
 template <class QT, class Rows, class Sink, int OCC>
 __global__ void __launch_bounds__(FAST_BLOCK, OCC)
     k_rows_volume(const __grid_constant__ Rows rows, const QT *__restrict__ Q,
                   const int *__restrict__ order, int64_t nrows, const RowHead *__restrict__ heads,
-                  const RowEntry *__restrict__ ents, Sink sink, LargeQueue lq, DevSummary *sum,
-                  int tile, unsigned long long *counter) {
+                  const RowEntry *__restrict__ ents, int *__restrict__ gen, Sink sink, LargeQueue lq,
+                  DevSummary *sum, int tile, unsigned long long *counter) {
     extern __shared__ __align__(16) unsigned char smem[];
     constexpr int G = FAST_G;
     constexpr int GPB = FAST_BLOCK / G;
@@ -1337,21 +1527,50 @@ __global__ void __launch_bounds__(FAST_BLOCK, OCC)
             const MeshView &M = rows.get(i, cur, &sview[threadIdx.x / G], g, cen);
             const dv3 q = load_query(Q, i, cen);
             RowInfo r{ST_OK, 0, 0, h.state == RS_OUTSIDE, false, 0.0, 0, 0, 0, 0, 0};
-            if (h.state == RS_OK) r = volume_row<G, VolWS, Sink::FULL>(M, q, ws, g, h, ents + s * REC_CAV);
+            RowLanes<1> L;
+            if (h.state == RS_OK)
+                split_row_body<G, VolWS, Sink::FULL, false>(M, q, ws, g, h, ents + s * REC_CAV, r, L);
             if (h.state == RS_WALK) r.status = ST_WALK;
-            if (r.status == ST_CAPACITY) {
-                if (g.lane == 0) lq.list[atomicAdd(&sum->large_count, 1)] = (int)i;
+            if (r.status == ST_GENERAL) {
+                if (g.lane == 0) gen[atomicAdd(&sum->general_count, 1)] = (int)s;
             } else {
-                if (r.status != ST_OK && g.lane == 0) {
-                    atomicAdd(&sum->rows_failed, 1ull);
-                    atomicCAS(&sum->first_status, 0, NIF_ERR_WALK);
-                }
-                record<G>(sum, r, g.lane);
-                sink.template emit<G>(i, r.status == ST_OK ? r.nnb : 0, ws, g, false, M, q, r);
+                finish_row(i, r, L, M, q, ws, g, sink, lq, sum);
             }
         }
         g.sync();
         s += tile <= 0 ? ng : 1;
+    }
+}
+
+// The rows k_rows_volume queued (about 2 % on random keys; all of them where
+// natinterp3d's degeneracy thresholds exceed the key spacing): a kernel of its
+// own, because the two bodies together outgrow the instruction cache (with
+// both in one kernel the volume pass took 11.1 ms a 2M-row call, 8.0 ms apart).
+template <class QT, class Rows, class Sink>
+__global__ void __launch_bounds__(FAST_BLOCK, GEN_OCC)
+    k_rows_general(const __grid_constant__ Rows rows, const QT *__restrict__ Q,
+                   const int *__restrict__ order, const RowHead *__restrict__ heads,
+                   const RowEntry *__restrict__ ents, const int *__restrict__ gen, Sink sink,
+                   LargeQueue lq, DevSummary *sum) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    constexpr int G = FAST_G;
+    constexpr int GPB = FAST_BLOCK / G;
+    __shared__ MeshView sview[GPB];
+    Grp<G> g;
+    GenWS &ws = reinterpret_cast<GenWS *>(smem)[threadIdx.x / G];
+    int cur = -1;
+    const int n = sum->general_count;
+    for (int j = blockIdx.x * GPB + threadIdx.x / G; j < n; j += gridDim.x * GPB) {
+        const int64_t s = gen[j];
+        const int64_t i = order[s];
+        const double *cen;
+        const MeshView &M = rows.get(i, cur, &sview[threadIdx.x / G], g, cen);
+        const dv3 q = load_query(Q, i, cen);
+        RowInfo r{ST_OK, 0, 0, false, false, 0.0, 0, 0, 0, 0, 0};
+        RowLanes<2> L;
+        split_row_body<G, GenWS, Sink::FULL, true>(M, q, ws, g, heads[s], ents + s * REC_CAV, r, L);
+        finish_row(i, r, L, M, q, ws, g, sink, lq, sum);
+        g.sync();
     }
 }
 
@@ -1555,6 +1774,7 @@ struct MeshLayout {
     int4 *tv, *tn;
     uint32_t *tinfo;
     d4 *tcc, *fcc;
+    d4 *corner;                  // corner terms, null beyond CORNER_TETS_MAX
     d4 *cs;                      // sorted centroids
     float4 *onode;               // octree node records, two float4 each
     unsigned long long *omask;   // octree child digits
@@ -1564,6 +1784,14 @@ struct MeshLayout {
     int *flag;
 };
 
+// Largest mesh that holds its corner terms: 512 bytes a tet, 34 GB here (about
+// 10M keys), next to 270 bytes a tet for the rest.  Larger meshes, which are to
+// leave room for others' data, compute them per row.
+#ifndef NIF_CORNER_TETS_MAX
+#define NIF_CORNER_TETS_MAX (1 << 26)
+#endif
+constexpr int CORNER_TETS_MAX = NIF_CORNER_TETS_MAX;
+
 MeshLayout carve_mesh(Carve &c, int nv, int nt) {
     MeshLayout L;
     L.vtx = c.take<d4>(nv);
@@ -1572,6 +1800,7 @@ MeshLayout carve_mesh(Carve &c, int nv, int nt) {
     L.tinfo = c.take<uint32_t>(nt);
     L.tcc = c.take<d4>(nt);
     L.fcc = c.take<d4>(fcc_slots(nt));
+    L.corner = nt <= CORNER_TETS_MAX ? c.take<d4>(16 * (size_t)nt) : nullptr;
     L.cs = c.take<d4>(nt);
     L.onode = c.take<float4>(2 * (size_t)oct_node_cap(nt));
     L.omask = c.take<unsigned long long>(oct_node_cap(nt));
@@ -1603,6 +1832,7 @@ struct QueryLayout {
     RowHead *heads;         // split-row records of one chunk of rows
     RowEntry *ents;
     int *wide;              // split rows whose cavity exceeds a record
+    int *gen;               // one chunk's rows for k_rows_general
     // weights mode only
     int *cnt;
     uint8_t *staged;
@@ -1644,6 +1874,7 @@ QueryLayout carve_query(Carve &c, int64_t M, int mode) {
         L.heads = c.take<RowHead>(ch);
         L.ents = c.take<RowEntry>(ch * REC_CAV);
         L.wide = c.take<int>(M > 0 ? M : 1);
+        L.gen = c.take<int>(ch);
     }
     if (mode == NIF_MODE_WEIGHTS) {
         const int64_t m1 = M > 0 ? M : 1;
@@ -1893,17 +2124,30 @@ constexpr int sink_occ() {
         return Sink::MIN_BLOCKS;
 }
 
+// k_rows_general over the rows that the launch before queued in `gen`
+template <class QT, class Rows, class Sink>
+void launch_general(const Launch &lc, const Rows &rows, const QT *Q, int64_t n, const int *order,
+                    const RowHead *h, const RowEntry *e, const int *gen, const Sink &sink,
+                    int *large, DevSummary *sum, cudaStream_t st) {
+    constexpr int GPB = FAST_BLOCK / FAST_G;
+    auto kern = k_rows_general<QT, Rows, Sink>;
+    const size_t smem = GPB * sizeof(GenWS);
+    const int64_t cap = (int64_t)resident_blocks(kern, FAST_BLOCK, smem) * lc.num_sms;
+    const int64_t blocks = min((n + GPB - 1) / GPB, cap);
+    kern<<<(unsigned)blocks, FAST_BLOCK, smem, st>>>(rows, Q, order, h, e, gen, sink, LargeQueue{large}, sum);
+}
+
 // The split row over positions [0, M) of R.order, whose rows `rows` maps to
 // their meshes: k_locate over all rows, then per chunk of REC_CHUNK rows the
 // cavity records and the volumes.  Rows whose cavity exceeds a record are
 // left in `wide` (count in R.sum->wide_count) for the fused kernel.
 template <class QT, class Rows, class Sink, int OCC, int PM = PM_PLAIN>
 void launch_split(const Launch &lc, const Rows &rows, const QT *Q, int64_t M, const RowSet &R,
-                  RowHead *heads, RowEntry *ents, int *wide, const Sink &sink, cudaStream_t st,
+                  RowHead *heads, RowEntry *ents, int *wide, int *gen, const Sink &sink, cudaStream_t st,
                   bool keep = false) {
     constexpr int GPB = FAST_BLOCK / FAST_G;
     constexpr int COCC = NIF_CAV_OCC > 0 ? NIF_CAV_OCC : OCC;
-    constexpr int VOCC = sink_occ<Sink, (NIF_VOL_OCC > 0 ? NIF_VOL_OCC : OCC)>();
+    constexpr int VOCC = sink_occ<Sink, (NIF_VOL_OCC > 0 ? NIF_VOL_OCC : (OCC == OCC_HI ? 7 : OCC))>();
     int *located = const_cast<int *>(R.located);
     prof_span(SPAN_LOCATE, false, st);
     launch_rows(k_locate<QT, Rows, PM>, lc, M, 0, R.counter, st, rows, Q, R.order, M, located,
@@ -1921,17 +2165,21 @@ void launch_split(const Launch &lc, const Rows &rows, const QT *Q, int64_t M, co
         prof_span(SPAN_CAVITY, true, st);
         prof_span(SPAN_ORDER, false, st);
         {
-            const int64_t groups = (n + 31) / 32;
+            // one row a warp while the rows fit the resident warps (14 KB each), up to 32
+            int per = 1;
+            while (per < 32 && n > (int64_t)per * ORD_RESIDENT * lc.num_sms) per *= 2;
+            const int64_t groups = (n + per - 1) / per;
             int64_t ob = (groups + ORD_WARPS - 1) / ORD_WARPS;
             if (ob > (int64_t)lc.num_sms * 32) ob = (int64_t)lc.num_sms * 32;
             k_rows_order<<<(unsigned)ob, 32 * ORD_WARPS, ORD_WARPS * sizeof(OrderWS), st>>>(
-                n, (const RowHead *)h, e);
+                n, per, (const RowHead *)h, e, R.sum);
         }
         prof_span(SPAN_ORDER, true, st);
         prof_span(SPAN_VOLUME, false, st);
         launch_rows(k_rows_volume<QT, Rows, Sink, VOCC>, lc, n, GPB * sizeof(VolWS), R.counter, st,
-                    rows, Q, R.order + c0, n, (const RowHead *)h, (const RowEntry *)e, sink,
+                    rows, Q, R.order + c0, n, (const RowHead *)h, (const RowEntry *)e, gen, sink,
                     LargeQueue{R.large}, R.sum);
+        launch_general(lc, rows, Q, n, R.order + c0, h, e, gen, sink, R.large, R.sum, st);
         prof_span(SPAN_VOLUME, true, st);
     }
 }
@@ -1943,17 +2191,17 @@ void launch_split(const Launch &lc, const Rows &rows, const QT *Q, int64_t M, co
 template <class QT, class Sink, int PM>
 void launch_fast(const nif_dmesh *m, const QT *Q, int64_t M, const Centroid &cen,
                  const RowSet &R, const Sink &sink, cudaStream_t st, RowHead *heads = nullptr,
-                 RowEntry *ents = nullptr, int *wide = nullptr, bool keep = false) {
+                 RowEntry *ents = nullptr, int *wide = nullptr, int *gen = nullptr, bool keep = false) {
     if constexpr (PM == PM_PLAIN || PM == PM_FILTER) {
         if (R.located && heads && !R.nrows_dev) {
             const Launch lc{m->tune.tile, m->num_sms};
             const OneMesh rows{m->view, cen};
             if (m->tune.blocks_per_sm == OCC_LO)
-                launch_split<QT, OneMesh, Sink, OCC_LO, PM>(lc, rows, Q, M, R, heads, ents, wide, sink,
-                                                            st, keep);
+                launch_split<QT, OneMesh, Sink, OCC_LO, PM>(lc, rows, Q, M, R, heads, ents, wide, gen,
+                                                            sink, st, keep);
             else
-                launch_split<QT, OneMesh, Sink, OCC_HI, PM>(lc, rows, Q, M, R, heads, ents, wide, sink,
-                                                            st, keep);
+                launch_split<QT, OneMesh, Sink, OCC_HI, PM>(lc, rows, Q, M, R, heads, ents, wide, gen,
+                                                            sink, st, keep);
             // rows whose cavity exceeds a record: the fused row kernel (which
             // queues what exceeds its own capacities for the large kernel)
             const RowSet W{wide, &R.sum->wide_count, R.large, R.sum, R.counter, nullptr};
@@ -1977,11 +2225,13 @@ void run_rows(const nif_dmesh *m, const QT *Q, int64_t M, const Centroid &cen, c
               const RecordLayout *rec = nullptr) {
     if (m->view.pmode == PRED_FAST && rec)
         launch_fast<QT, Sink, PM_PLAIN>(m, Q, M, cen, all_rows(L), sink, st, rec->heads, rec->ents,
-                                        L.wide, true);
+                                        L.wide, L.gen, true);
     else if (m->view.pmode == PRED_FAST)
-        launch_fast<QT, Sink, PM_PLAIN>(m, Q, M, cen, all_rows(L), sink, st, L.heads, L.ents, L.wide);
+        launch_fast<QT, Sink, PM_PLAIN>(m, Q, M, cen, all_rows(L), sink, st, L.heads, L.ents, L.wide,
+                                        L.gen);
     else
-        launch_fast<QT, Sink, PM_FILTER>(m, Q, M, cen, all_rows(L), sink, st, L.heads, L.ents, L.wide);
+        launch_fast<QT, Sink, PM_FILTER>(m, Q, M, cen, all_rows(L), sink, st, L.heads, L.ents, L.wide,
+                                        L.gen);
     prof_mark(2, st);
     k_rows_large<QT, Sink><<<large_groups, 32, 0, st>>>(m->view, Q, cen, LargeQueue{L.large_list},
                                                         sink, L.large_ws, L.exact, L.sum);
@@ -1996,9 +2246,9 @@ void refill_rows(const nif_dmesh *m, const QT *Q, int64_t M, const Centroid &cen
     // (few rows: the row kernel locates them itself)
     const RowSet R{L.refill, &L.sum->refill_count, L.large_list, L.fill_sum, L.counter, nullptr};
     if (m->view.pmode == PRED_FAST)
-        launch_fast<QT, Sink, PM_PLAIN>(m, Q, M, cen, R, sink, st);
+        launch_fast_loc<QT, Sink, PM_PLAIN>(m, Q, M, cen, R, sink, st);
     else
-        launch_fast<QT, Sink, PM_FILTER>(m, Q, M, cen, R, sink, st);
+        launch_fast_loc<QT, Sink, PM_FILTER>(m, Q, M, cen, R, sink, st);
     // the rows the large kernel handled (their queue is intact: refilled rows
     // all fit the fast kernel, so nothing is appended to it)
     k_rows_large<QT, Sink><<<LARGE_GROUPS, 32, 0, st>>>(m->view, Q, cen, LargeQueue{L.large_list},
@@ -2096,6 +2346,7 @@ NIF_EXPORT int nif_dmesh_create(const double *d_vxyz, const int32_t *d_tet_v,
     V.tinfo = L.tinfo;
     V.tcc = L.tcc;
     V.fcc = L.fcc;
+    V.corner = L.corner;
     V.n = n_vertices - 4;
     V.nv = n_vertices;
     V.nt = n_tets;
@@ -2267,6 +2518,8 @@ NIF_EXPORT int nif_dmesh_create(const double *d_vxyz, const int32_t *d_tet_v,
             k_grid_fill<<<nb, 256, 0, st>>>(V, T.gcursor, L.gitems);
         }
         k_prep_geometry<<<blocks_for(n_tets, 128), 128, 0, st>>>(V, L.tinfo, L.tcc, L.fcc, L.flag);
+        if (L.corner)
+            k_prep_corner<<<blocks_for(16 * (int64_t)n_tets, 128), 128, 0, st>>>(V, L.corner);
         int flag[4];
         if (cudaMemcpyAsync(flag, L.flag, sizeof(flag), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
             cudaStreamSynchronize(st) != cudaSuccess) {
@@ -2904,7 +3157,10 @@ void grad_records_typed(const nif_dmesh *m, const void *q, int64_t M, const Cent
         const int64_t n = min((int64_t)REC_CHUNK, M - c0);
         launch_rows(k_rows_volume<QT, OneMesh, Sink, Sink::MIN_BLOCKS>, lc, n, GPB * sizeof(VolWS),
                     R.counter, st, rows, Q, L.order + c0, n, (const RowHead *)(R.heads + c0),
-                    (const RowEntry *)(R.ents + c0 * REC_CAV), sink, LargeQueue{R.requeue}, R.sum);
+                    (const RowEntry *)(R.ents + c0 * REC_CAV), L.gen, sink, LargeQueue{R.requeue}, R.sum);
+        launch_general(lc, rows, Q, n, L.order + c0, R.heads + c0, R.ents + c0 * REC_CAV, L.gen, sink,
+                       R.requeue, R.sum, st);
+        if (c0 + REC_CHUNK < M) cudaMemsetAsync(&R.sum->general_count, 0, sizeof(int), st);
     }
     const RowSet W{L.wide, &L.sum->wide_count, R.requeue, R.sum, R.counter, nullptr};
     launch_fast_loc<QT, Sink, PM_PLAIN>(m, Q, M, cen, W, sink, st);
@@ -3073,6 +3329,12 @@ struct BatchInterpSink {
         InterpSink<WT, VT, CT> s{values + koff[p] * D, out, D};
         s.template emit<G>(i, nnb, ws, g, large, M, q, r);
     }
+    template <int G, class W, int IDS>
+    __device__ __forceinline__ void emit_lanes(int64_t i, W &ws, const Grp<G> &g, RowInfo &r,
+                                               RowLanes<IDS> &L) {
+        InterpSink<WT, VT, CT> s{values + koff[find_problem(qoff, P, i)] * D, out, D};
+        s.template emit_lanes<G>(i, ws, g, r, L);
+    }
 };
 
 // persistent row kernel of a batch: warps pull tiles of bucket-ordered
@@ -3196,7 +3458,7 @@ struct BatchLayout {
     double *exact;
     // split rows (the default predicate mode): located tets, one chunk's
     // records, rows whose cavity exceeds a record
-    int *located, *wide;
+    int *located, *wide, *gen;
     RowHead *heads;
     RowEntry *ents;
 };
@@ -3222,6 +3484,7 @@ BatchLayout carve_batch(Carve &c, int P, int64_t M) {
     L.wide = c.take<int>(m1);
     L.heads = c.take<RowHead>(ch);
     L.ents = c.take<RowEntry>(ch * REC_CAV);
+    L.gen = c.take<int>(ch);
     return L;
 }
 
@@ -3282,17 +3545,19 @@ void batch_typed(const nif_dbatch *b, const void *q, int64_t M, const int64_t *q
     if (b->filtered) {
         if (b->tune.blocks_per_sm == OCC_LO)
             launch_split<QT, ManyMeshes, Sink, OCC_LO, PM_FILTER>(lc, rows, Q, M, R, L.heads, L.ents,
-                                                                  L.wide, sink, st);
+                                                                  L.wide, L.gen, sink, st);
         else
             launch_split<QT, ManyMeshes, Sink, OCC_HI, PM_FILTER>(lc, rows, Q, M, R, L.heads, L.ents,
-                                                                  L.wide, sink, st);
+                                                                  L.wide, L.gen, sink, st);
         launch_batch_rows<QT, Sink, PM_FILTER>(b, Q, M, qoff, cens, sink, L, st, L.wide,
                                                &L.sum->wide_count);
     } else {
         if (b->tune.blocks_per_sm == OCC_LO)
-            launch_split<QT, ManyMeshes, Sink, OCC_LO>(lc, rows, Q, M, R, L.heads, L.ents, L.wide, sink, st);
+            launch_split<QT, ManyMeshes, Sink, OCC_LO>(lc, rows, Q, M, R, L.heads, L.ents, L.wide, L.gen,
+                                                       sink, st);
         else
-            launch_split<QT, ManyMeshes, Sink, OCC_HI>(lc, rows, Q, M, R, L.heads, L.ents, L.wide, sink, st);
+            launch_split<QT, ManyMeshes, Sink, OCC_HI>(lc, rows, Q, M, R, L.heads, L.ents, L.wide, L.gen,
+                                                       sink, st);
         launch_batch_rows<QT, Sink, PM_PLAIN>(b, Q, M, qoff, cens, sink, L, st, L.wide,
                                               &L.sum->wide_count);
     }

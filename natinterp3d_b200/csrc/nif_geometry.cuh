@@ -33,6 +33,24 @@ __device__ __forceinline__ double fsub(double a, double b) { return __dsub_rn(a,
 __device__ __forceinline__ double fmul(double a, double b) { return __dmul_rn(a, b); }
 __device__ __forceinline__ double fdiv(double a, double b) { return __ddiv_rn(a, b); }
 
+// 1 / x: the correctly rounded reciprocal, the same bits as fdiv(1.0, x)
+__device__ __forceinline__ double frcp(double x) { return __drcp_rn(x); }
+
+// x / 12, correctly rounded, in three operations: with y the correctly
+// rounded 1/12 and q = x y (within one ulp of the quotient), the residual
+// r = x - 12 q is exact and q + r y rounds to x / 12 (Markstein, "Computation
+// of elementary functions on the IBM RISC System/6000 processor", 1990,
+// theorem on division from a correctly rounded reciprocal).  That needs r
+// representable: numbers near the ends of the exponent range, infinities and
+// NaN take the plain division.
+__device__ __forceinline__ double div12(double x) {
+    const double y = 1.0 / 12.0;
+    const double q = fmul(x, y);
+    const unsigned e = ((unsigned)__double2hiint(x) >> 20) & 0x7ffu;
+    if (e - 100u < 1900u) return __fma_rn(__fma_rn(-12.0, q, x), y, q);
+    return fdiv(x, 12.0);
+}
+
 __device__ __forceinline__ dv3 mk(double x, double y, double z) { return dv3{x, y, z}; }
 __device__ __forceinline__ dv3 mk(const double4 &v) { return dv3{v.x, v.y, v.z}; }
 __device__ __forceinline__ dv3 vsub(dv3 a, dv3 b) { return dv3{fsub(a.x, b.x), fsub(a.y, b.y), fsub(a.z, b.z)}; }
@@ -77,24 +95,33 @@ NIF_GEOM_FN double insphere_fast(dv3 a, dv3 b, dv3 c, dv3 d, dv3 e) {
 }
 
 // circumcentre of triangle (a, b, c); centroid when |ab x ac|^2 < 1e-30
-NIF_GEOM_FN dv3 tri_cc(dv3 a, dv3 b, dv3 c) {
+// (tri_cc_regular: the circumcentre's own formula, `flat` set where the
+// centroid is wanted)
+__device__ __forceinline__ dv3 tri_cc_regular(dv3 a, dv3 b, dv3 c, bool &flat) {
     dv3 ab = vsub(b, a), ac = vsub(c, a);
     dv3 n = vcross(ab, ac);
     double n2 = vdot(n, n);
-    if (n2 < 1e-30) {
-        return dv3{fdiv(fadd(fadd(a.x, b.x), c.x), 3.0), fdiv(fadd(fadd(a.y, b.y), c.y), 3.0),
-                   fdiv(fadd(fadd(a.z, b.z), c.z), 3.0)};
-    }
+    flat = n2 < 1e-30;
     double ab2 = vdot(ab, ab), ac2 = vdot(ac, ac);
     dv3 t = dv3{fsub(fmul(ab2, ac.x), fmul(ac2, ab.x)), fsub(fmul(ab2, ac.y), fmul(ac2, ab.y)),
                 fsub(fmul(ab2, ac.z), fmul(ac2, ab.z))};
     dv3 cr = vcross(t, n);
-    double inv = fdiv(1.0, fmul(2.0, n2));
+    double inv = frcp(fmul(2.0, n2));
     return vadd(a, vscale(cr, inv));
 }
 
+NIF_GEOM_FN dv3 tri_cc(dv3 a, dv3 b, dv3 c) {
+    bool flat;
+    const dv3 r = tri_cc_regular(a, b, c, flat);
+    if (flat)
+        return dv3{fdiv(fadd(fadd(a.x, b.x), c.x), 3.0), fdiv(fadd(fadd(a.y, b.y), c.y), 3.0),
+                   fdiv(fadd(fadd(a.z, b.z), c.z), 3.0)};
+    return r;
+}
+
 // circumcentre of tetrahedron (a, b, c, d); centroid when |denominator| < 1e-30
-NIF_GEOM_FN dv3 tet_cc(dv3 a, dv3 b, dv3 c, dv3 d) {
+// (tet_cc_regular: as tri_cc_regular)
+__device__ __forceinline__ dv3 tet_cc_regular(dv3 a, dv3 b, dv3 c, dv3 d, bool &flat) {
     dv3 ba = vsub(b, a), ca = vsub(c, a), da = vsub(d, a);
     dv3 x1 = vcross(ba, ca), x2 = vcross(da, ba), x3 = vcross(ca, da);
     dv3 m1 = vscale(x1, vdot(da, da));
@@ -102,12 +129,41 @@ NIF_GEOM_FN dv3 tet_cc(dv3 a, dv3 b, dv3 c, dv3 d) {
     dv3 m3 = vscale(x3, vdot(ba, ba));
     dv3 s = vadd(m3, vadd(m1, m2));
     double den = fmul(2.0, vdot(ba, x3));
-    if (fabs(den) < 1e-30) {
+    flat = fabs(den) < 1e-30;
+    return vadd(vscale(s, frcp(den)), a);
+}
+
+NIF_GEOM_FN dv3 tet_cc(dv3 a, dv3 b, dv3 c, dv3 d) {
+    bool flat;
+    const dv3 r = tet_cc_regular(a, b, c, d, flat);
+    if (flat)
         return dv3{fmul(fadd(fadd(fadd(a.x, b.x), c.x), d.x), 0.25),
                    fmul(fadd(fadd(fadd(a.y, b.y), c.y), d.y), 0.25),
                    fmul(fadd(fadd(fadd(a.z, b.z), c.z), d.z), 0.25)};
+    return r;
+}
+
+// The subcell volume from the orientation sv of (pa, pb, pc) about pk, the
+// edges e1 = pa - pb, e2 = pa - pc, e3 = pb - pc, and the face circumcentres
+// (dab, dac, dbc) and the tet's (dt), relative to pk.  natinterp3d swaps pa
+// with pb and dac with dbc when sv < 0: that negates e1, exchanges e2 with e3
+// and turns the cross products into (c1, -c3, -c2), so that the swapped sum is
+// the negated sum of the same nine products in the order 1, 3, 2 (a rounded
+// operation on negated operands gives the negated result).
+__device__ __forceinline__ double subcell_from(double sv, dv3 e1, dv3 e2, dv3 e3, dv3 dab, dv3 dac,
+                                               dv3 dbc, dv3 dt) {
+    const dv3 c1 = vcross(dab, dt), c2 = vcross(dt, dac), c3 = vcross(dbc, dt);
+    const dv3 m2{fmul(e2.x, c2.x), fmul(e2.y, c2.y), fmul(e2.z, c2.z)};
+    const dv3 m3{fmul(e3.x, c3.x), fmul(e3.y, c3.y), fmul(e3.z, c3.z)};
+    double vol = fadd(fadd(fmul(e1.x, c1.x), fmul(e1.y, c1.y)), fmul(e1.z, c1.z));
+    if (sv < 0) {
+        vol = fadd(fadd(fadd(vol, m3.x), m3.y), m3.z);
+        vol = -fadd(fadd(fadd(vol, m2.x), m2.y), m2.z);
+    } else {
+        vol = fadd(fadd(fadd(vol, m2.x), m2.y), m2.z);
+        vol = fadd(fadd(fadd(vol, m3.x), m3.y), m3.z);
     }
-    return vadd(vscale(s, fdiv(1.0, den)), a);
+    return div12(vol);
 }
 
 // Signed volume of the part of tet (pk, pa, pb, pc) closer to pk than to the
@@ -117,28 +173,9 @@ NIF_GEOM_FN dv3 tet_cc(dv3 a, dv3 b, dv3 c, dv3 d) {
 NIF_GEOM_FN double subcell_volume(dv3 pk, dv3 pa, dv3 pb, dv3 pc, dv3 ct, dv3 fab,
                                                 dv3 fac, dv3 fbc) {
     dv3 ta = vsub(pa, pk), tb = vsub(pb, pk), tc = vsub(pc, pk);
-    double sv = vdot(ta, vcross(tb, tc));
-    dv3 a = pa, b = pb;
-    if (sv < 0) {
-        a = pb;
-        b = pa;
-        dv3 t = fac;
-        fac = fbc;
-        fbc = t;
-    }
-    dv3 df = vsub(fab, pk), dg = vsub(fac, pk), dh = vsub(fbc, pk), dt = vsub(ct, pk);
-    dv3 c1 = vcross(df, dt), c2 = vcross(dt, dg), c3 = vcross(dh, dt);
-    dv3 e1 = vsub(a, b), e2 = vsub(a, pc), e3 = vsub(b, pc);
-    double vol = fmul(e1.x, c1.x);
-    vol = fadd(vol, fmul(e1.y, c1.y));
-    vol = fadd(vol, fmul(e1.z, c1.z));
-    vol = fadd(vol, fmul(e2.x, c2.x));
-    vol = fadd(vol, fmul(e2.y, c2.y));
-    vol = fadd(vol, fmul(e2.z, c2.z));
-    vol = fadd(vol, fmul(e3.x, c3.x));
-    vol = fadd(vol, fmul(e3.y, c3.y));
-    vol = fadd(vol, fmul(e3.z, c3.z));
-    return fdiv(vol, 12.0);
+    const double sv = vdot(ta, vcross(tb, tc));
+    return subcell_from(sv, vsub(pa, pb), vsub(pa, pc), vsub(pb, pc), vsub(fab, pk), vsub(fac, pk),
+                        vsub(fbc, pk), vsub(ct, pk));
 }
 
 }  // namespace nif

@@ -40,6 +40,8 @@
 #include <stddef.h>
 #include <stdint.h>
 
+#include <type_traits>
+
 #include "nif_exact.h"
 #include "nif_geometry.cuh"
 
@@ -81,6 +83,7 @@ struct MeshView {
                                        // bits 8+2j: mirror slot of face j
     const d4 *__restrict__ tcc;        // [nt] tet circumcentre
     const d4 *__restrict__ fcc;        // [nt*4] circumcentre of the face opposite p[i]
+    const d4 *__restrict__ corner;     // [nt*16] corner terms (corner_term), or null
     // Tet centroids, (p0 + p1 + p2 + p3) / 4 per axis as natinterp3d's
     // constructor computes them for its k-d tree (delaunay.c:151-157), sorted
     // by a 60-bit Morton code of their cell in a 2^20 grid per axis over the
@@ -455,6 +458,7 @@ __device__ int grid_nearest(const MeshView &M, const dv3 q) {
 // visiting order.  Index types are the narrowest that hold each capacity.
 template <int HS_, int CAV_, int BF_, int NBR_, int VH_, int G_, class SlotT, class CavT>
 struct Workspace {
+    static constexpr bool SPLIT = false;
     static constexpr int HS = HS_;        // tested-tet hash slots (power of two)
     static constexpr int QCAP = HS_ * 3 / 4;
     static constexpr int CAV = CAV_;      // cavity tets
@@ -514,28 +518,68 @@ struct CavWorkspace {
     CavT pos[CAV_];
 };
 
-template <int CAV_, int BF_, int NBR_, int VH_, int G_>
-struct VolWorkspace {
+// Workspace of the split row's volume phase (split_row): room for BF boundary
+// faces.  The phases reuse one arena.  A vertex's id is its number in the row,
+// in no particular order: the natural neighbours, then the super-simplex's
+// four vertices.
+constexpr int VOL_VERTS = 56;      // ids of a row (columns are below 63)
+constexpr int VOL_NO_ID = 255;     // a cavity vertex that is on no boundary face
+template <int CAV_, int BF_, int VH_, int G_>
+struct alignas(16) VolWorkspace {
+    static constexpr bool SPLIT = true;
     static constexpr int CAV = CAV_;
     static constexpr int BF = BF_;
-    static constexpr int NBR = NBR_;
+    static constexpr int FW = (BF_ + 63) / 64;  // 64-bit words of a face set
+    using edge_t = typename std::conditional<(BF_ <= 85), uint8_t, uint16_t>::type;
+    static constexpr unsigned NO_EDGE = (1u << 8 * sizeof(edge_t)) - 1u;
+    static constexpr int PAIR_IDS = FW == 1 ? 36 : VOL_VERTS;  // ids of a row that this size takes
+    static constexpr int NBR = VOL_VERTS - 4;
     static constexpr int VH = VH_;
     static constexpr int G = G_;
     union U {
-        double buf[4 * G_ * 10 / 8];  // the fold's item buffer (4 G terms + slots); sink staging
+        struct {
+            int tet[CAV_];       // cavity tets in visiting order
+            unsigned lid[CAV_];  // their vertices' ids, one byte each (first: hash slots)
+            uint8_t mask[CAV_];  // boundary faces, and << 4 the faces that take a neighbour's copy
+            unsigned long long tm[VOL_VERTS];       // per neighbour, the set of its cavity tets
+            unsigned firsts[(3 * BF_ + 31) / 32];   // the set of corners that are a vertex's first
+            union {
+                struct {
+                    alignas(16) int vh_key[VH_];
+                    int vh_first[VH_];
+                } h;
+                double term[4 * CAV_];              // cavity terms, by neighbour
+            };
+        } c;
+        // directed boundary edge (u, w) -> 3 * face + corner of u, all ones: none
+        edge_t pair[PAIR_IDS * PAIR_IDS + 16 / sizeof(edge_t)];
+        struct {
+            // circumcentre of (u, q, w) relative to u, per directed boundary edge
+            double ec[3 * BF_][3];
+            double ct[BF_][3];     // circumcentre of (q, face)
+        } v;
     } u;
-    double acc[NBR_];
-    int4 ctv[CAV_];     // vertex record of the o-th visited cavity tet
-    int4 cfp[CAV_];     // fcc[] indices of its faces (natinterp3d's face cache)
-    int cav_tet[CAV_];  // cavity tets in visiting order
-    int ftet[CAV_];     // cavity tets in the flood's order (the record's)
-    int8_t fpos[CAV_];  // visiting position of the e-th record entry
-    int nbr_vid[NBR_];
-    int vh_key[VH_];
-    int vh_first[VH_];
-    uint16_t bface[BF_];
-    int16_t vh_slot[VH_];
-    uint8_t bmask[CAV_];  // boundary faces of each cavity tet, one bit per face
+    union {
+        double pos[VOL_VERTS][3];  // vertex positions by id
+        struct {
+            double acc[64];        // weights by neighbour, once the terms are added
+            int vh_first[64];      // scratch of the sinks
+        };
+    };
+    union {
+        unsigned long long fm[FW * VOL_VERTS];  // per id, the set of its boundary faces
+        double fterm[3 * BF_];   // face terms, by neighbour
+    };
+    // per face corner: ids of its vertex u, of the next w and the one after x (6
+    // bits each), another face's edge u -> x (EB bits, all ones: none), and the
+    // place of its term
+    using corner_t = typename std::conditional<(BF_ < 43), unsigned, unsigned long long>::type;
+    static constexpr int EB = BF_ < 43 ? 7 : 10;
+    corner_t corner[3 * BF_];
+    int start[VOL_VERTS];        // first term of a neighbour: cavity, face << 16 (first: its first corner)
+    int nbr_vid[VOL_VERTS];
+    unsigned fid[BF_];           // ids of the face's three vertices, one byte each
+    int bff[BF_];                // fcc[] index of the face (first: visiting position << 2 | face)
 };
 
 // One row between k_rows_cavity, k_rows_order and k_rows_volume: a header
@@ -589,7 +633,8 @@ __device__ __forceinline__ int hash_upsert(int *keys, int hs, int key, bool &ful
     unsigned h = mix_hash(key) & (unsigned)(hs - 1);
 #pragma unroll 1
     for (int probe = 0; probe < hs; ++probe) {
-        const int old = atomicCAS(&keys[h], -1, key);
+        int old = *(volatile int *)&keys[h];  // most keys are there already
+        if (old == -1) old = atomicCAS(&keys[h], -1, key);
         if (old == -1 || old == key) return (int)h;
         h = (h + 1) & (unsigned)(hs - 1);
     }
@@ -1357,68 +1402,495 @@ __device__ int cavity_record(const MeshView &M, const dv3 q, W &ws, const Grp<G>
     return REC_DONE;
 }
 
+// The corner term of cavity tet t at its vertex vi (natural_insertionfree.c:
+// 642-676): the subcell volume at p[vi] from the tet's circumcentre and those
+// of its three faces through p[vi].  Bit i of mask: the face opposite p[i]
+// takes the copy of the neighbour across it, as natinterp3d's face cache does
+// when that neighbour was visited earlier (:233-253).  A term depends on
+// nothing but the mesh and the mask, so that meshes of up to CORNER_TETS_MAX
+// tets hold all of them (MeshView::corner, four a tet and mask: a cavity tet
+// is one 32-byte sector to a row instead of four vertices, five circumcentres
+// and some 110 FP64 operations a corner).
+__device__ __forceinline__ double corner_term(const MeshView &M, int t, unsigned mask, int vi) {
+    const int4 p = M.tv[t];
+    const int4 n = M.tn[t];
+    const uint32_t info = M.tinfo[t];
+    auto face = [&](int i) {
+        const int j = 3 - i;
+        const int nb = comp(n, j);
+        const int k = ((mask >> i) & 1u) && nb >= 0 ? 4 * nb + (3 - (int)((info >> (8 + 2 * j)) & 3u))
+                                                    : 4 * t + i;
+        return cload(&M.fcc[k]);
+    };
+    // the other three vertices in ascending slot order
+    const int o0 = vi == 0 ? 1 : 0, o1 = vi <= 1 ? 2 : 1, o2 = vi <= 2 ? 3 : 2;
+    return subcell_volume(vload(M, comp(p, vi)), vload(M, comp(p, o0)), vload(M, comp(p, o1)),
+                          vload(M, comp(p, o2)), cload(&M.tcc[t]), face(o2), face(o1), face(o0));
+}
+
+// all four, out of line, for the rows of a mesh without the table
+__device__ __noinline__ d4 corner_terms_direct(const MeshView &M, int t, unsigned mask) {
+    double v[4];
+#pragma unroll 1
+    for (int i = 0; i < 4; i++) v[i] = corner_term(M, t, mask, i);
+    return d4{v[0], v[1], v[2], v[3]};
+}
+
+// the ids of a face's three vertices, one byte each, from its tet's ids
+__device__ __forceinline__ unsigned face_ids(unsigned lid, int f) {
+    // byte selectors of getFaceVerticies3's slots: (0, 1, 2), (3, 1, 0), (0, 2, 3), (3, 2, 1)
+    const unsigned sel = f == 0 ? 0x0210u : (f == 1 ? 0x0013u : (f == 2 ? 0x0320u : 0x0123u));
+    return __byte_perm(lid, 0, sel) & 0xffffffu;
+}
+
+__device__ __forceinline__ dv3 sload(const double (&p)[3]) { return dv3{p[0], p[1], p[2]}; }
+__device__ __forceinline__ void sstore(double (&p)[3], const dv3 &v) {
+    p[0] = v.x;
+    p[1] = v.y;
+    p[2] = v.z;
+}
+
 // The split row, part 2: from a record of part 1 (state RS_OK) the row as
-// sibson_row returns it (steps 3-5, or the coincident-vertex row).
-template <int G, class W, bool FULL>
-__device__ RowInfo volume_row(const MeshView &M, const dv3 q, W &ws, const Grp<G> &g,
-                              const RowHead &head, const RowEntry *__restrict__ ent) {
-    RowInfo r{ST_OK, 0, 0, false, false, 0.0, 0, 0, 0, 0, 0};
-    const int ncav = head.ncav;
-    if (ncav == 0) {
-        coincident_row<G>(M, q, ws, g, head.start, r);
-        return r;
+// sibson_row returns it (steps 3-5, or the coincident-vertex row).  With
+// FULL = false it stops at the neighbours and the boundary faces.
+//
+// Bound by instruction issue, and by instruction fetch where the code
+// outgrows the instruction cache: loops are not unrolled, and what a row
+// shares is computed once.
+//  - vertices get their id once per cavity tet (one hash pass over the tets'
+//    vertices), and their positions are staged by id;
+//  - cavity terms come from the mesh's corner table;
+//  - a lane takes a corner of a boundary face;
+//  - a triangle circumcentre (u, q, w) belongs to a directed boundary edge:
+//    the two faces that share the edge each need both directions, so a corner
+//    computes one and reads the other from the face that the sets of u's and
+//    w's faces have in common;
+//  - a neighbour's terms are stored next to each other, in natinterp3d's item
+//    order (a term's place is the number of the neighbour's tets or faces
+//    before it, from the same sets), and one lane a neighbour adds them.
+// GENERAL = false gives up (ST_GENERAL) on rows of more than 32 neighbours or
+// W::BF faces, on flat triangles and tets (natinterp3d's centroid fallbacks)
+// and on edges that are not shared by two faces; GENERAL = true, a kernel of
+// its own, takes those from the start.
+constexpr int ST_GENERAL = 8;
+
+__device__ __forceinline__ int scan_add(int v, int lane) {  // inclusive, over the warp
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int t = __shfl_up_sync(0xffffffffu, v, o);
+        if (lane >= o) v += t;
     }
-    // the record is in the flood's order: place each tet at its position in
-    // natinterp3d's visiting order
-    for (int e = g.lane; e < ncav; e += G) {
+    return v;
+}
+
+// term[0 .. n) added to a in order
+__device__ __forceinline__ void add_terms(double &a, const double *term, int n) {
+#pragma unroll 1
+    for (int i = 0; i < n; i++) a = fadd(a, term[i]);
+}
+
+// The row's neighbours as lane l of the warp holds them: neighbour l (and
+// l + 32), its vertex, its column and its stolen volume (split_row_body), or its
+// weight (split_weights).
+template <int IDS>
+struct RowLanes {
+    double a[IDS];
+    int col[IDS], vid[IDS];
+    __device__ __forceinline__ RowLanes() {  // no neighbour
+#pragma unroll
+        for (int i = 0; i < IDS; i++) {
+            a[i] = 0.0;
+            col[i] = 63;
+            vid[i] = 0;
+        }
+    }
+};
+
+template <int G, class W, bool FULL, bool GENERAL, int IDS>
+__device__ __forceinline__ void split_row_body(const MeshView &M, const dv3 q, W &ws, const Grp<G> &g,
+                                               const RowHead &head, const RowEntry *__restrict__ ent,
+                                               RowInfo &r, RowLanes<IDS> &out) {
+    static_assert(G == 32, "one warp a row");
+    constexpr int FW = W::FW;
+    static_assert(GENERAL || FW == 1, "a face set is one word of the common rows");
+    static_assert(IDS == (GENERAL ? 2 : 1), "neighbours of a lane");
+    const int ncav = head.ncav;
+    const int lane = g.lane;
+    if (ncav == 0) {
+        // natural_insertionfree.c:596-622, as coincident_row
+        int v = -1;
+        bool co = false;
+        if (lane < 4) {
+            v = comp(M.tv[head.start], lane);
+            co = v < M.n && veq(vload(M, v), q);
+        }
+        const unsigned cm = g.ballot(co);
+        r.nnb = __popc(cm);
+        r.coincident = true;
+        out.vid[0] = v;
+        if (co) out.col[0] = __popc(cm & g.lt());
+        out.a[0] = r.nnb > 0 ? fdiv(1.0, (double)r.nnb) : 0.0;
+        return;
+    }
+    if (FULL && !GENERAL && !M.corner) {
+        r.status = ST_GENERAL;
+        return;
+    }
+    auto &C = ws.u.c;
+
+    // ---- the cavity's vertices, numbered by hash slot -----------------------
+    static_assert(W::VH == 64, "one 8-byte clear a lane");
+    reinterpret_cast<int2 *>(C.h.vh_key)[lane] = make_int2(-1, -1);
+    reinterpret_cast<int2 *>(C.h.vh_first)[lane] = make_int2(INT_MAX, INT_MAX);
+    if (lane < VOL_VERTS / 2)
+        reinterpret_cast<ulonglong2 *>(C.tm)[lane] = make_ulonglong2(0ull, 0ull);
+#pragma unroll
+    for (int w = 0; w < FW; w++)
+        if (lane < VOL_VERTS / 2)
+            reinterpret_cast<ulonglong2 *>(ws.fm)[w * (VOL_VERTS / 2) + lane] = make_ulonglong2(0ull, 0ull);
+    static_assert(sizeof(C.firsts) <= 32 * sizeof(unsigned), "one clear a lane");
+    if (lane < (int)(sizeof(C.firsts) / sizeof(unsigned))) C.firsts[lane] = 0u;
+    g.sync();
+    bool vfull = false;
+    d4 terms{0.0, 0.0, 0.0, 0.0};  // the corner terms of the lane's first tet, on their way early
+    int first_o = 0;
+#pragma unroll 1
+    for (int e = lane; e < ncav; e += 32) {
+        // the record is in the flood's order: each tet goes to its position in
+        // natinterp3d's visiting order
         const RowEntry x = ent[e];
         const int o = min(x.pos & 0xff, ncav - 1);  // a permutation of 0..ncav-1
-        ws.cav_tet[o] = x.tet;
-        ws.bmask[o] = (uint8_t)(x.bmask & 0xfu);
-        ws.ctv[o] = M.tv[x.tet];
-        ws.ftet[e] = x.tet;
-        ws.fpos[e] = (int8_t)o;
-    }
-    g.sync();
-    // natinterp3d's face cache (natural_insertionfree.c:233-253): a face
-    // shared with a cavity tet visited earlier returns that tet's copy, the
-    // mirror slot of the face in it; otherwise the tet's own slot
-    // (k_rows_order marked those faces; cfp is first read after the syncs of
-    // the boundary-face step)
-    for (int e = g.lane; e < ncav; e += G) {
-        const RowEntry x = ent[e];
-        const int o = ws.fpos[e];
-        const unsigned wd = (unsigned)x.nbr;
-        const unsigned mir = (x.bmask >> 8) & 0xffu;
-        const unsigned take = ((unsigned)x.pos >> 8) & 0xfu;
-        int fp[4];
+        const int4 p = M.tv[x.tet];
+        if (FULL && e < 32) {
+            first_o = o;
+            if (!GENERAL) terms = M.corner[16 * (size_t)x.tet + (((unsigned)x.pos >> 8) & 15u)];
+        }
+        unsigned slots = 0;
+        // most vertices get the slot of their hash, all four tried at once
+        int s[4];
 #pragma unroll
         for (int i = 0; i < 4; i++) {
-            const int jf = 3 - i;
-            const int n = (int8_t)((wd >> (8 * jf)) & 0xffu);
-            if (((take >> i) & 1u) && n >= 0 && n < ncav) {
-                const int jm = (mir >> (2 * jf)) & 3;
-                fp[i] = 4 * ws.ftet[n] + (3 - jm);
+            const int v = comp(p, i);
+            s[i] = (int)(mix_hash(v) & (unsigned)(W::VH - 1));
+            if (v < M.n) {
+                const int old = atomicCAS(&C.h.vh_key[s[i]], -1, v);
+                if (old != -1 && old != v) s[i] = -1;
             } else {
-                fp[i] = 4 * x.tet + i;
+                s[i] = 0x80 | (v - M.n);
             }
         }
-        ws.cfp[o] = make_int4(fp[0], fp[1], fp[2], fp[3]);
+#pragma unroll
+        for (int i = 0; i < 4; i++) slots |= ((unsigned)s[i] & 0xffu) << (8 * i);
+        if ((s[0] | s[1] | s[2] | s[3]) < 0) {
+#pragma unroll 1
+            for (int i = 0; i < 4; i++)
+                if (((slots >> (8 * i)) & 0xffu) == 0xffu) {
+                    const int t = hash_upsert(C.h.vh_key, W::VH, comp(p, i), vfull);
+                    slots ^= (0xffu ^ ((unsigned)t & 0xffu)) << (8 * i);
+                }
+        }
+        C.tet[o] = x.tet;
+        C.lid[o] = slots;
+        C.mask[o] = (uint8_t)((x.bmask & 0xfu) | (((unsigned)x.pos >> 4) & 0xf0u));
     }
-    auto face = [&](int k, int &c) {
-        c = k >> 2;
-        return ((ws.bmask[c] >> (k & 3)) & 1u) != 0u;
-    };
-    auto tet_fp = [&](int o, int &c, int (&fp)[4]) {
-        c = o;
-        const int4 f = ws.cfp[o];
-        fp[0] = f.x;
-        fp[1] = f.y;
-        fp[2] = f.z;
-        fp[3] = f.w;
-    };
-    auto tet_tv = [&](int c) { return ws.ctv[c]; };
-    return row_volumes<G, W, FULL>(M, q, ws, g, ncav, r, face, tet_fp, tet_tv);
+    if (g.any(vfull)) {
+        r.status = ST_CAPACITY;
+        return;
+    }
+    g.sync();
+
+    // ---- 3. boundary faces (visiting order, then face order) -----------------
+    int nbf = 0;
+#pragma unroll 1
+    for (int o0 = 0; o0 < ncav; o0 += 32) {
+        const int o = o0 + lane;
+        const unsigned m = o < ncav ? C.mask[o] & 15u : 0u;
+        const int end = nbf + scan_add(__popc(m), lane);
+        int b = end - __popc(m);
+#pragma unroll
+        for (int f = 0; f < 4; f++)
+            if ((m >> f) & 1u) {
+                if (b < W::BF) ws.bff[b] = 4 * o + f;
+                b++;
+            }
+        nbf = g.shfl(end, 31);
+    }
+    if (nbf > W::BF) {
+        r.status = GENERAL ? ST_CAPACITY : ST_GENERAL;
+        return;
+    }
+    r.nbf = nbf;
+    g.sync();
+#pragma unroll 1
+    for (int b = lane; b < nbf; b += 32) {
+        const int cf = ws.bff[b];
+        const unsigned ids = face_ids(C.lid[cf >> 2], cf & 3);
+        ws.fid[b] = ids;
+#pragma unroll
+        for (int j = 0; j < 3; j++) {
+            const int s = (ids >> (8 * j)) & 0xff;
+            if (s < 0x80) atomicMin(&C.h.vh_first[s], 3 * b + j);
+        }
+    }
+    g.sync();
+
+    // ids of the boundary faces' vertices; vh_first becomes the slot's id
+    int nnb = 0;
+#pragma unroll
+    for (int i = 0; i < W::VH; i += 32) {
+        const int s = i + lane;
+        const int k = C.h.vh_first[s];
+        const unsigned m = g.ballot(k != INT_MAX);
+        const int id = nnb + __popc(m & g.lt());
+        C.h.vh_first[s] = k == INT_MAX ? VOL_NO_ID : id;
+        if (k != INT_MAX && id < W::NBR) {
+            ws.nbr_vid[id] = C.h.vh_key[s];
+            ws.start[id] = k;
+            atomicOr(&C.firsts[k >> 5], 1u << (k & 31));
+        }
+        nnb += __popc(m);
+    }
+    if (nnb > W::NBR) {
+        r.status = ST_CAPACITY;
+        return;
+    }
+    if (!GENERAL && nnb > 32) {
+        r.status = ST_GENERAL;
+        return;
+    }
+    g.sync();
+    if (nnb == 0) return;
+
+    // the neighbour of each lane: its vertex and column (the order of first corners)
+#pragma unroll
+    for (int i = 0; i < IDS; i++) {
+        const int id = lane + 32 * i;
+        if (id < nnb) {
+            const int k = ws.start[id];
+            const int v = ws.nbr_vid[id];
+            sstore(ws.pos[id], vload(M, v));
+            out.vid[i] = v;
+            int c = __popc(C.firsts[k >> 5] & ((1u << (k & 31)) - 1u));
+#pragma unroll 1
+            for (int w = 0; w < k >> 5; w++) c += __popc(C.firsts[w]);
+            out.col[i] = c;
+        }
+    }
+    if (lane < 4) sstore(ws.pos[nnb + lane], vload(M, M.n + lane));
+
+    // hash slots to ids, and each id's sets of tets and faces
+    auto to_id = [&](unsigned s) { return s < 0x80u ? C.h.vh_first[s] : nnb + (int)(s & 3u); };
+    if constexpr (FULL) {
+#pragma unroll 1
+        for (int o = lane; o < ncav; o += 32) {
+            const unsigned w = C.lid[o];
+            unsigned ids = 0;
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                const int id = to_id((w >> (8 * i)) & 0xffu);
+                ids |= (unsigned)id << (8 * i);
+                if (id < nnb) atomicOr(reinterpret_cast<unsigned *>(&C.tm[id]) + (o >> 5), 1u << (o & 31));
+            }
+            C.lid[o] = ids;
+        }
+    }
+#pragma unroll 1
+    for (int b = lane; b < nbf; b += 32) {
+        const int cf = ws.bff[b];
+        const unsigned w = ws.fid[b];
+        unsigned ids = 0;
+#pragma unroll
+        for (int j = 0; j < 3; j++) {
+            const int id = to_id((w >> (8 * j)) & 0xffu);
+            ids |= (unsigned)id << (8 * j);
+            atomicOr(reinterpret_cast<unsigned *>(&ws.fm[FW * id]) + (b >> 5), 1u << (b & 31));
+        }
+        ws.fid[b] = ids;
+        ws.bff[b] = 4 * C.tet[cf >> 2] + 3 - (cf & 3);
+    }
+    g.sync();
+    if constexpr (!FULL) {
+        // the neighbours in column order, and each id's column
+#pragma unroll
+        for (int i = 0; i < IDS; i++)
+            if (lane + 32 * i < nnb) {
+                ws.nbr_vid[out.col[i]] = out.vid[i];
+                ws.start[lane + 32 * i] = out.col[i];
+            }
+        g.sync();
+        r.nnb = nnb;
+        return;
+    }
+
+    // where each neighbour's terms go: lane l adds up those of neighbour l (and l + 32)
+    int n[IDS], at[IDS];  // number and first place, cavity terms | face terms << 16
+    {
+        int base = 0;
+#pragma unroll
+        for (int i = 0; i < IDS; i++) {
+            const int id = lane + 32 * i;
+            n[i] = 0;
+            if (id < nnb) {
+                n[i] = __popcll(C.tm[id]);
+#pragma unroll
+                for (int w = 0; w < FW; w++) n[i] += __popcll(ws.fm[FW * id + w]) << 16;
+            }
+            at[i] = base + scan_add(n[i], lane);
+            base = g.shfl(at[i], 31);
+            at[i] -= n[i];
+            if (id < nnb) ws.start[id] = at[i];
+        }
+    }
+    g.sync();
+
+    // ---- 4. stolen volumes -----------------------------------------------------
+#pragma unroll 1
+    for (int e = lane; e < ncav; e += 32) {
+        int o = first_o;
+        if (e >= 32) o = min(ent[e].pos & 0xff, ncav - 1);
+        if (GENERAL || e >= 32) {
+            const int t = C.tet[o];
+            const unsigned m = C.mask[o] >> 4;
+            if (GENERAL && !M.corner)
+                terms = corner_terms_direct(M, t, m);
+            else
+                terms = M.corner[16 * (size_t)t + m];
+        }
+        const unsigned ids = C.lid[o];
+        const unsigned long long below = (1ull << o) - 1ull;
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const int id = (ids >> (8 * i)) & 0xff;
+            if (id < nnb)
+                C.term[(ws.start[id] & 0xffff) + __popcll(C.tm[id] & below)] =
+                    i == 0 ? terms.x : (i == 1 ? terms.y : (i == 2 ? terms.z : terms.w));
+        }
+    }
+    g.sync();
+#pragma unroll
+    for (int i = 0; i < IDS; i++) {
+        add_terms(out.a[i], C.term + (at[i] & 0xffff), n[i] & 0xffff);
+    }
+    g.sync();
+
+    // virtual-tet terms, query + boundary face (:681-719), a lane a face corner
+    bool general = false;  // !GENERAL: the row is not for this body
+    auto &V = ws.u.v;
+    using corner_t = typename W::corner_t;
+    const int ne = 3 * nbf;
+    const int S = nnb + 4;
+    using edge_t = typename W::edge_t;
+#pragma unroll 1
+    for (int i = lane; i < (S * S * (int)sizeof(edge_t) + 15) / 16; i += 32)
+        reinterpret_cast<uint4 *>(ws.u.pair)[i] = make_uint4(~0u, ~0u, ~0u, ~0u);
+    g.sync();
+#pragma unroll 1
+    for (int k = lane; k < ne; k += 32) {
+        const int b = k / 3, j = k - 3 * b;
+        const unsigned rot = __byte_perm(ws.fid[b], 0, j == 0 ? 0x3210u : (j == 1 ? 0x3021u : 0x3102u));
+        const unsigned u = rot & 0xffu, w = (rot >> 8) & 0xffu, x = rot >> 16;
+        ws.u.pair[u * S + w] = (edge_t)k;
+        // the faces of u before this one
+        int place = 0;
+        if (u < (unsigned)nnb) {
+            place = ws.start[u] >> 16;
+#pragma unroll
+            for (int i = 0; i < FW; i++) {
+                const unsigned long long mu = ws.fm[FW * u + i];
+                if (FW == 1 || b >> 6 == i)
+                    place += __popcll(mu & ((1ull << (b & 63)) - 1ull));
+                else if (b >> 6 > i)
+                    place += __popcll(mu);
+            }
+        }
+        ws.corner[k] = (corner_t)(u | w << 6 | x << 12) | (corner_t)place << (18 + W::EB);
+    }
+    g.sync();
+#pragma unroll 1
+    for (int k = lane; k < ne; k += 32) {
+        const corner_t cn = ws.corner[k];
+        const unsigned e = ws.u.pair[((unsigned)cn & 63) * S + (((unsigned)cn >> 12) & 63)];
+        ws.corner[k] = cn | (corner_t)(e & ((1u << W::EB) - 1u)) << 18;
+        if (!GENERAL) general |= e == W::NO_EDGE;
+    }
+    g.sync();
+#pragma unroll 1
+    for (int k = lane; k < ne; k += 32) {
+        const unsigned cn = (unsigned)ws.corner[k];
+        const int u = cn & 63;
+        if (u < nnb) {
+            const dv3 pu = sload(ws.pos[u]), pw = sload(ws.pos[(cn >> 6) & 63]);
+            bool flat = false;
+            const dv3 c = GENERAL ? tri_cc(pu, q, pw) : tri_cc_regular(pu, q, pw, flat);
+            general |= flat;
+            sstore(V.ec[k], vsub(c, pu));
+        }
+    }
+#pragma unroll 1
+    for (int b = lane; b < nbf; b += 32) {
+        const unsigned ids = ws.fid[b];
+        const dv3 pa = sload(ws.pos[ids & 0xff]), pb = sload(ws.pos[(ids >> 8) & 0xff]),
+                  pc = sload(ws.pos[ids >> 16]);
+        bool flat = false;
+        const dv3 c = GENERAL ? tet_cc(q, pa, pb, pc) : tet_cc_regular(q, pa, pb, pc, flat);
+        general |= flat;
+        sstore(V.ct[b], c);
+    }
+    if (!GENERAL && g.any(general)) {
+        r.status = ST_GENERAL;
+        return;
+    }
+    g.sync();
+#pragma unroll 1
+    for (int k = lane; k < ne; k += 32) {
+        const corner_t cn = ws.corner[k];
+        const int u = (unsigned)cn & 63;
+        if (u < nnb) {
+            const int b = k / 3;
+            constexpr unsigned NONE = (1u << W::EB) - 1u;
+            const unsigned e = (unsigned)(cn >> 18) & NONE;
+            const dv3 cf = cload(&M.fcc[ws.bff[b]]);
+            const dv3 pu = sload(ws.pos[u]), pw = sload(ws.pos[((unsigned)cn >> 6) & 63]),
+                      px = sload(ws.pos[((unsigned)cn >> 12) & 63]);
+            dv3 dac;
+            if (GENERAL && e == NONE)
+                dac = vsub(tri_cc(pu, q, px), pu);
+            else
+                dac = sload(V.ec[e]);
+            // subcell_volume(u, q, w, x, ct, cc(u, q, w), cc(u, q, x), cf)
+            const double sv = vdot(vsub(q, pu), vcross(vsub(pw, pu), vsub(px, pu)));
+            ws.fterm[(unsigned)(cn >> (18 + W::EB))] =
+                -subcell_from(sv, vsub(q, pw), vsub(q, px), vsub(pw, px), sload(V.ec[k]), dac, vsub(cf, pu),
+                              vsub(sload(V.ct[b]), pu));
+        }
+    }
+    g.sync();
+#pragma unroll
+    for (int i = 0; i < IDS; i++) add_terms(out.a[i], ws.fterm + (at[i] >> 16), n[i] >> 16);
+    r.nnb = nnb;
+}
+
+// ---- 5. normalisation: the lanes' stolen volumes to weights; r.nnb = 0 where
+// the row is empty.  The total is added up in column order.
+template <int G, class W, int IDS>
+__device__ __forceinline__ void split_weights(W &ws, const Grp<G> &g, RowInfo &r, RowLanes<IDS> &out) {
+    if (r.coincident || r.nnb == 0) return;
+    const int nnb = r.nnb;
+#pragma unroll
+    for (int i = 0; i < IDS; i++)
+        if (out.col[i] < nnb) ws.acc[out.col[i]] = out.a[i];
+    g.sync();
+    double total = 0.0;
+#pragma unroll 4
+    for (int s = 0; s < nnb; s++) total = fadd(total, ws.acc[s]);
+    if (!(total > 1e-30)) {
+        r.nnb = 0;
+        return;
+    }
+    const double inv = frcp(total);
+#pragma unroll
+    for (int i = 0; i < IDS; i++) out.a[i] = fmul(out.a[i], inv);
+    r.total = total;
 }
 
 }  // namespace nif
