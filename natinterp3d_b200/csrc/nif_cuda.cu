@@ -808,7 +808,9 @@ struct InterpSink {
 template <class QT, class VT, class GT>
 struct GradSink {
     static constexpr bool FULL = false;
-    // the dual-number face gradient holds many FP64 values: fewer, larger threads
+    static constexpr int VOL_BLOCKS = 7;  // resident blocks of k_rows_volume
+    // of k_rows_fast: the dual-number face gradient holds many FP64 values, so
+    // fewer, larger threads
 #ifndef NIF_GRAD_MINB
 #define NIF_GRAD_MINB 4
 #endif
@@ -821,10 +823,163 @@ struct GradSink {
     QT *__restrict__ gq;             // [M][3]
     int D;
 
+    // Split rows.  Only the part of the query's new cell that borders neighbour
+    // k moves s_k with the query: its facet, the polygon through the
+    // circumcentres of the tets (q, face) around k, on the bisector of q and k.
+    // With area A_k and centroid c_k, ds_k/dq = A_k (c_k - q) / |k - q|, which
+    // is what the derivatives of the virtual-tet terms add up to where the
+    // faces close around k (face by face they differ by terms that two faces
+    // with a common edge cancel).  A corner u of a face, with the edge u -> w
+    // to the next vertex and the other face of that edge, is one triangle of
+    // u's facet: about 40 operations instead of the 3,000 of the dual numbers,
+    // so that the pass is bound by the same row setup as the weights (1M rows,
+    // 200k keys, 16 columns: 10.1 ms with dual numbers, 2.6 ms).
+    // Returns false where that does not hold: faces that do not close or that
+    // differ in orientation, or tets and triangles near natinterp3d's
+    // degeneracy thresholds; k_rows_general takes those rows, with the dual
+    // numbers where it must.
     template <int G, class W, int IDS>
-    __device__ __forceinline__ void emit_lanes(int64_t i, W &ws, const Grp<G> &g, RowInfo &r,
-                                               RowLanes<IDS> &, const MeshView &M, dv3 q) {
-        emit<G>(i, r.nnb, ws, g, false, M, q, r);
+    __device__ __forceinline__ bool emit_lanes(int64_t i, W &ws, const Grp<G> &g, RowInfo &r,
+                                               RowLanes<IDS> &L, const MeshView &M, dv3 q) {
+        constexpr bool GENERAL = IDS > 1;
+        const int nnb = r.nnb, nbf = r.nbf;
+        double gx = 0.0, gy = 0.0, gz = 0.0;
+        const int64_t r0 = rowptr[i];
+        const double S = total[i];
+        if (nnb > 0 && !r.coincident && S > 1e-30 && rowptr[i + 1] - r0 == nnb) {
+            // each neighbour's dL/ds, the lanes' own
+            const GT *go = gout + i * (int64_t)D;
+            double ck[IDS], gbar = 0.0;
+#pragma unroll
+            for (int k = 0; k < IDS; k++) {
+                ck[k] = 0.0;
+                if (L.col[k] < nnb) {
+                    const VT *vr = values + (int64_t)L.vid[k] * D;
+                    double a = 0.0;
+#pragma unroll 4
+                    for (int d = 0; d < D; d++) a = __fma_rn((double)go[d], (double)vr[d], a);
+                    ck[k] = a;
+                    ws.fterm[L.col[k]] = a * w[r0 + L.col[k]];
+                }
+            }
+            // summed by column: a neighbour's lane may differ from call to call
+            g.sync();
+#pragma unroll
+            for (int k = 0; k < IDS; k++)
+                if (g.lane + 32 * k < nnb) gbar += ws.fterm[g.lane + 32 * k];
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) gbar += g.shfl_xor_d(gbar, o);
+            g.sync();
+            const double inv_total = 1.0 / S;
+#pragma unroll
+            for (int k = 0; k < IDS; k++) {
+                ck[k] = (ck[k] - gbar) * inv_total;
+                if (L.col[k] < nnb) ws.fterm[g.lane + 32 * k] = ck[k];
+            }
+            // circumcentres of (q, face) relative to q, and the faces' edges
+            using edge_t = typename W::edge_t;
+            const int n4 = nnb + 4;
+            for (int k = g.lane; k < (n4 * n4 * (int)sizeof(edge_t) + 15) / 16; k += 32)
+                reinterpret_cast<uint4 *>(ws.u.pair)[k] = make_uint4(~0u, ~0u, ~0u, ~0u);
+            static_assert(sizeof(ws.u.pair) <= sizeof(ws.u.v.ec), "beside the circumcentres");
+            g.sync();
+            bool odd = false, plus = false, minus = false;
+#pragma unroll 1
+            for (int b = g.lane; b < nbf; b += 32) {
+                const unsigned ids = ws.fid[b];
+                const int ia = ids & 0xff, ib = (ids >> 8) & 0xff, ic = ids >> 16;
+                ws.u.pair[ia * n4 + ib] = (edge_t)b;
+                ws.u.pair[ib * n4 + ic] = (edge_t)b;
+                ws.u.pair[ic * n4 + ia] = (edge_t)b;
+                const dv3 ba = vsub(sload(ws.pos[ia]), q), ca = vsub(sload(ws.pos[ib]), q),
+                          da = vsub(sload(ws.pos[ic]), q);
+                const dv3 x1 = vcross(ba, ca), x2 = vcross(da, ba), x3 = vcross(ca, da);
+                const double lb = vdot(ba, ba), lc = vdot(ca, ca), ld = vdot(da, da);
+                const double den = 2.0 * vdot(ba, x3);
+                // natinterp3d's formulas change where |den| < 1e-30, or where a
+                // triangle of the tet has (2 area)^2 < 1e-30; den^2 is at most
+                // 4 (2 area)^2 times the longest edge squared, itself at most
+                // 4 times the longest of q's
+                odd |= !(den * den > 1.7e-29 * fmax(lb, fmax(lc, ld))) || !(fabs(den) >= 1e-30);
+                plus |= den > 0.0;
+                minus |= den < 0.0;
+                const double inv = frcp(den);
+                ws.u.v.ct[b][0] = (x3.x * lb + (x1.x * ld + x2.x * lc)) * inv;
+                ws.u.v.ct[b][1] = (x3.y * lb + (x1.y * ld + x2.y * lc)) * inv;
+                ws.u.v.ct[b][2] = (x3.z * lb + (x1.z * ld + x2.z * lc)) * inv;
+            }
+            const bool up = g.any(plus);
+            odd = g.any(odd) || (up && g.any(minus));
+            g.sync();
+            if (!odd) {
+                // dL/ds_u over 6 |u - q|^2, signed by the faces' orientation
+#pragma unroll
+                for (int k = 0; k < IDS; k++)
+                    if (L.col[k] < nnb) {
+                        const dv3 ru = vsub(sload(ws.pos[g.lane + 32 * k]), q);
+                        const double f = ck[k] / (6.0 * vdot(ru, ru));
+                        ws.fterm[g.lane + 32 * k] = up ? f : -f;
+                    }
+                g.sync();
+#pragma unroll 1
+                for (int k = g.lane; k < 3 * nbf; k += 32) {
+                    const int b = k / 3, j = k - 3 * b;
+                    const unsigned rot =
+                        __byte_perm(ws.fid[b], 0, j == 0 ? 0x3210u : (j == 1 ? 0x3021u : 0x3102u));
+                    const int u = rot & 0xff;
+                    const unsigned b2 = ws.u.pair[((rot >> 8) & 0xff) * n4 + u];
+                    if (u >= nnb) continue;
+                    if (b2 == W::NO_EDGE) {
+                        odd = true;
+                        continue;
+                    }
+                    const dv3 A = sload(ws.u.v.ct[b]), B = sload(ws.u.v.ct[b2]);
+                    const dv3 ru = vsub(sload(ws.pos[u]), q);
+                    const double f = ws.fterm[u] * vdot(vcross(B, A), ru);
+                    gx = __fma_rn(f, A.x + B.x + 0.5 * ru.x, gx);
+                    gy = __fma_rn(f, A.y + B.y + 0.5 * ru.y, gy);
+                    gz = __fma_rn(f, A.z + B.z + 0.5 * ru.z, gz);
+                }
+                odd = g.any(odd);
+            }
+            if (odd) {
+                if (!GENERAL) return false;
+                gx = gy = gz = 0.0;
+                g.sync();
+#pragma unroll
+                for (int k = 0; k < IDS; k++)
+                    if (L.col[k] < nnb) ws.fterm[g.lane + 32 * k] = ck[k];
+                g.sync();
+#pragma unroll 1
+                for (int b = g.lane; b < (GENERAL ? nbf : 0); b += 32) {
+                    const unsigned ids = ws.fid[b];
+                    const int ia = ids & 0xff, ib = (ids >> 8) & 0xff, ic = ids >> 16;
+                    // virtual terms enter the stolen volumes with a minus sign
+                    const double c0 = ia < nnb ? -ws.fterm[ia] : 0.0;
+                    const double c1 = ib < nnb ? -ws.fterm[ib] : 0.0;
+                    const double c2 = ic < nnb ? -ws.fterm[ic] : 0.0;
+                    if (c0 == 0.0 && c1 == 0.0 && c2 == 0.0) continue;
+                    const dv3 gf = virtual_face_grad(q, sload(ws.pos[ia]), sload(ws.pos[ib]),
+                                                     sload(ws.pos[ic]), cload(&M.fcc[ws.bff[b]]), c0, c1, c2);
+                    gx += gf.x;
+                    gy += gf.y;
+                    gz += gf.z;
+                }
+            }
+#pragma unroll
+            for (int o = G / 2; o > 0; o >>= 1) {
+                gx += g.shfl_xor_d(gx, o);
+                gy += g.shfl_xor_d(gy, o);
+                gz += g.shfl_xor_d(gz, o);
+            }
+            g.sync();
+        }
+        if (g.lane == 0) {
+            gq[3 * i] = (QT)gx;
+            gq[3 * i + 1] = (QT)gy;
+            gq[3 * i + 2] = (QT)gz;
+        }
+        return true;
     }
 
     template <int G, class W>
@@ -851,35 +1006,23 @@ struct GradSink {
             for (int s = g.lane; s < nnb; s += G) ck[s] = (ck[s] - gbar) * inv_total;
             g.sync();
             for (int b = g.lane; b < r.nbf; b += G) {
-                dv3 pa, pb, pc;
-                int sa, sb, sc, ffi;
-                if constexpr (W::SPLIT) {
-                    const unsigned ids = ws.fid[b];
-                    sa = ids & 0xff, sb = (ids >> 8) & 0xff, sc = ids >> 16;
-                    pa = sload(ws.pos[sa]), pb = sload(ws.pos[sb]), pc = sload(ws.pos[sc]);
-                    sa = sa < nnb ? ws.start[sa] : -1, sb = sb < nnb ? ws.start[sb] : -1,
-                    sc = sc < nnb ? ws.start[sc] : -1;
-                    ffi = ws.bff[b];
-                } else {
-                    const int cf = ws.bface[b];
-                    const int f = cf & 3;
-                    const int tt = ws.cav_tet[cf >> 2];
-                    const int4 p = M.tv[tt];
-                    const int va = comp(p, face_vslot(f, 0));
-                    const int vb = comp(p, face_vslot(f, 1));
-                    const int vc = comp(p, face_vslot(f, 2));
-                    sa = va < M.n ? neighbour_slot(ws, va) : -1;
-                    sb = vb < M.n ? neighbour_slot(ws, vb) : -1;
-                    sc = vc < M.n ? neighbour_slot(ws, vc) : -1;
-                    pa = vload(M, va), pb = vload(M, vb), pc = vload(M, vc);
-                    ffi = 4 * tt + (3 - f);
-                }
+                const int cf = ws.bface[b];
+                const int f = cf & 3;
+                const int tt = ws.cav_tet[cf >> 2];
+                const int4 p = M.tv[tt];
+                const int va = comp(p, face_vslot(f, 0));
+                const int vb = comp(p, face_vslot(f, 1));
+                const int vc = comp(p, face_vslot(f, 2));
+                const int sa = va < M.n ? neighbour_slot(ws, va) : -1;
+                const int sb = vb < M.n ? neighbour_slot(ws, vb) : -1;
+                const int sc = vc < M.n ? neighbour_slot(ws, vc) : -1;
                 // virtual terms enter the stolen volumes with a minus sign
                 const double c0 = sa >= 0 ? -ck[sa] : 0.0;
                 const double c1 = sb >= 0 ? -ck[sb] : 0.0;
                 const double c2 = sc >= 0 ? -ck[sc] : 0.0;
                 if (c0 == 0.0 && c1 == 0.0 && c2 == 0.0) continue;
-                const dv3 gf = virtual_face_grad(q, pa, pb, pc, cload(&M.fcc[ffi]), c0, c1, c2);
+                const dv3 gf = virtual_face_grad(q, vload(M, va), vload(M, vb), vload(M, vc),
+                                                 cload(&M.fcc[4 * (size_t)tt + (3 - f)]), c0, c1, c2);
                 gx += gf.x;
                 gy += gf.y;
                 gz += gf.z;
@@ -1470,15 +1613,17 @@ __global__ void __launch_bounds__(32 * ORD_WARPS) k_rows_order(int64_t nrows, in
     }
 }
 
-// what the split row kernels do with a finished row i
+// what the split row kernels do with a finished row i; false: the row is for
+// k_rows_general
 template <class W, class Sink, int IDS>
-__device__ __forceinline__ void finish_row(int64_t i, RowInfo &r, RowLanes<IDS> &L, const MeshView &M,
+__device__ __forceinline__ bool finish_row(int64_t i, RowInfo &r, RowLanes<IDS> &L, const MeshView &M,
                                            const dv3 q, W &ws, const Grp<FAST_G> &g, Sink &sink,
                                            const LargeQueue &lq, DevSummary *sum) {
     if (r.status == ST_CAPACITY) {
         if (g.lane == 0) lq.list[atomicAdd(&sum->large_count, 1)] = (int)i;
-        return;
+        return true;
     }
+    if (r.status == ST_GENERAL) return false;
     if (r.status != ST_OK) {
         r.nnb = 0;
         if (g.lane == 0) {
@@ -1487,10 +1632,12 @@ __device__ __forceinline__ void finish_row(int64_t i, RowInfo &r, RowLanes<IDS> 
         }
     }
     record<FAST_G>(sum, r, g.lane);
-    if constexpr (Sink::FULL)
+    if constexpr (Sink::FULL) {
         sink.template emit_lanes<FAST_G>(i, ws, g, r, L);
-    else
-        sink.template emit_lanes<FAST_G>(i, ws, g, r, L, M, q);
+        return true;
+    } else {
+        return sink.template emit_lanes<FAST_G>(i, ws, g, r, L, M, q);
+    }
 }
 
 // Rows that split_row_body gives up on (ST_GENERAL) are queued in `gen`, by
@@ -1531,11 +1678,8 @@ __global__ void __launch_bounds__(FAST_BLOCK, OCC)
             if (h.state == RS_OK)
                 split_row_body<G, VolWS, Sink::FULL, false>(M, q, ws, g, h, ents + s * REC_CAV, r, L);
             if (h.state == RS_WALK) r.status = ST_WALK;
-            if (r.status == ST_GENERAL) {
-                if (g.lane == 0) gen[atomicAdd(&sum->general_count, 1)] = (int)s;
-            } else {
-                finish_row(i, r, L, M, q, ws, g, sink, lq, sum);
-            }
+            if (!finish_row(i, r, L, M, q, ws, g, sink, lq, sum) && g.lane == 0)
+                gen[atomicAdd(&sum->general_count, 1)] = (int)s;
         }
         g.sync();
         s += tile <= 0 ? ng : 1;
@@ -2121,7 +2265,7 @@ constexpr int sink_occ() {
     if constexpr (Sink::FULL)
         return OCC;
     else
-        return Sink::MIN_BLOCKS;
+        return Sink::VOL_BLOCKS;
 }
 
 // k_rows_general over the rows that the launch before queued in `gen`
@@ -3155,7 +3299,7 @@ void grad_records_typed(const nif_dmesh *m, const void *q, int64_t M, const Cent
     cudaMemsetAsync(R.sum, 0, sizeof(DevSummary), st);
     for (int64_t c0 = 0; c0 < M; c0 += REC_CHUNK) {
         const int64_t n = min((int64_t)REC_CHUNK, M - c0);
-        launch_rows(k_rows_volume<QT, OneMesh, Sink, Sink::MIN_BLOCKS>, lc, n, GPB * sizeof(VolWS),
+        launch_rows(k_rows_volume<QT, OneMesh, Sink, Sink::VOL_BLOCKS>, lc, n, GPB * sizeof(VolWS),
                     R.counter, st, rows, Q, L.order + c0, n, (const RowHead *)(R.heads + c0),
                     (const RowEntry *)(R.ents + c0 * REC_CAV), L.gen, sink, LargeQueue{R.requeue}, R.sum);
         launch_general(lc, rows, Q, n, L.order + c0, R.heads + c0, R.ents + c0 * REC_CAV, L.gen, sink,
