@@ -79,7 +79,7 @@ constexpr int REC_CHUNK = NIF_REC_CHUNK;
 // workspace holds 42 boundary faces (2M queries, 200k keys: 7.1 ms at 7
 // blocks, 7.4 ms at 6, 10.1 ms at 8 with 64 registers and 34 faces).
 #ifndef NIF_CAV_OCC
-#define NIF_CAV_OCC 10
+#define NIF_CAV_OCC 8
 #endif
 #ifndef NIF_VOL_OCC
 #define NIF_VOL_OCC 0
@@ -157,7 +157,8 @@ __global__ void k_prep_geometry(MeshView M, uint32_t *__restrict__ tinfo, d4 *__
         // bit 2 (the exact sign) equals it unless k_prep_exact_orient corrects it
         const double o = orient_fast(P0, P1, P2, P3);
         uint32_t info = o > 0 ? 5u : 0u;
-        if (orient_uncertain(P0, P1, P2, P3, o)) {
+        const bool unc = orient_uncertain(P0, P1, P2, P3, o);
+        if (unc) {
             info |= 2u;
             atomicAdd(&bad[1], 1);
         }
@@ -178,7 +179,7 @@ __global__ void k_prep_geometry(MeshView M, uint32_t *__restrict__ tinfo, d4 *__
         }
         tinfo[t] = info;
         const dv3 c = tet_cc(P0, P1, P2, P3);
-        tcc[t] = d4{c.x, c.y, c.z, 0.0};
+        tcc[t] = d4{c.x, c.y, c.z, prep_sphere(c, P0, P1, P2, P3, o, unc)};
         // face opposite p[i], remaining vertices in ascending slot order
         // (natural_insertionfree.c:649-652)
         const dv3 f0 = tri_cc(P1, P2, P3);
@@ -1387,8 +1388,11 @@ __global__ void __launch_bounds__(FAST_BLOCK, OCC) k_rows_fast(MeshView M, const
 // the row kernels take them; located[i] = the tet, -1 outside the
 // super-simplex, -2 a walk that hit its step limit, -3 (PM_FILTER) a walk
 // test the error bound cannot certify (the large kernel resolves the row).
+#ifndef NIF_LOC_OCC
+#define NIF_LOC_OCC 12
+#endif
 template <class QT, class Rows, int PM = PM_PLAIN>
-__global__ void __launch_bounds__(FAST_BLOCK) k_locate(const __grid_constant__ Rows rows,
+__global__ void __launch_bounds__(FAST_BLOCK, NIF_LOC_OCC) k_locate(const __grid_constant__ Rows rows,
                                                        const QT *__restrict__ Q,
                                                        const int *__restrict__ order, int64_t nrows,
                                                        int *__restrict__ located, DevSummary *sum,

@@ -81,7 +81,7 @@ struct MeshView {
     const uint32_t *__restrict__ tinfo;// [nt] bit0: orient3dfast(p0..p3) > 0; bit1: that sign is
                                        // uncertain; bit2: exact orient3d(p0..p3) > 0;
                                        // bits 8+2j: mirror slot of face j
-    const d4 *__restrict__ tcc;        // [nt] tet circumcentre
+    const d4 *__restrict__ tcc;        // [nt] tet circumcentre; w: see sphere_side
     const d4 *__restrict__ fcc;        // [nt*4] circumcentre of the face opposite p[i]
     const d4 *__restrict__ corner;     // [nt*16] corner terms (corner_term), or null
     // Tet centroids, (p0 + p1 + p2 + p3) / 4 per axis as natinterp3d's
@@ -453,6 +453,51 @@ __device__ int grid_nearest(const MeshView &M, const dv3 q) {
     return -1;
 }
 
+// Which side of tet t's circumsphere q lies on, from the cached circumcentre c
+// and squared radius w: 1 inside, -1 outside, 0 where this does not decide.  A
+// decision has the sign of natinterp3d's inspherefast and lies outside its
+// error bound, because prep_sphere gives only those tets a radius for which
+//   6V |d2 - w| > 2 E  for |d2 - w| > SPHERE_REL w and d2 < SPHERE_FAR w,
+// d2 = |q - c|^2, E the static error bound of inspherefast; the others have
+// w = NaN, which decides nothing.  Ten FP64 operations on one 32-byte record
+// for some 80 on four vertices behind the tet's vertex record.
+constexpr double SPHERE_REL = 1e-6, SPHERE_FAR = 1e4;
+__device__ __forceinline__ int sphere_side(const d4 &c, const dv3 &q) {
+    const double x = q.x - c.x, y = q.y - c.y, z = q.z - c.z;
+    const double d2 = x * x + y * y + z * z;
+    const double f = d2 - c.w;
+    if (!(fabs(f) > SPHERE_REL * c.w && d2 < SPHERE_FAR * c.w)) return 0;
+    return f < 0.0 ? 1 : -1;
+}
+
+// The w of sphere_side for a tet with circumcentre c and orientation
+// determinant o (6V up to its error), NaN where it cannot be relied on.
+//
+// With R the radius, s >= every |v_i - q| and V the volume, the exact insphere
+// determinant is 6V (|q - C|^2 - R^2), C and R exact, and inspherefast's error
+// is at most E <= 24 (16 + 224 eps) eps s^5 < 4.3e-14 s^5 (its permanent: four
+// lifts of at most s^2 times six products of at most s^3).  f(q) = |q - c|^2 - w
+// and the exact |q - C|^2 - R^2 differ by an affine function that is f(v_i) at
+// the vertices: by at most rho = max |f(v_i)| times the sum of |barycentric
+// coordinates|, each at most s^3 / 6V.  Evaluating f rounds by less than
+// 8 eps (d2 + w).  So a decision is right, and certified, when
+//   |f| > 8 eps (d2 + w) + (4 rho s^3 + 8.6e-14 s^5) / 6V.
+// For d2 <= 4 w, s <= 3.01 R, the right side is below
+// 5e-15 w + (110 rho R^3 + 2.2e-11 R^5) / 6V, which is held to SPHERE_REL w / 2.
+// For 4 w < d2 < SPHERE_FAR w, s <= 1.51 d and |f| > 0.75 d2, and with those
+// limits on rho and 1 / 6V the right side is below 2e-15 d2 +
+// (14 rho + 6.8e-13 d2) d^3 / 6V < 0.1 d2.
+__device__ __forceinline__ double prep_sphere(const dv3 &c, const dv3 &p0, const dv3 &p1, const dv3 &p2,
+                                              const dv3 &p3, double o, bool uncertain) {
+    auto dist2 = [&](const dv3 &p) { return vdot(vsub(p, c), vsub(p, c)); };
+    const double w = dist2(p0);
+    const double rho = fmax(fmax(fabs(dist2(p1) - w), fabs(dist2(p2) - w)), fabs(dist2(p3) - w)) + 4e-15 * w;
+    const double r = sqrt(w), v6 = 0.9 * fabs(o);
+    const bool ok = !uncertain && w > 1e-60 && w < 1e60 &&
+                    110.0 * rho * r * w + 2.2e-11 * r * w * w <= 0.4e-6 * w * v6;
+    return ok ? w : NAN;
+}
+
 // Per-group scratch.  The first union member is live during the cavity
 // search, the second only during the single-lane replay of natinterp3d's
 // visiting order.  Index types are the narrowest that hold each capacity.
@@ -489,6 +534,7 @@ struct Workspace {
     CavT pos[CAV_];              // inverse of order
     uint16_t bface[BF_];         // (cavity index << 2) | face
     int16_t vh_slot[VH_];
+    alignas(16) int4 wave[G_];   // neighbours of the flood wave's cavity tets
 };
 
 // Workspaces of the split row (k_rows_cavity, then k_rows_volume): the same
@@ -514,8 +560,7 @@ struct CavWorkspace {
     } u;
     int cav_tet[CAV_];
     alignas(4) CavT cav_nbr[4 * CAV_];
-    CavT order[CAV_];
-    CavT pos[CAV_];
+    alignas(16) int4 wave[G_];  // neighbours of the wave's cavity tets
 };
 
 // Workspace of the split row's volume phase (split_row): room for BF boundary
@@ -584,11 +629,9 @@ struct alignas(16) VolWorkspace {
 
 // One row between k_rows_cavity, k_rows_order and k_rows_volume: a header
 // and, per cavity tet in the flood's order, the tet, which of its faces bound
-// the cavity (bits 0-3) and the mirror slots of its faces (bits 8-15, the
-// mesh's tinfo bits 8-15), the cavity indices of its four neighbours (four
-// signed bytes, -1 outside the cavity); k_rows_order adds the tet's position
-// in natinterp3d's visiting order, from which k_rows_volume derives the fcc[]
-// indices of its faces' circumcentres as natinterp3d's face cache returns them.
+// the cavity (bits 0-3) and the cavity indices of its four neighbours (four
+// signed bytes, -1 outside the cavity); k_rows_order adds the tet's position in
+// natinterp3d's visiting order and which of its faces take a neighbour's copy.
 constexpr int REC_CAV = 48;  // cavity tets a record holds (larger cavities take the large kernel)
 constexpr int RS_OK = 0, RS_OUTSIDE = 1, RS_WALK = 2, RS_QUEUED = 3;
 struct __align__(16) RowHead {
@@ -599,7 +642,7 @@ struct __align__(16) RowHead {
 };
 struct __align__(16) RowEntry {
     int tet;
-    unsigned bmask;  // boundary faces | mirror slots << 8
+    unsigned bmask;  // boundary faces
     int nbr;         // cavity indices of neighbours 0..3, one signed byte each
     int pos;         // position in natinterp3d's visiting order (bits 0-7); bit 8 + i: face
                      // 3 - i takes the copy of the neighbour visited earlier
@@ -870,10 +913,11 @@ __device__ int flood_replay(const MeshView &M, const dv3 q, W &ws, const Grp<G> 
     static_assert(sizeof(slot_t) == sizeof(cav_t), "nsl aliases cav_nbr");
     constexpr int NO_TET = -2;
     slot_t *nsl = reinterpret_cast<slot_t *>(ws.cav_nbr);
-    for (int i = g.lane; i < W::HS; i += G) {
-        ws.u.a.hkey[i] = -1;
-        ws.u.a.hval[i] = (cav_t)-1;
-    }
+    static_assert(offsetof(decltype(ws.u.a), hval) == sizeof(ws.u.a.hkey) &&
+                      (sizeof(ws.u.a.hkey) + sizeof(ws.u.a.hval)) % 16 == 0,
+                  "one run of -1s");
+    for (int i = g.lane; i < (int)((sizeof(ws.u.a.hkey) + sizeof(ws.u.a.hval)) / 16); i += G)
+        reinterpret_cast<int4 *>(ws.u.a.hkey)[i] = make_int4(-1, -1, -1, -1);
     g.sync();
     int none_slot = 0;
     if (g.lane == 0) {
@@ -915,25 +959,34 @@ __device__ int flood_replay(const MeshView &M, const dv3 q, W &ws, const Grp<G> 
     while (!overflow && qhead < qtail) {
         const int n = min(G, qtail - qhead);
         int slot = -1, tt = -1;
-        bool inc = false, unc = false;
+        bool inc = false, unc = false, open = false;
+        int4 nb4 = make_int4(-1, -1, -1, -1);
         dv3 ia{0.0, 0.0, 0.0}, ib = ia, ic = ia, id = ia;
-        double sv = 0.0;
         if (g.lane < n) {
             slot = ws.u.a.queue[qhead + g.lane];
             tt = ws.u.a.hkey[slot];
-            const int4 p = M.tv[tt];
-            const dv3 a = vload(M, p.x), b = vload(M, p.y);
-            ic = vload(M, p.z);
-            id = vload(M, p.w);
-            // insphere argument order fixed by the tet's orientation
-            // (natural_insertionfree.c:511-515); PRED_EXACT uses the exact one
-            const uint32_t info = M.tinfo[tt];
-            const bool pos = (info & ((PM != PM_PLAIN && M.pmode == PRED_EXACT) ? 4u : 1u)) != 0;
-            ia = pos ? a : b;
-            ib = pos ? b : a;
-            sv = insphere_fast(ia, ib, ic, id, q);
-            inc = sv > 0;
-            if (filt) unc = insphere_uncertain(ia, ib, ic, id, q, sv);
+            nb4 = M.tn[tt];  // with the sphere: no second trip for the tets inside
+            const int side = sphere_side(M.tcc[tt], q);
+            inc = side > 0;
+            open = side == 0;
+        }
+        // tests that the cached sphere does not decide: the determinant itself
+        if (g.any(open)) {
+            if (open) {
+                const int4 p = M.tv[tt];
+                const dv3 a = vload(M, p.x), b = vload(M, p.y);
+                ic = vload(M, p.z);
+                id = vload(M, p.w);
+                // insphere argument order fixed by the tet's orientation
+                // (natural_insertionfree.c:511-515); PRED_EXACT uses the exact one
+                const uint32_t info = M.tinfo[tt];
+                const bool pos = (info & ((PM != PM_PLAIN && M.pmode == PRED_EXACT) ? 4u : 1u)) != 0;
+                ia = pos ? a : b;
+                ib = pos ? b : a;
+                const double sv = insphere_fast(ia, ib, ic, id, q);
+                inc = sv > 0;
+                if (filt) unc = insphere_uncertain(ia, ib, ic, id, q, sv);
+            }
         }
         if constexpr (PM == PM_FILTER) {
             if (g.any(unc)) {
@@ -954,8 +1007,8 @@ __device__ int flood_replay(const MeshView &M, const dv3 q, W &ws, const Grp<G> 
         if (g.lane < n) ws.u.a.hval[slot] = (cav_t)(inc ? ci : -1);
         if (inc && ci < W::CAV) {
             ws.cav_tet[ci] = tt;
-            // the volume phase reads this tet's cached circumcentres
-            prefetch_l2(&M.tcc[tt]);
+            ws.wave[ci - ncav] = nb4;
+            // the volume phase reads this tet's face circumcentres
             prefetch_l2(&M.fcc[4 * (size_t)tt]);
         }
         const int nnew = __popc(cm);
@@ -972,7 +1025,7 @@ __device__ int flood_replay(const MeshView &M, const dv3 q, W &ws, const Grp<G> 
             int ns = -1;
             bool full = false, fresh = false;
             if (k < 4 * nnew) {
-                const int nb = comp(M.tn[ws.cav_tet[base + (k >> 2)]], k & 3);
+                const int nb = reinterpret_cast<const int *>(ws.wave)[k];
                 int sl = none_slot;
                 if (nb >= 0) sl = hash_insert(ws.u.a.hkey, W::HS, nb, fresh, full);
                 if (fresh) ns = sl;
@@ -1382,9 +1435,7 @@ __device__ int cavity_record(const MeshView &M, const dv3 q, W &ws, const Grp<G>
     head.ncav = ncav;
     for (int c = g.lane; c < ncav; c += G) {
         const int tt = ws.cav_tet[c];
-        unsigned bm = (M.tinfo[tt] >> 8) & 0xffu;
-        bm <<= 8;
-        unsigned nb = 0;
+        unsigned bm = 0, nb = 0;
 #pragma unroll
         for (int f = 0; f < 4; f++) {
             const int nc = ws.cav_nbr[4 * c + f];
