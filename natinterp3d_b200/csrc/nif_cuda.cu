@@ -105,12 +105,17 @@ struct DevSummary {
     int large_count;  // rows queued for the large kernel
     int refill_count; // get_weights: fast-kernel rows longer than ROW_STAGE
     int wide_count;   // split rows whose cavity exceeds a record (the fused kernel takes them)
+    // work-item counters of the tiled row kernels (WORK_*), zero at a call's
+    // start like the rest; k_rows_order clears those of the next chunk
+    unsigned long long work[4];
     int general_count; // rows of the current chunk for k_rows_general
     int reserved;
     // predicate evaluations the filter could not certify / whose decision the
     // exact sign changes (PRED_AUDIT and PRED_EXACT meshes)
     unsigned long long orient_unc, orient_flip, insphere_unc, insphere_flip;
 };
+
+enum { WORK_LOCATE = 0, WORK_FUSED = 1, WORK_CAVITY = 2, WORK_VOLUME = 3 };
 
 // ---------------------------------------------------------------------------
 // resident mesh preparation
@@ -458,6 +463,12 @@ __global__ void k_scatter(const int *__restrict__ bucket, int64_t M, int *__rest
         const int pos = atomicAdd(&cursor[bucket[i]], 1);
         order[pos] = (int)i;
     }
+}
+
+__global__ void k_identity(int64_t M, int *__restrict__ order) {
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < M;
+         i += (int64_t)gridDim.x * blockDim.x)
+        order[i] = (int)i;
 }
 
 // ---------------------------------------------------------------------------
@@ -1341,6 +1352,7 @@ __global__ void __launch_bounds__(FAST_BLOCK, OCC) k_rows_fast(MeshView M, const
                                                           DevSummary *sum, int tile,
                                                           unsigned long long *counter) {
     extern __shared__ __align__(16) unsigned char smem[];
+    asm volatile("griddepcontrol.launch_dependents;");  // k_rows_volume beside the few wide rows
     // a row count known only on the device (a queue's length) bounds nrows
     if (nrows_dev) nrows = min(nrows, (int64_t)*nrows_dev);
     constexpr int G = FAST_G;
@@ -1519,7 +1531,10 @@ struct OrderWS {
 
 __global__ void __launch_bounds__(32 * ORD_WARPS) k_rows_order(int64_t nrows, int per, const RowHead *__restrict__ heads,
                                                                RowEntry *__restrict__ ents, DevSummary *sum) {
-    if (blockIdx.x == 0 && threadIdx.x == 0) sum->general_count = 0;  // k_rows_volume's queue, per chunk
+    if (blockIdx.x == 0 && threadIdx.x == 0) {  // k_rows_volume's queue, per chunk, and the counters
+        sum->general_count = 0;
+        sum->work[WORK_CAVITY] = sum->work[WORK_VOLUME] = 0ull;
+    }
     extern __shared__ __align__(16) unsigned char smem[];
     OrderWS &w = reinterpret_cast<OrderWS *>(smem)[threadIdx.x >> 5];
     const int lane = threadIdx.x & 31;
@@ -1688,6 +1703,7 @@ __global__ void __launch_bounds__(FAST_BLOCK, OCC)
         g.sync();
         s += tile <= 0 ? ng : 1;
     }
+    asm volatile("griddepcontrol.wait;" ::: "memory");  // the launch this one may run beside
 }
 
 // The rows k_rows_volume queued (about 2 % on random keys; all of them where
@@ -1969,7 +1985,7 @@ int blocks_for(int64_t n, int threads, int cap = 148 * 32) {
 // query workspace layout
 struct QueryLayout {
     DevSummary *sum;
-    unsigned long long *counter;  // work-item counter of the tiled row schedule
+    unsigned long long *counter;  // work-item counter of the fill pass's rows
     int bits_cap;                 // largest bucket resolution bcount holds (bits per axis)
     int *bucket, *bcount, *order, *large_list;
     int64_t *scan_bsum;     // block sums for the scans
@@ -2049,7 +2065,6 @@ struct RecordLayout {
     DevSummary *sum;         // counters of the gradient's record and wide passes
     DevSummary *large_sum;   // the forward's counters: the large pass's queue length
     int *requeue;            // [M]
-    unsigned long long *counter;
 };
 
 RecordLayout carve_records(Carve &c, int64_t M) {
@@ -2060,7 +2075,6 @@ RecordLayout carve_records(Carve &c, int64_t M) {
     R.sum = c.take<DevSummary>(1);
     R.large_sum = c.take<DevSummary>(1);
     R.requeue = c.take<int>(m1);
-    R.counter = c.take<unsigned long long>(1);
     return R;
 }
 
@@ -2162,6 +2176,12 @@ inline void prof_span(int kind, bool end, cudaStream_t st) {
     if (end) g_prof.skind[r][n++] = kind;
 }
 
+// Calls of at most this many rows take them as they come: every warp then has
+// one row, so that their order decides nothing, and the five launches of the
+// bucketing are one (with the launches' counters cleared together, 64 rows take
+// 10 launches for 15).
+constexpr int64_t IDENTITY_ROWS = 4096;
+
 // bucket the queries (writes L.order); positions fit int32 because M < 2^31
 template <class QT>
 void run_bucketing(const nif_dmesh *m, const QT *Q, int64_t M, const Centroid &cen,
@@ -2169,6 +2189,11 @@ void run_bucketing(const nif_dmesh *m, const QT *Q, int64_t M, const Centroid &c
     const int bits = max(1, min(L.bits_cap, bucket_bits(M) + m->tune.bucket_shift));
     const int64_t nbk = (int64_t)1 << (3 * bits);
     prof_mark(0, st);
+    if (M <= IDENTITY_ROWS) {
+        k_identity<<<blocks_for(M, 256), 256, 0, st>>>(M, L.order);
+        prof_mark(1, st);
+        return;
+    }
     cudaMemsetAsync(L.bcount, 0, sizeof(int) * (nbk + 1), st);
     k_bucket<QT><<<blocks_for(M, 256), 256, 0, st>>>(Q, M, cen, m->view, bits, L.bucket, L.bcount);
     // in-place exclusive scan: bucket starts become the scatter cursors
@@ -2186,12 +2211,12 @@ struct RowSet {
     const int *nrows_dev;
     int *large;
     DevSummary *sum;
-    unsigned long long *counter;
+    unsigned long long *counter;  // to clear before the launch; null: sum->work, clear already
     const int *located;  // k_locate's tets of these rows, or null (the row kernel locates)
 };
 
 inline RowSet all_rows(const QueryLayout &L) {
-    return RowSet{L.order, nullptr, L.large_list, L.sum, L.counter, L.located};
+    return RowSet{L.order, nullptr, L.large_list, L.sum, nullptr, L.located};
 }
 
 // queries per work item of the tiled schedule: at most `tile`, smaller for a
@@ -2221,9 +2246,10 @@ void launch_fast_occ(const nif_dmesh *m, const QT *Q, int64_t M, const Centroid 
     const int64_t cap = (int64_t)per_sm * m->num_sms;
     if (blocks > cap) blocks = cap;
     if (blocks < 1) blocks = 1;
-    if (tile > 0) cudaMemsetAsync(R.counter, 0, sizeof(unsigned long long), st);
+    if (tile > 0 && R.counter) cudaMemsetAsync(R.counter, 0, sizeof(unsigned long long), st);
     kern<<<(unsigned)blocks, FAST_BLOCK, smem, st>>>(m->view, Q, cen, R.order, M, R.nrows_dev, sink,
-                                                    LargeQueue{R.large}, R.sum, tile, R.counter);
+                                                    LargeQueue{R.large}, R.sum, tile,
+                                                    R.counter ? R.counter : &R.sum->work[WORK_FUSED]);
 }
 
 // the structure-only (gradient) rows keep their own occupancy; the others
@@ -2246,10 +2272,13 @@ struct Launch {
     int num_sms;
 };
 
-// one persistent launch of kernel `kern` over n rows (tiled schedule)
+// One persistent launch of kernel `kern` over n rows (tiled schedule; the
+// counter is clear).  With `beside` it starts beside the launch before it, once
+// all of that one's blocks have started (griddepcontrol.launch_dependents), and
+// waits for its end before its own.
 template <class Kern, class... Args>
 void launch_rows(Kern kern, const Launch &lc, int64_t n, size_t smem, unsigned long long *counter,
-                 cudaStream_t st, Args... args) {
+                 bool beside, cudaStream_t st, Args... args) {
     constexpr int GPB = FAST_BLOCK / FAST_G;
     const int per_sm = resident_blocks(kern, FAST_BLOCK, smem);
     const int tile = fit_tile(lc.tile, n, per_sm, lc.num_sms, GPB);
@@ -2258,8 +2287,17 @@ void launch_rows(Kern kern, const Launch &lc, int64_t n, size_t smem, unsigned l
     const int64_t cap = (int64_t)per_sm * lc.num_sms;
     if (blocks > cap) blocks = cap;
     if (blocks < 1) blocks = 1;
-    if (tile > 0) cudaMemsetAsync(counter, 0, sizeof(unsigned long long), st);
-    kern<<<(unsigned)blocks, FAST_BLOCK, smem, st>>>(args..., tile, counter);
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)blocks);
+    cfg.blockDim = dim3(FAST_BLOCK);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cfg.attrs = &attr;
+    cfg.numAttrs = beside ? 1 : 0;
+    cudaLaunchKernelEx(&cfg, kern, args..., tile, counter);
 }
 
 // resident blocks per SM of a row kernel with this sink: the mesh's setting,
@@ -2288,17 +2326,20 @@ void launch_general(const Launch &lc, const Rows &rows, const QT *Q, int64_t n, 
 // The split row over positions [0, M) of R.order, whose rows `rows` maps to
 // their meshes: k_locate over all rows, then per chunk of REC_CHUNK rows the
 // cavity records and the volumes.  Rows whose cavity exceeds a record are
-// left in `wide` (count in R.sum->wide_count) for the fused kernel.
-template <class QT, class Rows, class Sink, int OCC, int PM = PM_PLAIN>
+// left in `wide` (count in R.sum->wide_count) for the fused kernel, which
+// launch_wide launches once all cavities are known: the last chunk's volumes run
+// beside it, since the few such rows take one warp each some 60 us (5,003
+// rows: a 43 us volume launch and 61 us of wide rows end after 81 us).
+template <class QT, class Rows, class Sink, int OCC, int PM = PM_PLAIN, class Wide>
 void launch_split(const Launch &lc, const Rows &rows, const QT *Q, int64_t M, const RowSet &R,
                   RowHead *heads, RowEntry *ents, int *wide, int *gen, const Sink &sink, cudaStream_t st,
-                  bool keep = false) {
+                  const Wide &launch_wide, bool keep = false) {
     constexpr int GPB = FAST_BLOCK / FAST_G;
     constexpr int COCC = NIF_CAV_OCC > 0 ? NIF_CAV_OCC : OCC;
     constexpr int VOCC = sink_occ<Sink, (NIF_VOL_OCC > 0 ? NIF_VOL_OCC : (OCC == OCC_HI ? 7 : OCC))>();
     int *located = const_cast<int *>(R.located);
     prof_span(SPAN_LOCATE, false, st);
-    launch_rows(k_locate<QT, Rows, PM>, lc, M, 0, R.counter, st, rows, Q, R.order, M, located,
+    launch_rows(k_locate<QT, Rows, PM>, lc, M, 0, &R.sum->work[WORK_LOCATE], false, st, rows, Q, R.order, M, located,
                 R.sum);
     prof_span(SPAN_LOCATE, true, st);
     for (int64_t c0 = 0; c0 < M; c0 += REC_CHUNK) {
@@ -2307,8 +2348,8 @@ void launch_split(const Launch &lc, const Rows &rows, const QT *Q, int64_t M, co
         RowHead *h = keep ? heads + c0 : heads;
         RowEntry *e = keep ? ents + c0 * REC_CAV : ents;
         prof_span(SPAN_CAVITY, false, st);
-        launch_rows(k_rows_cavity<QT, Rows, COCC, PM>, lc, n, GPB * sizeof(CavWS), R.counter, st,
-                    rows, Q, R.order + c0, n, (const int *)located, h, e, wide, LargeQueue{R.large},
+        launch_rows(k_rows_cavity<QT, Rows, COCC, PM>, lc, n, GPB * sizeof(CavWS),
+                    &R.sum->work[WORK_CAVITY], false, st, rows, Q, R.order + c0, n, (const int *)located, h, e, wide, LargeQueue{R.large},
                     R.sum);
         prof_span(SPAN_CAVITY, true, st);
         prof_span(SPAN_ORDER, false, st);
@@ -2323,9 +2364,11 @@ void launch_split(const Launch &lc, const Rows &rows, const QT *Q, int64_t M, co
                 n, per, (const RowHead *)h, e, R.sum);
         }
         prof_span(SPAN_ORDER, true, st);
+        const bool last = c0 + n == M;
+        if (last) launch_wide();
         prof_span(SPAN_VOLUME, false, st);
-        launch_rows(k_rows_volume<QT, Rows, Sink, VOCC>, lc, n, GPB * sizeof(VolWS), R.counter, st,
-                    rows, Q, R.order + c0, n, (const RowHead *)h, (const RowEntry *)e, gen, sink,
+        launch_rows(k_rows_volume<QT, Rows, Sink, VOCC>, lc, n, GPB * sizeof(VolWS),
+                    &R.sum->work[WORK_VOLUME], last, st, rows, Q, R.order + c0, n, (const RowHead *)h, (const RowEntry *)e, gen, sink,
                     LargeQueue{R.large}, R.sum);
         launch_general(lc, rows, Q, n, R.order + c0, h, e, gen, sink, R.large, R.sum, st);
         prof_span(SPAN_VOLUME, true, st);
@@ -2344,18 +2387,20 @@ void launch_fast(const nif_dmesh *m, const QT *Q, int64_t M, const Centroid &cen
         if (R.located && heads && !R.nrows_dev) {
             const Launch lc{m->tune.tile, m->num_sms};
             const OneMesh rows{m->view, cen};
-            if (m->tune.blocks_per_sm == OCC_LO)
-                launch_split<QT, OneMesh, Sink, OCC_LO, PM>(lc, rows, Q, M, R, heads, ents, wide, gen,
-                                                            sink, st, keep);
-            else
-                launch_split<QT, OneMesh, Sink, OCC_HI, PM>(lc, rows, Q, M, R, heads, ents, wide, gen,
-                                                            sink, st, keep);
             // rows whose cavity exceeds a record: the fused row kernel (which
             // queues what exceeds its own capacities for the large kernel)
-            const RowSet W{wide, &R.sum->wide_count, R.large, R.sum, R.counter, nullptr};
-            prof_span(SPAN_FUSED, false, st);
-            launch_fast_loc<QT, Sink, PM>(m, Q, M, cen, W, sink, st);
-            prof_span(SPAN_FUSED, true, st);
+            auto launch_wide = [&]() {
+                const RowSet W{wide, &R.sum->wide_count, R.large, R.sum, nullptr, nullptr};
+                prof_span(SPAN_FUSED, false, st);
+                launch_fast_loc<QT, Sink, PM>(m, Q, M, cen, W, sink, st);
+                prof_span(SPAN_FUSED, true, st);
+            };
+            if (m->tune.blocks_per_sm == OCC_LO)
+                launch_split<QT, OneMesh, Sink, OCC_LO, PM>(lc, rows, Q, M, R, heads, ents, wide, gen,
+                                                            sink, st, launch_wide, keep);
+            else
+                launch_split<QT, OneMesh, Sink, OCC_HI, PM>(lc, rows, Q, M, R, heads, ents, wide, gen,
+                                                            sink, st, launch_wide, keep);
             return;
         }
     }
@@ -3303,15 +3348,20 @@ void grad_records_typed(const nif_dmesh *m, const void *q, int64_t M, const Cent
     cudaMemsetAsync(R.sum, 0, sizeof(DevSummary), st);
     for (int64_t c0 = 0; c0 < M; c0 += REC_CHUNK) {
         const int64_t n = min((int64_t)REC_CHUNK, M - c0);
+        const bool last = c0 + n == M;
+        if (last) {
+            const RowSet W{L.wide, &L.sum->wide_count, R.requeue, R.sum, nullptr, nullptr};
+            launch_fast_loc<QT, Sink, PM_PLAIN>(m, Q, M, cen, W, sink, st);
+        }
         launch_rows(k_rows_volume<QT, OneMesh, Sink, Sink::VOL_BLOCKS>, lc, n, GPB * sizeof(VolWS),
-                    R.counter, st, rows, Q, L.order + c0, n, (const RowHead *)(R.heads + c0),
-                    (const RowEntry *)(R.ents + c0 * REC_CAV), L.gen, sink, LargeQueue{R.requeue}, R.sum);
+                    &R.sum->work[WORK_VOLUME], last, st, rows, Q, L.order + c0, n,
+                    (const RowHead *)(R.heads + c0), (const RowEntry *)(R.ents + c0 * REC_CAV), L.gen, sink,
+                    LargeQueue{R.requeue}, R.sum);
         launch_general(lc, rows, Q, n, L.order + c0, R.heads + c0, R.ents + c0 * REC_CAV, L.gen, sink,
                        R.requeue, R.sum, st);
-        if (c0 + REC_CHUNK < M) cudaMemsetAsync(&R.sum->general_count, 0, sizeof(int), st);
+        if (!last)  // the next chunk's counter and queue
+            cudaMemsetAsync(&R.sum->work[WORK_VOLUME], 0, sizeof(unsigned long long) + sizeof(int), st);
     }
-    const RowSet W{L.wide, &L.sum->wide_count, R.requeue, R.sum, R.counter, nullptr};
-    launch_fast_loc<QT, Sink, PM_PLAIN>(m, Q, M, cen, W, sink, st);
     cudaMemcpyAsync(R.large_sum, L.sum, sizeof(DevSummary), cudaMemcpyDeviceToDevice, st);
     k_rows_large<QT, Sink><<<LARGE_GROUPS, 32, 0, st>>>(m->view, Q, cen, LargeQueue{L.large_list},
                                                         sink, L.large_ws, L.exact, R.large_sum);
@@ -3495,6 +3545,7 @@ __global__ void __launch_bounds__(FAST_BLOCK, OCC)
                  const int *__restrict__ order, int64_t nrows, const int *nrows_dev, Sink sink,
                  LargeQueue lq, DevSummary *sum, unsigned long long *counter, int tile) {
     extern __shared__ __align__(16) unsigned char smem[];
+    asm volatile("griddepcontrol.launch_dependents;");  // k_rows_volume beside the few wide rows
     // a row count known only on the device (a queue's length) bounds nrows
     if (nrows_dev) nrows = min(nrows, (int64_t)*nrows_dev);
     constexpr int G = FAST_G;
@@ -3599,7 +3650,6 @@ namespace {
 
 struct BatchLayout {
     DevSummary *sum;
-    unsigned long long *counter;
     int *bits, *bucket, *bcount, *order, *large_list, *bsum, *btotal;
     int64_t *bbase;
     LargeWS *large_ws;
@@ -3615,7 +3665,6 @@ BatchLayout carve_batch(Carve &c, int P, int64_t M) {
     BatchLayout L{};
     const int64_t nbk = 8 * (int64_t)P + M / 2 + 1;
     L.sum = c.take<DevSummary>(1);
-    L.counter = c.take<unsigned long long>(1);
     L.bits = c.take<int>(P);
     L.bbase = c.take<int64_t>(P + 1);
     L.bucket = c.take<int>(M > 0 ? M : 1);
@@ -3649,10 +3698,9 @@ void launch_batch_rows_occ(const nif_dbatch *b, const QT *Q, int64_t M, const in
     int64_t blocks = (int64_t)per_sm * b->num_sms;
     if (blocks > want) blocks = want;
     if (blocks < 1) blocks = 1;
-    cudaMemsetAsync(L.counter, 0, sizeof(unsigned long long), st);
     kern<<<(unsigned)blocks, FAST_BLOCK, smem, st>>>(b->d_views, qoff, b->P, Q, cens, order, M, nrows_dev,
-                                                    sink, LargeQueue{L.large_list}, L.sum, L.counter,
-                                                    tile);
+                                                    sink, LargeQueue{L.large_list}, L.sum,
+                                                    &L.sum->work[WORK_FUSED], tile);
 }
 
 // the fused batch row kernel over positions [0, M) of `order` (bounded by
@@ -3675,7 +3723,6 @@ void batch_typed(const nif_dbatch *b, const void *q, int64_t M, const int64_t *q
     const QT *Q = static_cast<const QT *>(q);
     const int64_t nbk = 8 * (int64_t)b->P + M / 2 + 1;
     cudaMemsetAsync(L.sum, 0, sizeof(DevSummary), st);
-    cudaMemsetAsync(L.counter, 0, sizeof(unsigned long long), st);
     cudaMemsetAsync(L.bcount, 0, sizeof(int) * (nbk + 1), st);
     k_batch_setup<<<1, 1, 0, st>>>(qoff, b->P, L.bits, L.bbase);
     k_batch_bucket<QT><<<blocks_for(M, 256), 256, 0, st>>>(Q, M, qoff, b->P, cens, b->d_views, L.bits,
@@ -3689,26 +3736,23 @@ void batch_typed(const nif_dbatch *b, const void *q, int64_t M, const int64_t *q
     // through the fused kernel
     const Launch lc{b->tune.tile, b->num_sms};
     const ManyMeshes rows{b->d_views, qoff, b->P, cens};
-    const RowSet R{L.order, nullptr, L.large_list, L.sum, L.counter, L.located};
-    if (b->filtered) {
+    const RowSet R{L.order, nullptr, L.large_list, L.sum, nullptr, L.located};
+    auto split = [&](auto pm, auto occ) {
+        constexpr int PM = decltype(pm)::value, OCC = decltype(occ)::value;
+        launch_split<QT, ManyMeshes, Sink, OCC, PM>(
+            lc, rows, Q, M, R, L.heads, L.ents, L.wide, L.gen, sink, st,
+            [&]() { launch_batch_rows<QT, Sink, PM>(b, Q, M, qoff, cens, sink, L, st, L.wide, &L.sum->wide_count); });
+    };
+    auto by_occ = [&](auto pm) {
         if (b->tune.blocks_per_sm == OCC_LO)
-            launch_split<QT, ManyMeshes, Sink, OCC_LO, PM_FILTER>(lc, rows, Q, M, R, L.heads, L.ents,
-                                                                  L.wide, L.gen, sink, st);
+            split(pm, std::integral_constant<int, OCC_LO>());
         else
-            launch_split<QT, ManyMeshes, Sink, OCC_HI, PM_FILTER>(lc, rows, Q, M, R, L.heads, L.ents,
-                                                                  L.wide, L.gen, sink, st);
-        launch_batch_rows<QT, Sink, PM_FILTER>(b, Q, M, qoff, cens, sink, L, st, L.wide,
-                                               &L.sum->wide_count);
-    } else {
-        if (b->tune.blocks_per_sm == OCC_LO)
-            launch_split<QT, ManyMeshes, Sink, OCC_LO>(lc, rows, Q, M, R, L.heads, L.ents, L.wide, L.gen,
-                                                       sink, st);
-        else
-            launch_split<QT, ManyMeshes, Sink, OCC_HI>(lc, rows, Q, M, R, L.heads, L.ents, L.wide, L.gen,
-                                                       sink, st);
-        launch_batch_rows<QT, Sink, PM_PLAIN>(b, Q, M, qoff, cens, sink, L, st, L.wide,
-                                              &L.sum->wide_count);
-    }
+            split(pm, std::integral_constant<int, OCC_HI>());
+    };
+    if (b->filtered)
+        by_occ(std::integral_constant<int, PM_FILTER>());
+    else
+        by_occ(std::integral_constant<int, PM_PLAIN>());
     k_rows_batch_large<QT, Sink><<<LARGE_GROUPS, 32, 0, st>>>(b->d_views, qoff, b->P, Q, cens,
                                                              LargeQueue{L.large_list}, sink,
                                                              L.large_ws, L.exact, L.sum);
