@@ -60,8 +60,8 @@ constexpr int THREADS = 32 * WARPS;
 constexpr int HS = 512;                // tested-tet hash slots per insertion (power of two)
 constexpr int CAV = 256;               // cavity tets per insertion
 constexpr int BF = 2 * CAV + 2;        // boundary faces per insertion
-constexpr int WALK_LIMIT = 1 << 16;    // steps of one relocation walk
 constexpr int ROUND_LIMIT = 1 << 14;   // insertion rounds
+constexpr int ROUND_BATCH = 8;         // rounds enqueued at a time
 constexpr unsigned FULL = 0xffffffffu;
 
 enum : int {
@@ -84,6 +84,8 @@ struct State {
     int inserted;           // keys inserted so far
     int deferred;           // nominees skipped for capacity this round
     int max_cav;            // largest cavity seen
+    int rounds;             // rounds run
+    int pad;
     unsigned long long exact_evals;  // predicates decided by expansion arithmetic
 };
 
@@ -93,7 +95,7 @@ struct Cavity {
     long long off;
     int ncav, nbf;
     int status;  // 0 ok, 1 skipped this round, 2 failed, 3 outranked nearby (no flood)
-    int pad;
+    int base;    // a winner's new tets: slots L[0..ncav), then base, base + 1, ...
 };
 
 struct Dev {
@@ -101,9 +103,9 @@ struct Dev {
     int4 *tv, *tn;          // [cap]
     unsigned long long *own, *nom;  // [cap] round-stamped claims
     int *kround;            // [cap] round in which the slot's tet died
-    int *startnew;          // [cap] a live tet of the winner that killed it
+    int *killer;            // [cap] the winner that killed it (its place among the round's nominees)
     int *ptet;              // [n] containing tet of an uninserted key, -1 once inserted
-    int *noms, *wins, *reloc;  // [n] lists of the round
+    int *noms, *reloc;      // [n] lists of the round
     Cavity *cav;            // [n]
     int *lists;             // [list_cap]
     long long list_cap;
@@ -307,7 +309,22 @@ __global__ void k_check_inside(Dev D) {
 // ---------------------------------------------------------------------------
 // one insertion round
 
+// A build that is finished or has failed: the rest of the rounds the host has
+// enqueued do nothing.
+__device__ __forceinline__ bool over(const Dev &D) {
+    return D.st->err != ERR_NONE || D.st->inserted >= D.n;
+}
+
+// (also clears the round's counters: their last readers are done)
 __global__ void k_nominate(Dev D, int round) {
+    if (over(D)) return;
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        if (round > 1 && D.st->nwin == 0) set_err(D.st, ERR_CAPACITY);  // no way on
+        D.st->nnom = D.st->nwin = D.st->nreloc = 0;
+        D.st->listtop = 0;
+        D.st->deferred = 0;
+        D.st->rounds = round;
+    }
     for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < D.n; p += gridDim.x * blockDim.x) {
         const int t = D.ptet[p];
         if (t >= 0) atomicMin(&D.nom[t], key_of(round, p));
@@ -315,6 +332,7 @@ __global__ void k_nominate(Dev D, int round) {
 }
 
 __global__ void k_collect(Dev D, int round) {
+    if (over(D)) return;
     for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < D.n; p += gridDim.x * blockDim.x) {
         const int t = D.ptet[p];
         if (t >= 0 && D.nom[t] == key_of(round, p)) D.noms[atomicAdd(&D.st->nnom, 1)] = p;
@@ -327,6 +345,7 @@ struct CavWS {
     int hkey[HS];
     int8_t hstate[HS];
     int cav[CAV];
+    int4 cavn[CAV];  // the cavity tets' neighbours, read with the tets' vertices
     int ncav;
 };
 
@@ -368,6 +387,7 @@ __global__ void __launch_bounds__(THREADS) k_cavity(Dev D, int round) {
     CavWS &w = wsv[threadIdx.x >> 5];
     const int lane = threadIdx.x & 31;
     const int warps = (gridDim.x * blockDim.x) >> 5;
+    if (over(D)) return;
     const int nnom = D.st->nnom;
     for (int i = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5); i < nnom; i += warps) {
         const int p = D.noms[i];
@@ -381,8 +401,9 @@ __global__ void __launch_bounds__(THREADS) k_cavity(Dev D, int round) {
         // nominees it conflicts with have higher priorities), and the
         // nominees it removes claim nothing, so no winner is lost.
         bool lower = false;
+        const int4 tn0 = D.tn[t0];
         if (lane < 16) {
-            const int n1 = comp4(D.tn[t0], lane >> 2);
+            const int n1 = comp4(tn0, lane >> 2);
             if (n1 >= 0) {
                 lower = D.nom[n1] < key;
                 const int n2 = comp4(D.tn[n1], lane & 3);
@@ -395,7 +416,7 @@ __global__ void __launch_bounds__(THREADS) k_cavity(Dev D, int round) {
                 cv.off = 0;
                 cv.ncav = cv.nbf = 0;
                 cv.status = 3;
-                cv.pad = 0;
+                cv.base = 0;
                 D.cav[i] = cv;
             }
             __syncwarp();
@@ -408,6 +429,7 @@ __global__ void __launch_bounds__(THREADS) k_cavity(Dev D, int round) {
             const int s = h_upsert(w, t0, &fr);
             w.hstate[s] = 1;
             w.cav[0] = t0;
+            w.cavn[0] = tn0;
             w.ncav = 1;
         }
         __syncwarp();
@@ -421,8 +443,7 @@ __global__ void __launch_bounds__(THREADS) k_cavity(Dev D, int round) {
                 bool test = false;
                 int nb = -1, slot = -1;
                 if (k < 4 * (end - head)) {
-                    const int c = w.cav[head + (k >> 2)];
-                    nb = comp4(D.tn[c], k & 3);
+                    nb = reinterpret_cast<const int *>(&w.cavn[head])[k];
                     if (nb >= 0) {
                         bool fresh = false;
                         slot = h_upsert(w, nb, &fresh);
@@ -431,8 +452,10 @@ __global__ void __launch_bounds__(THREADS) k_cavity(Dev D, int round) {
                     }
                 }
                 dv3 a{0, 0, 0}, b = a, c = a, d = a;
+                int4 nn = make_int4(-1, -1, -1, -1);
                 if (test) {
                     const int4 v = D.tv[nb];
+                    nn = D.tn[nb];
                     a = P3(D.pts[v.x]);
                     b = P3(D.pts[v.y]);
                     c = P3(D.pts[v.z]);
@@ -444,10 +467,12 @@ __global__ void __launch_bounds__(THREADS) k_cavity(Dev D, int round) {
                     if (s > 0) {
                         w.hstate[slot] = 1;
                         const int at = atomicAdd(&w.ncav, 1);
-                        if (at < CAV)
+                        if (at < CAV) {
                             w.cav[at] = nb;
-                        else
+                            w.cavn[at] = nn;
+                        } else {
                             status = 1;
+                        }
                     } else {
                         w.hstate[slot] = 2;
                     }
@@ -465,7 +490,7 @@ __global__ void __launch_bounds__(THREADS) k_cavity(Dev D, int round) {
                 const int k = k0 + lane;
                 bool isb = false;
                 if (k < 4 * ncav) {
-                    const int nb = comp4(D.tn[w.cav[k >> 2]], k & 3);
+                    const int nb = reinterpret_cast<const int *>(w.cavn)[k];
                     const int hs = nb < 0 ? -1 : h_find(w, nb);
                     isb = hs < 0 || w.hstate[hs] != 1;
                 }
@@ -490,7 +515,7 @@ __global__ void __launch_bounds__(THREADS) k_cavity(Dev D, int round) {
                 int c = -1, nb = -1;
                 if (k < 4 * ncav) {
                     c = w.cav[k >> 2];
-                    nb = comp4(D.tn[c], k & 3);
+                    nb = reinterpret_cast<const int *>(w.cavn)[k];
                     const int hs = nb < 0 ? -1 : h_find(w, nb);
                     isb = hs < 0 || w.hstate[hs] != 1;
                 }
@@ -530,7 +555,7 @@ __global__ void __launch_bounds__(THREADS) k_cavity(Dev D, int round) {
             cv.ncav = ncav;
             cv.nbf = nbf;
             cv.status = status;
-            cv.pad = 0;
+            cv.base = 0;
             D.cav[i] = cv;
             if (status == 1) atomicAdd(&D.st->deferred, 1);
             if (status == 2) set_err(D.st, ERR_DEGENERATE);
@@ -540,43 +565,37 @@ __global__ void __launch_bounds__(THREADS) k_cavity(Dev D, int round) {
     }
 }
 
-// winners: nominees that hold every one of their claims
-__global__ void k_check(Dev D, int round) {
-    const int nnom = D.st->nnom;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nnom; i += gridDim.x * blockDim.x) {
-        const Cavity cv = D.cav[i];
-        if (cv.status != 0) continue;
-        const unsigned long long key = key_of(round, D.noms[i]);
-        const int *L = D.lists + cv.off;
-        bool won = true;
-        for (int k = 0; k < cv.ncav && won; k++) won = D.own[L[k]] == key;
-        for (int k = 0; k < cv.nbf && won; k++) {
-            const int o = L[cv.ncav + 2 * k + 1];
-            won = o < 0 || D.own[o] == key;
-        }
-        if (won) D.wins[atomicAdd(&D.st->nwin, 1)] = i;
-    }
-}
-
-// shared state of one winner's insertion
+// A winner's boundary faces: vertices, and the slot of the cavity tet in the
+// outside tet's neighbours.
 struct InsWS {
-    int fv[BF][3];   // boundary face vertices
-    int slotg[BF];   // slot of the cavity tet in the outside tet's neighbours
+    int4 face[BF];
 };
 
-// The winners' insertions.  One warp per winner.
+// Winners, the nominees that hold every one of their claims, and their
+// insertions: one warp per nominee.  (Claims and lists are not written here,
+// and two winners' tets are disjoint, so that a nominee can be checked while
+// another is inserted.)
 __global__ void __launch_bounds__(THREADS) k_insert(Dev D, int round) {
     extern __shared__ __align__(16) unsigned char smem[];
     InsWS &w = reinterpret_cast<InsWS *>(smem)[threadIdx.x >> 5];
     const int lane = threadIdx.x & 31;
     const int warps = (gridDim.x * blockDim.x) >> 5;
-    const int nwin = D.st->nwin;
-    for (int wi = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5); wi < nwin; wi += warps) {
-        const int i = D.wins[wi];
-        const int p = D.noms[i];
+    if (D.st->err != ERR_NONE) return;
+    const int nnom = D.st->nnom;
+    for (int i = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5); i < nnom; i += warps) {
         const Cavity cv = D.cav[i];
+        if (cv.status != 0) continue;
+        const int p = D.noms[i];
         const int *L = D.lists + cv.off;
         const int ncav = cv.ncav, nbf = cv.nbf;
+        const unsigned long long key = key_of(round, p);
+        bool won = true;
+        for (int k = lane; k < ncav; k += 32) won = won && D.own[L[k]] == key;
+        for (int k = lane; k < nbf; k += 32) {
+            const int o = L[ncav + 2 * k + 1];
+            won = won && (o < 0 || D.own[o] == key);
+        }
+        if (!__all_sync(FULL, won)) continue;
         // slots of the new tets: the cavity's, then fresh ones
         int base = 0;
         if (lane == 0 && nbf > ncav) base = atomicAdd(&D.st->tet_top, nbf - ncav);
@@ -591,104 +610,130 @@ __global__ void __launch_bounds__(THREADS) k_insert(Dev D, int round) {
             const int cf = L[ncav + 2 * k], o = L[ncav + 2 * k + 1];
             const int c = cf >> 2, f = cf & 3;
             const int4 v = D.tv[c];
-            w.fv[k][0] = comp4(v, fslot(f, 0));
-            w.fv[k][1] = comp4(v, fslot(f, 1));
-            w.fv[k][2] = comp4(v, fslot(f, 2));
             int g = -1;
             if (o >= 0) {
                 const int4 on = D.tn[o];
                 for (int j = 0; j < 4; j++)
                     if (comp4(on, j) == c) g = j;
             }
-            w.slotg[k] = g;
+            w.face[k] = make_int4(comp4(v, fslot(f, 0)), comp4(v, fslot(f, 1)), comp4(v, fslot(f, 2)), g);
         }
         __syncwarp();
         for (int k = lane; k < nbf; k += 32) {
             const int T = slot_of(k);
-            const int a = w.fv[k][0], b = w.fv[k][1], c = w.fv[k][2];
+            const int4 fk = w.face[k];
+            const int a = fk.x, b = fk.y, c = fk.z;
             const int o = L[ncav + 2 * k + 1];
             // (a, b, c, p): face 0 = (a, b, c) faces the outside tet; faces
-            // 1, 2, 3 = (p, b, a), (a, c, p), (p, c, b) hold the edges ab, ac, bc
+            // 1, 2, 3 = (p, b, a), (a, c, p), (p, c, b) hold the edges ab, ac, bc,
+            // each shared with one other boundary face
             int nbr[3] = {-1, -1, -1};
-            const int eu[3] = {a, a, b}, ev[3] = {b, c, c};
-            for (int e = 0; e < 3; e++) {
-                for (int j = 0; j < nbf; j++) {
-                    if (j == k) continue;
-                    const int x = w.fv[j][0], y = w.fv[j][1], z = w.fv[j][2];
-                    const bool hu = x == eu[e] || y == eu[e] || z == eu[e];
-                    const bool hv = x == ev[e] || y == ev[e] || z == ev[e];
-                    if (hu && hv) {
-                        nbr[e] = slot_of(j);
-                        break;
-                    }
-                }
+#pragma unroll 4
+            for (int j = 0; j < nbf; j++) {
+                const int4 fj = w.face[j];
+                const bool ha = fj.x == a || fj.y == a || fj.z == a;
+                const bool hb = fj.x == b || fj.y == b || fj.z == b;
+                const bool hc = fj.x == c || fj.y == c || fj.z == c;
+                if (j == k) continue;
+                if (ha && hb) nbr[0] = j;
+                if (ha && hc) nbr[1] = j;
+                if (hb && hc) nbr[2] = j;
             }
+#pragma unroll
+            for (int e = 0; e < 3; e++)
+                if (nbr[e] >= 0) nbr[e] = slot_of(nbr[e]);
             D.tv[T] = make_int4(a, b, c, p);
             D.tn[T] = make_int4(o, nbr[0], nbr[1], nbr[2]);
             if (nbr[0] < 0 || nbr[1] < 0 || nbr[2] < 0) set_err(D.st, ERR_INTERNAL);
-            if (o >= 0 && w.slotg[k] >= 0)
-                reinterpret_cast<int *>(&D.tn[o])[w.slotg[k]] = T;
+            if (o >= 0 && fk.w >= 0)
+                reinterpret_cast<int *>(&D.tn[o])[fk.w] = T;
             else if (o >= 0)
                 set_err(D.st, ERR_INTERNAL);
         }
-        // cavity slots: the round they died in and where their keys restart
-        const int first = slot_of(0);
+        // cavity slots: the round they died in, and who took their place
         for (int k = lane; k < ncav; k += 32) {
             D.kround[L[k]] = round;
-            D.startnew[L[k]] = first;
+            D.killer[L[k]] = i;
             if (k >= nbf) D.tv[L[k]] = make_int4(-1, -1, -1, -1);  // slot left unused
         }
         if (lane == 0) {
             D.ptet[p] = -1;
+            D.cav[i].base = base;
             atomicAdd(&D.st->inserted, 1);
+            atomicAdd(&D.st->nwin, 1);
         }
         __syncwarp();
     }
 }
 
 __global__ void k_reloc_collect(Dev D, int round) {
+    if (over(D)) return;
     for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < D.n; p += gridDim.x * blockDim.x) {
         const int t = D.ptet[p];
         if (t >= 0 && D.kround[t] == round) D.reloc[atomicAdd(&D.st->nreloc, 1)] = p;
     }
 }
 
-// visibility walk of each key whose tet died, from a tet of its killer
-// (4 lanes, one per face; the first face the key lies strictly outside of)
+// Each key whose tet died goes to the tet of its killer's star that holds it: a
+// lane a tet, three face tests (the faces at the killer; the key is inside the
+// star), so that a key takes one step where a walk through the star took several
+// in a row.  Exact signs; a key on a common face takes the first.
 __global__ void __launch_bounds__(THREADS) k_relocate(Dev D) {
     const int lane = threadIdx.x & 31;
     const int warps = (gridDim.x * blockDim.x) >> 5;
+    if (over(D)) return;
     const int nreloc = D.st->nreloc;
     for (int i = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5); i < nreloc; i += warps) {
         const int p = D.reloc[i];
         const dv3 q = P3(D.pts[p]);
-        int t = D.startnew[D.ptet[p]];
-        int steps = 0;
-        for (;;) {
-            if (++steps > WALK_LIMIT) {
-                if (lane == 0) set_err(D.st, ERR_WALK);
-                t = -1;
-                break;
+        const Cavity cv = D.cav[D.killer[D.ptet[p]]];
+        const int *L = D.lists + cv.off;
+        // first the rounded determinants, certified for the lane they single out;
+        // then, where that is undecided, all signs exactly
+        int t = -1;
+        for (int exact = 0; exact < 2 && t < 0; exact++) {
+            for (int k0 = 0; k0 < cv.nbf && t < 0; k0 += 32) {
+                const int k = k0 + lane;
+                bool in = k < cv.nbf;
+                const int T = in ? (k < cv.ncav ? L[k] : cv.base + (k - cv.ncav)) : 0;
+                dv3 a{0, 0, 0}, b = a, c = a, d = a;
+                if (in) {
+                    const int4 v = D.tv[T];
+                    a = P3(D.pts[v.x]);
+                    b = P3(D.pts[v.y]);
+                    c = P3(D.pts[v.z]);
+                    d = P3(D.pts[v.w]);
+                }
+                // faces 1, 2, 3: (3, 1, 0), (0, 2, 3), (3, 2, 1)
+                if (exact) {
+                    const int s1 = orient_sign(D, d, b, a, q, in);
+                    in = in && s1 >= 0;
+                    const int s2 = orient_sign(D, a, c, d, q, in);
+                    in = in && s2 >= 0;
+                    const int s3 = orient_sign(D, d, c, b, q, in);
+                    in = in && s3 >= 0;
+                } else {
+                    const double o1 = orient_fast(d, b, a, q), o2 = orient_fast(a, c, d, q),
+                                 o3 = orient_fast(d, c, b, q);
+                    in = in && o1 > 0.0 && o2 > 0.0 && o3 > 0.0;
+                    if (in) {
+                        const double A[3] = {a.x, a.y, a.z}, B[3] = {b.x, b.y, b.z}, C[3] = {c.x, c.y, c.z},
+                                     E[3] = {d.x, d.y, d.z}, Q[3] = {q.x, q.y, q.z};
+                        in = !nif_orient_uncertain(o1, nif_orient_permanent(E, B, A, Q)) &&
+                             !nif_orient_uncertain(o2, nif_orient_permanent(A, C, E, Q)) &&
+                             !nif_orient_uncertain(o3, nif_orient_permanent(E, C, B, Q));
+                    }
+                }
+                const unsigned m = __ballot_sync(FULL, in);
+                if (m) t = __shfl_sync(FULL, T, __ffs(m) - 1);
             }
-            const int4 v = D.tv[t];
-            dv3 a{0, 0, 0}, b = a, c = a;
-            if (lane < 4) {
-                a = P3(D.pts[comp4(v, fslot(lane, 0))]);
-                b = P3(D.pts[comp4(v, fslot(lane, 1))]);
-                c = P3(D.pts[comp4(v, fslot(lane, 2))]);
-            }
-            const int s = orient_sign(D, a, b, c, q, lane < 4);
-            const unsigned neg = __ballot_sync(FULL, lane < 4 && s < 0);
-            if (!neg) break;
-            const int nt = comp4(D.tn[t], __ffs(neg) - 1);
-            if (nt < 0) {
-                if (lane == 0) set_err(D.st, ERR_OUTSIDE);
-                t = -1;
-                break;
-            }
-            t = nt;
         }
-        if (lane == 0 && t >= 0) D.ptet[p] = t;
+        if (lane == 0) {
+            if (t >= 0)
+                D.ptet[p] = t;
+            else
+                set_err(D.st, ERR_INTERNAL);
+        }
         __syncwarp();
     }
 }
@@ -838,10 +883,9 @@ Layout carve(Carve &c, int n, int cap) {
     D.own = c.take<unsigned long long>(cap);
     D.nom = c.take<unsigned long long>(cap);
     D.kround = c.take<int>(cap);
-    D.startnew = c.take<int>(cap);
+    D.killer = c.take<int>(cap);
     D.ptet = c.take<int>(n);
     D.noms = c.take<int>(n);
-    D.wins = c.take<int>(n);
     D.reloc = c.take<int>(n);
     D.cav = c.take<Cavity>(n);
     D.list_cap = 96ll * n + (1 << 16);
@@ -922,29 +966,28 @@ NIF_EXPORT int nif_delaunay_build(const double *d_keys, int n, void *d_ws, size_
     State h{};
     DT_CHECK(cudaMemcpyAsync(&h, D.st, sizeof(State), cudaMemcpyDeviceToHost, st));
     DT_CHECK(cudaStreamSynchronize(st));
+    // rounds, ROUND_BATCH of them between looks at the state: those after the
+    // last insertion or an error do nothing
     int round = 0;
     while (h.err == ERR_NONE && h.inserted < n) {
-        if (++round > ROUND_LIMIT) {
+        if (round >= ROUND_LIMIT) {
             h.err = ERR_CAPACITY;
             break;
         }
-        // clear the round's counters (nnom, nwin, nreloc, listtop, deferred)
-        DT_CHECK(cudaMemsetAsync(&D.st->nnom, 0, 3 * sizeof(int), st));
-        DT_CHECK(cudaMemsetAsync(&D.st->listtop, 0, sizeof(long long), st));
-        DT_CHECK(cudaMemsetAsync(&D.st->deferred, 0, sizeof(int), st));
-        k_nominate<<<pblocks, 256, 0, st>>>(D, round);
-        k_collect<<<pblocks, 256, 0, st>>>(D, round);
-        k_cavity<<<wblocks, THREADS, 0, st>>>(D, round);
-        k_check<<<pblocks, 256, 0, st>>>(D, round);
-        k_insert<<<wblocks, THREADS, ins_smem, st>>>(D, round);
-        k_reloc_collect<<<pblocks, 256, 0, st>>>(D, round);
-        k_relocate<<<wblocks, THREADS, 0, st>>>(D);
+        for (int k = 0; k < ROUND_BATCH; k++) {
+            ++round;
+            k_nominate<<<pblocks, 256, 0, st>>>(D, round);
+            k_collect<<<pblocks, 256, 0, st>>>(D, round);
+            k_cavity<<<wblocks, THREADS, 0, st>>>(D, round);
+            k_insert<<<wblocks, THREADS, ins_smem, st>>>(D, round);
+            k_reloc_collect<<<pblocks, 256, 0, st>>>(D, round);
+            k_relocate<<<wblocks, THREADS, 0, st>>>(D);
+        }
         DT_CHECK(cudaGetLastError());
         DT_CHECK(cudaMemcpyAsync(&h, D.st, sizeof(State), cudaMemcpyDeviceToHost, st));
         DT_CHECK(cudaStreamSynchronize(st));
-        if (h.err == ERR_NONE && h.nwin == 0 && h.inserted < n) h.err = ERR_CAPACITY;
     }
-    info->rounds = round;
+    info->rounds = h.rounds;
     info->max_cavity = h.max_cav;
     info->exact_evaluations = (int64_t)h.exact_evals;
     info->tet_slots = h.tet_top;
