@@ -55,7 +55,8 @@ constexpr int FAST_G = NIF_FAST_G;    // lanes per query in the shared-memory ke
 using FastWS = Workspace<256, 96, 128, 64, 128, FAST_G, uint8_t, int8_t>;
 constexpr int LARGE_G = 32;
 using LargeWS = Workspace<16384, 4096, 8192, 2048, 8192, LARGE_G, uint16_t, int16_t>;
-constexpr int ROW_STAGE = 24;         // get_weights: entries staged per row (mean about 15.5)
+constexpr int ROW_STAGE = 32;         // get_weights: entries staged per row (mean about 15.5; one row in
+                                      // 10,000 on random keys is longer)
 using CavWS = CavWorkspace<256, 96, FAST_G, uint8_t, int8_t>;
 #ifndef NIF_VOL_BF
 #define NIF_VOL_BF 42
@@ -108,8 +109,9 @@ struct DevSummary {
     // work-item counters of the tiled row kernels (WORK_*), zero at a call's
     // start like the rest; k_rows_order clears those of the next chunk
     unsigned long long work[4];
-    int general_count; // rows of the current chunk for k_rows_general
-    int reserved;
+    // rows of the current chunk for k_rows_general: known to k_rows_order (cleared
+    // by k_rows_cavity), and found by k_rows_volume (cleared by k_rows_order)
+    int general_count, late_count;
     // predicate evaluations the filter could not certify / whose decision the
     // exact sign changes (PRED_AUDIT and PRED_EXACT meshes)
     unsigned long long orient_unc, orient_flip, insphere_unc, insphere_flip;
@@ -1394,6 +1396,7 @@ __global__ void __launch_bounds__(FAST_BLOCK, OCC) k_rows_fast(MeshView M, const
         s += tile <= 0 ? ng : 1;
     }
     if (g.lane == 0 && steps) atomicAdd(&sum->walk_steps, steps);
+    asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
 // Point location of every row: one warp per row, rows in bucket order as
@@ -1462,6 +1465,7 @@ __global__ void __launch_bounds__(FAST_BLOCK, OCC)
     constexpr int G = FAST_G;
     constexpr int GPB = FAST_BLOCK / G;
     __shared__ MeshView sview[GPB];
+    if (blockIdx.x == 0 && threadIdx.x == 0) sum->general_count = 0;  // k_rows_order's queue, per chunk
     Grp<G> g;
     CavWS &ws = reinterpret_cast<CavWS *>(smem)[threadIdx.x / G];
     int cur = -1;
@@ -1529,10 +1533,11 @@ struct OrderWS {
     int start[33];
 };
 
-__global__ void __launch_bounds__(32 * ORD_WARPS) k_rows_order(int64_t nrows, int per, const RowHead *__restrict__ heads,
-                                                               RowEntry *__restrict__ ents, DevSummary *sum) {
+__global__ void __launch_bounds__(32 * ORD_WARPS) k_rows_order(int64_t nrows, int per, RowHead *__restrict__ heads,
+                                                               RowEntry *__restrict__ ents, int *__restrict__ gen,
+                                                               DevSummary *sum) {
     if (blockIdx.x == 0 && threadIdx.x == 0) {  // k_rows_volume's queue, per chunk, and the counters
-        sum->general_count = 0;
+        sum->late_count = 0;
         sum->work[WORK_CAVITY] = sum->work[WORK_VOLUME] = 0ull;
     }
     extern __shared__ __align__(16) unsigned char smem[];
@@ -1597,7 +1602,7 @@ __global__ void __launch_bounds__(32 * ORD_WARPS) k_rows_order(int64_t nrows, in
             const int *nb = w.nbr[lane];
             for (int c = 0; c < nc; c++) pos[c] = 0;
             uint64_t vis = 0;
-            int sp = 0, nord = 0;
+            int sp = 0, nord = 0, nbf = 0;
             stack[sp++] = 0;  // the flood put the located tet first
             while (sp > 0) {
                 const int c = stack[--sp];
@@ -1605,11 +1610,16 @@ __global__ void __launch_bounds__(32 * ORD_WARPS) k_rows_order(int64_t nrows, in
                 vis |= 1ull << c;
                 pos[c] = (int8_t)nord++;
                 const unsigned wd = (unsigned)nb[c];
+                nbf += __popc(wd & 0x80808080u);
 #pragma unroll
                 for (int f = 0; f < 4; f++) {
                     const int n = (int8_t)((wd >> (8 * f)) & 0xffu);
                     if (n >= 0 && !((vis >> n) & 1ull)) stack[sp++] = (int8_t)n;
                 }
+            }
+            if (nbf > VolWS::BF) {
+                heads[s].state = RS_GENERAL;
+                gen[atomicAdd(&sum->general_count, 1)] = (int)s;
             }
         }
         __syncwarp();
@@ -1659,14 +1669,15 @@ __device__ __forceinline__ bool finish_row(int64_t i, RowInfo &r, RowLanes<IDS> 
     }
 }
 
-// Rows that split_row_body gives up on (ST_GENERAL) are queued in `gen`, by
-// position, for k_rows_general.
+// Rows that split_row_body gives up on (ST_GENERAL) are queued for
+// k_rows_general, by position, from the end of `gen` (gen_end); with `late` so
+// are those that k_rows_order found too large and queued from its start.
 template <class QT, class Rows, class Sink, int OCC>
 __global__ void __launch_bounds__(FAST_BLOCK, OCC)
     k_rows_volume(const __grid_constant__ Rows rows, const QT *__restrict__ Q,
                   const int *__restrict__ order, int64_t nrows, const RowHead *__restrict__ heads,
-                  const RowEntry *__restrict__ ents, int *__restrict__ gen, Sink sink, LargeQueue lq,
-                  DevSummary *sum, int tile, unsigned long long *counter) {
+                  const RowEntry *__restrict__ ents, int *__restrict__ gen_end, bool late, Sink sink,
+                  LargeQueue lq, DevSummary *sum, int tile, unsigned long long *counter) {
     extern __shared__ __align__(16) unsigned char smem[];
     constexpr int G = FAST_G;
     constexpr int GPB = FAST_BLOCK / G;
@@ -1688,7 +1699,9 @@ __global__ void __launch_bounds__(FAST_BLOCK, OCC)
         }
         const int64_t i = order[s];
         const RowHead h = heads[s];
-        if (h.state != RS_QUEUED) {
+        if (h.state == RS_GENERAL) {
+            if (late && g.lane == 0) gen_end[-1 - atomicAdd(&sum->late_count, 1)] = (int)s;
+        } else if (h.state != RS_QUEUED) {
             const double *cen;
             const MeshView &M = rows.get(i, cur, &sview[threadIdx.x / G], g, cen);
             const dv3 q = load_query(Q, i, cen);
@@ -1698,7 +1711,7 @@ __global__ void __launch_bounds__(FAST_BLOCK, OCC)
                 split_row_body<G, VolWS, Sink::FULL, false>(M, q, ws, g, h, ents + s * REC_CAV, r, L);
             if (h.state == RS_WALK) r.status = ST_WALK;
             if (!finish_row(i, r, L, M, q, ws, g, sink, lq, sum) && g.lane == 0)
-                gen[atomicAdd(&sum->general_count, 1)] = (int)s;
+                gen_end[-1 - atomicAdd(&sum->late_count, 1)] = (int)s;
         }
         g.sync();
         s += tile <= 0 ? ng : 1;
@@ -1706,26 +1719,28 @@ __global__ void __launch_bounds__(FAST_BLOCK, OCC)
     asm volatile("griddepcontrol.wait;" ::: "memory");  // the launch this one may run beside
 }
 
-// The rows k_rows_volume queued (about 2 % on random keys; all of them where
-// natinterp3d's degeneracy thresholds exceed the key spacing): a kernel of its
-// own, because the two bodies together outgrow the instruction cache (with
+// The queued rows (about 2 % on random keys; all of them where natinterp3d's
+// degeneracy thresholds exceed the key spacing), those k_rows_order knows beside
+// k_rows_volume (`late` = false), those k_rows_volume finds after it: a kernel of
+// its own, because the two bodies together outgrow the instruction cache (with
 // both in one kernel the volume pass took 11.1 ms a 2M-row call, 8.0 ms apart).
 template <class QT, class Rows, class Sink>
 __global__ void __launch_bounds__(FAST_BLOCK, GEN_OCC)
     k_rows_general(const __grid_constant__ Rows rows, const QT *__restrict__ Q,
                    const int *__restrict__ order, const RowHead *__restrict__ heads,
-                   const RowEntry *__restrict__ ents, const int *__restrict__ gen, Sink sink,
+                   const RowEntry *__restrict__ ents, const int *__restrict__ gen, bool late, Sink sink,
                    LargeQueue lq, DevSummary *sum) {
     extern __shared__ __align__(16) unsigned char smem[];
+    asm volatile("griddepcontrol.launch_dependents;");
     constexpr int G = FAST_G;
     constexpr int GPB = FAST_BLOCK / G;
     __shared__ MeshView sview[GPB];
     Grp<G> g;
     GenWS &ws = reinterpret_cast<GenWS *>(smem)[threadIdx.x / G];
     int cur = -1;
-    const int n = sum->general_count;
+    const int n = late ? sum->late_count : sum->general_count;
     for (int j = blockIdx.x * GPB + threadIdx.x / G; j < n; j += gridDim.x * GPB) {
-        const int64_t s = gen[j];
+        const int64_t s = late ? gen[-1 - j] : gen[j];
         const int64_t i = order[s];
         const double *cen;
         const MeshView &M = rows.get(i, cur, &sview[threadIdx.x / G], g, cen);
@@ -2213,10 +2228,11 @@ struct RowSet {
     DevSummary *sum;
     unsigned long long *counter;  // to clear before the launch; null: sum->work, clear already
     const int *located;  // k_locate's tets of these rows, or null (the row kernel locates)
+    bool beside;         // start beside the launch before (as launch_rows)
 };
 
 inline RowSet all_rows(const QueryLayout &L) {
-    return RowSet{L.order, nullptr, L.large_list, L.sum, nullptr, L.located};
+    return RowSet{L.order, nullptr, L.large_list, L.sum, nullptr, L.located, false};
 }
 
 // queries per work item of the tiled schedule: at most `tile`, smaller for a
@@ -2227,6 +2243,25 @@ inline int fit_tile(int tile, int64_t M, int per_sm, int num_sms, int gpb) {
         if (fit < tile) tile = (int)fit;
     }
     return tile;
+}
+
+// A launch of a row kernel; with `beside` it starts beside the launch before it,
+// once all of that one's blocks have started (griddepcontrol.launch_dependents),
+// and waits for its end before its own (griddepcontrol.wait).
+template <class... Params, class... Args>
+void launch_beside(void (*kern)(Params...), unsigned blocks, size_t smem, bool beside, cudaStream_t st,
+                   Args... args) {
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(blocks);
+    cfg.blockDim = dim3(FAST_BLOCK);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cfg.attrs = &attr;
+    cfg.numAttrs = beside ? 1 : 0;
+    cudaLaunchKernelEx(&cfg, kern, args...);
 }
 
 // persistent grid of the fast row kernel: resident blocks per SM x SMs
@@ -2247,9 +2282,8 @@ void launch_fast_occ(const nif_dmesh *m, const QT *Q, int64_t M, const Centroid 
     if (blocks > cap) blocks = cap;
     if (blocks < 1) blocks = 1;
     if (tile > 0 && R.counter) cudaMemsetAsync(R.counter, 0, sizeof(unsigned long long), st);
-    kern<<<(unsigned)blocks, FAST_BLOCK, smem, st>>>(m->view, Q, cen, R.order, M, R.nrows_dev, sink,
-                                                    LargeQueue{R.large}, R.sum, tile,
-                                                    R.counter ? R.counter : &R.sum->work[WORK_FUSED]);
+    launch_beside(kern, (unsigned)blocks, smem, R.beside, st, m->view, Q, cen, R.order, M, R.nrows_dev, sink,
+                  LargeQueue{R.large}, R.sum, tile, R.counter ? R.counter : &R.sum->work[WORK_FUSED]);
 }
 
 // the structure-only (gradient) rows keep their own occupancy; the others
@@ -2273,9 +2307,7 @@ struct Launch {
 };
 
 // One persistent launch of kernel `kern` over n rows (tiled schedule; the
-// counter is clear).  With `beside` it starts beside the launch before it, once
-// all of that one's blocks have started (griddepcontrol.launch_dependents), and
-// waits for its end before its own.
+// counter is clear).
 template <class Kern, class... Args>
 void launch_rows(Kern kern, const Launch &lc, int64_t n, size_t smem, unsigned long long *counter,
                  bool beside, cudaStream_t st, Args... args) {
@@ -2287,17 +2319,7 @@ void launch_rows(Kern kern, const Launch &lc, int64_t n, size_t smem, unsigned l
     const int64_t cap = (int64_t)per_sm * lc.num_sms;
     if (blocks > cap) blocks = cap;
     if (blocks < 1) blocks = 1;
-    cudaLaunchAttribute attr;
-    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr.val.programmaticStreamSerializationAllowed = 1;
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3((unsigned)blocks);
-    cfg.blockDim = dim3(FAST_BLOCK);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
-    cfg.attrs = &attr;
-    cfg.numAttrs = beside ? 1 : 0;
-    cudaLaunchKernelEx(&cfg, kern, args..., tile, counter);
+    launch_beside(kern, (unsigned)blocks, smem, beside, st, args..., tile, counter);
 }
 
 // resident blocks per SM of a row kernel with this sink: the mesh's setting,
@@ -2310,17 +2332,18 @@ constexpr int sink_occ() {
         return Sink::VOL_BLOCKS;
 }
 
-// k_rows_general over the rows that the launch before queued in `gen`
+// k_rows_general over the rows queued from the start of `gen`, or before it (late)
 template <class QT, class Rows, class Sink>
 void launch_general(const Launch &lc, const Rows &rows, const QT *Q, int64_t n, const int *order,
-                    const RowHead *h, const RowEntry *e, const int *gen, const Sink &sink,
+                    const RowHead *h, const RowEntry *e, const int *gen, bool late, const Sink &sink,
                     int *large, DevSummary *sum, cudaStream_t st) {
     constexpr int GPB = FAST_BLOCK / FAST_G;
     auto kern = k_rows_general<QT, Rows, Sink>;
     const size_t smem = GPB * sizeof(GenWS);
     const int64_t cap = (int64_t)resident_blocks(kern, FAST_BLOCK, smem) * lc.num_sms;
     const int64_t blocks = min((n + GPB - 1) / GPB, cap);
-    kern<<<(unsigned)blocks, FAST_BLOCK, smem, st>>>(rows, Q, order, h, e, gen, sink, LargeQueue{large}, sum);
+    kern<<<(unsigned)blocks, FAST_BLOCK, smem, st>>>(rows, Q, order, h, e, gen, late, sink, LargeQueue{large},
+                                                    sum);
 }
 
 // The split row over positions [0, M) of R.order, whose rows `rows` maps to
@@ -2338,6 +2361,7 @@ void launch_split(const Launch &lc, const Rows &rows, const QT *Q, int64_t M, co
     constexpr int COCC = NIF_CAV_OCC > 0 ? NIF_CAV_OCC : OCC;
     constexpr int VOCC = sink_occ<Sink, (NIF_VOL_OCC > 0 ? NIF_VOL_OCC : (OCC == OCC_HI ? 7 : OCC))>();
     int *located = const_cast<int *>(R.located);
+    const int64_t gen_room = min(M, (int64_t)REC_CHUNK);
     prof_span(SPAN_LOCATE, false, st);
     launch_rows(k_locate<QT, Rows, PM>, lc, M, 0, &R.sum->work[WORK_LOCATE], false, st, rows, Q, R.order, M, located,
                 R.sum);
@@ -2361,16 +2385,18 @@ void launch_split(const Launch &lc, const Rows &rows, const QT *Q, int64_t M, co
             int64_t ob = (groups + ORD_WARPS - 1) / ORD_WARPS;
             if (ob > (int64_t)lc.num_sms * 32) ob = (int64_t)lc.num_sms * 32;
             k_rows_order<<<(unsigned)ob, 32 * ORD_WARPS, ORD_WARPS * sizeof(OrderWS), st>>>(
-                n, per, (const RowHead *)h, e, R.sum);
+                n, per, h, e, gen, R.sum);
         }
         prof_span(SPAN_ORDER, true, st);
-        const bool last = c0 + n == M;
-        if (last) launch_wide();
+        // the rows already known to be for the general kernel, the last chunk's
+        // wide rows and the volumes, beside one another
+        launch_general(lc, rows, Q, n, R.order + c0, h, e, gen, false, sink, R.large, R.sum, st);
+        if (c0 + n == M) launch_wide();
         prof_span(SPAN_VOLUME, false, st);
         launch_rows(k_rows_volume<QT, Rows, Sink, VOCC>, lc, n, GPB * sizeof(VolWS),
-                    &R.sum->work[WORK_VOLUME], last, st, rows, Q, R.order + c0, n, (const RowHead *)h, (const RowEntry *)e, gen, sink,
-                    LargeQueue{R.large}, R.sum);
-        launch_general(lc, rows, Q, n, R.order + c0, h, e, gen, sink, R.large, R.sum, st);
+                    &R.sum->work[WORK_VOLUME], true, st, rows, Q, R.order + c0, n, (const RowHead *)h, (const RowEntry *)e, gen + gen_room,
+                    false, sink, LargeQueue{R.large}, R.sum);
+        launch_general(lc, rows, Q, n, R.order + c0, h, e, gen + gen_room, true, sink, R.large, R.sum, st);
         prof_span(SPAN_VOLUME, true, st);
     }
 }
@@ -2390,7 +2416,7 @@ void launch_fast(const nif_dmesh *m, const QT *Q, int64_t M, const Centroid &cen
             // rows whose cavity exceeds a record: the fused row kernel (which
             // queues what exceeds its own capacities for the large kernel)
             auto launch_wide = [&]() {
-                const RowSet W{wide, &R.sum->wide_count, R.large, R.sum, nullptr, nullptr};
+                const RowSet W{wide, &R.sum->wide_count, R.large, R.sum, nullptr, nullptr, true};
                 prof_span(SPAN_FUSED, false, st);
                 launch_fast_loc<QT, Sink, PM>(m, Q, M, cen, W, sink, st);
                 prof_span(SPAN_FUSED, true, st);
@@ -2437,7 +2463,7 @@ void refill_rows(const nif_dmesh *m, const QT *Q, int64_t M, const Centroid &cen
                  const Sink &sink, cudaStream_t st) {
     // fast-kernel rows longer than ROW_STAGE: the queue's length is on the device
     // (few rows: the row kernel locates them itself)
-    const RowSet R{L.refill, &L.sum->refill_count, L.large_list, L.fill_sum, L.counter, nullptr};
+    const RowSet R{L.refill, &L.sum->refill_count, L.large_list, L.fill_sum, L.counter, nullptr, false};
     if (m->view.pmode == PRED_FAST)
         launch_fast_loc<QT, Sink, PM_PLAIN>(m, Q, M, cen, R, sink, st);
     else
@@ -3346,21 +3372,22 @@ void grad_records_typed(const nif_dmesh *m, const void *q, int64_t M, const Cent
     const Launch lc{m->tune.tile, m->num_sms};
     const OneMesh rows{m->view, cen};
     cudaMemsetAsync(R.sum, 0, sizeof(DevSummary), st);
+    int *gen_end = L.gen + min(M, (int64_t)REC_CHUNK);
     for (int64_t c0 = 0; c0 < M; c0 += REC_CHUNK) {
         const int64_t n = min((int64_t)REC_CHUNK, M - c0);
         const bool last = c0 + n == M;
         if (last) {
-            const RowSet W{L.wide, &L.sum->wide_count, R.requeue, R.sum, nullptr, nullptr};
+            const RowSet W{L.wide, &L.sum->wide_count, R.requeue, R.sum, nullptr, nullptr, false};
             launch_fast_loc<QT, Sink, PM_PLAIN>(m, Q, M, cen, W, sink, st);
         }
         launch_rows(k_rows_volume<QT, OneMesh, Sink, Sink::VOL_BLOCKS>, lc, n, GPB * sizeof(VolWS),
                     &R.sum->work[WORK_VOLUME], last, st, rows, Q, L.order + c0, n,
-                    (const RowHead *)(R.heads + c0), (const RowEntry *)(R.ents + c0 * REC_CAV), L.gen, sink,
-                    LargeQueue{R.requeue}, R.sum);
-        launch_general(lc, rows, Q, n, L.order + c0, R.heads + c0, R.ents + c0 * REC_CAV, L.gen, sink,
+                    (const RowHead *)(R.heads + c0), (const RowEntry *)(R.ents + c0 * REC_CAV), gen_end, true,
+                    sink, LargeQueue{R.requeue}, R.sum);
+        launch_general(lc, rows, Q, n, L.order + c0, R.heads + c0, R.ents + c0 * REC_CAV, gen_end, true, sink,
                        R.requeue, R.sum, st);
         if (!last)  // the next chunk's counter and queue
-            cudaMemsetAsync(&R.sum->work[WORK_VOLUME], 0, sizeof(unsigned long long) + sizeof(int), st);
+            cudaMemsetAsync(&R.sum->work[WORK_VOLUME], 0, sizeof(unsigned long long) + 2 * sizeof(int), st);
     }
     cudaMemcpyAsync(R.large_sum, L.sum, sizeof(DevSummary), cudaMemcpyDeviceToDevice, st);
     k_rows_large<QT, Sink><<<LARGE_GROUPS, 32, 0, st>>>(m->view, Q, cen, LargeQueue{L.large_list},
@@ -3593,6 +3620,7 @@ __global__ void __launch_bounds__(FAST_BLOCK, OCC)
         }
     }
     if (g.lane == 0 && steps) atomicAdd(&sum->walk_steps, steps);
+    asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
 template <class QT, class Sink>
@@ -3698,9 +3726,8 @@ void launch_batch_rows_occ(const nif_dbatch *b, const QT *Q, int64_t M, const in
     int64_t blocks = (int64_t)per_sm * b->num_sms;
     if (blocks > want) blocks = want;
     if (blocks < 1) blocks = 1;
-    kern<<<(unsigned)blocks, FAST_BLOCK, smem, st>>>(b->d_views, qoff, b->P, Q, cens, order, M, nrows_dev,
-                                                    sink, LargeQueue{L.large_list}, L.sum,
-                                                    &L.sum->work[WORK_FUSED], tile);
+    launch_beside(kern, (unsigned)blocks, smem, true, st, (const MeshView *)b->d_views, qoff, b->P, Q, cens,
+                  order, M, nrows_dev, sink, LargeQueue{L.large_list}, L.sum, &L.sum->work[WORK_FUSED], tile);
 }
 
 // the fused batch row kernel over positions [0, M) of `order` (bounded by
@@ -3736,7 +3763,7 @@ void batch_typed(const nif_dbatch *b, const void *q, int64_t M, const int64_t *q
     // through the fused kernel
     const Launch lc{b->tune.tile, b->num_sms};
     const ManyMeshes rows{b->d_views, qoff, b->P, cens};
-    const RowSet R{L.order, nullptr, L.large_list, L.sum, nullptr, L.located};
+    const RowSet R{L.order, nullptr, L.large_list, L.sum, nullptr, L.located, false};
     auto split = [&](auto pm, auto occ) {
         constexpr int PM = decltype(pm)::value, OCC = decltype(occ)::value;
         launch_split<QT, ManyMeshes, Sink, OCC, PM>(

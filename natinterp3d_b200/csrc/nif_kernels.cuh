@@ -634,6 +634,7 @@ struct alignas(16) VolWorkspace {
 // natinterp3d's visiting order and which of its faces take a neighbour's copy.
 constexpr int REC_CAV = 48;  // cavity tets a record holds (larger cavities take the large kernel)
 constexpr int RS_OK = 0, RS_OUTSIDE = 1, RS_WALK = 2, RS_QUEUED = 3;
+constexpr int RS_GENERAL = 4;  // a record of more boundary faces than k_rows_volume takes (k_rows_order)
 struct __align__(16) RowHead {
     int ncav;   // cavity tets (0: the coincident-vertex row)
     int start;  // located tet
@@ -1617,15 +1618,20 @@ __device__ __forceinline__ void split_row_body(const MeshView &M, const dv3 q, W
             if (!GENERAL) terms = M.corner[16 * (size_t)x.tet + (((unsigned)x.pos >> 8) & 15u)];
         }
         unsigned slots = 0;
-        // most vertices get the slot of their hash, all four tried at once
+        // most vertices get the slot of their hash or the one beside it, all four
+        // tried at once
         int s[4];
 #pragma unroll
         for (int i = 0; i < 4; i++) {
             const int v = comp(p, i);
-            s[i] = (int)(mix_hash(v) & (unsigned)(W::VH - 1));
+            s[i] = (int)(mix_hash(v) >> 26);
             if (v < M.n) {
-                const int old = atomicCAS(&C.h.vh_key[s[i]], -1, v);
-                if (old != -1 && old != v) s[i] = -1;
+                int old = atomicCAS(&C.h.vh_key[s[i]], -1, v);
+                if (old != -1 && old != v) {
+                    s[i] ^= 1;
+                    old = atomicCAS(&C.h.vh_key[s[i]], -1, v);
+                    if (old != -1 && old != v) s[i] = -1;
+                }
             } else {
                 s[i] = 0x80 | (v - M.n);
             }
