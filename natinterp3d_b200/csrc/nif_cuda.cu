@@ -57,7 +57,7 @@ constexpr int LARGE_G = 32;
 using LargeWS = Workspace<16384, 4096, 8192, 2048, 8192, LARGE_G, uint16_t, int16_t>;
 constexpr int ROW_STAGE = 32;         // get_weights: entries staged per row (mean about 15.5; one row in
                                       // 10,000 on random keys is longer)
-using CavWS = CavWorkspace<256, 96, FAST_G, uint8_t, int8_t>;
+using CavWS = CavWorkspace<256, 96>;
 #ifndef NIF_VOL_BF
 #define NIF_VOL_BF 42
 #endif
@@ -74,8 +74,8 @@ constexpr int GEN_OCC = 3;
 #endif
 constexpr int REC_CHUNK = NIF_REC_CHUNK;
 // resident blocks per SM of the split kernels (0: the mesh's blocks_per_sm).
-// The cavity kernel is issue-bound and fits 10 blocks in 48 registers (1-2 %
-// faster than 8 on 10M queries).  The volume kernel takes 6 or, for the
+// The cavity kernel takes 8 (64 registers; 10 blocks spill: 2.57 ms a 2M-row call
+// for 2.25).  The volume kernel takes 6 or, for the
 // setting of 8, 7: with 72 registers a thread it barely spills, and a warp's
 // workspace holds 42 boundary faces (2M queries, 200k keys: 7.1 ms at 7
 // blocks, 7.4 ms at 6, 10.1 ms at 8 with 64 registers and 34 faces).
@@ -1290,7 +1290,8 @@ __device__ __forceinline__ int find_problem(const int64_t *__restrict__ off, int
 struct OneMesh {
     MeshView M;
     Centroid cen;
-    __device__ __forceinline__ const MeshView &get(int64_t, int &, MeshView *, const Grp<FAST_G> &,
+    template <int G>
+    __device__ __forceinline__ const MeshView &get(int64_t, int &, MeshView *, const Grp<G> &,
                                                    const double *&c) const {
         c = cen.c;
         return M;
@@ -1302,8 +1303,9 @@ struct ManyMeshes {
     const int64_t *__restrict__ qoff;
     int P;
     const double *__restrict__ cens;
-    __device__ __forceinline__ const MeshView &get(int64_t i, int &cur, MeshView *slot,
-                                                   const Grp<FAST_G> &g, const double *&c) const {
+    template <int G>
+    __device__ __forceinline__ const MeshView &get(int64_t i, int &cur, MeshView *slot, const Grp<G> &g,
+                                                   const double *&c) const {
         const int p = find_problem(qoff, P, i);
         if (p != cur) {
             g.sync();
@@ -1320,15 +1322,16 @@ struct ManyMeshes {
 // then the last `tail` rows (about `tile` per resident group) one at a
 // time, so that the groups finish together instead of waiting on the last
 // full tiles.
+// (`unit` rows: what a group takes at once)
 __device__ __forceinline__ void tile_range(unsigned long long t, int tile, int64_t nrows, int64_t tail,
-                                           int64_t &s, int64_t &s1) {
+                                           int64_t &s, int64_t &s1, int unit = 1) {
     const int64_t nhead = nrows > tail ? (nrows - tail) / tile : 0;
     if ((int64_t)t < nhead) {
         s = (int64_t)t * tile;
         s1 = s + tile;
     } else {
-        s = nhead * tile + ((int64_t)t - nhead);
-        s1 = min(nrows, s + 1);
+        s = nhead * tile + ((int64_t)t - nhead) * unit;
+        s1 = min(nrows, s + unit);
     }
 }
 
@@ -1462,53 +1465,58 @@ __global__ void __launch_bounds__(FAST_BLOCK, OCC)
                   RowHead *__restrict__ heads, RowEntry *__restrict__ ents, int *__restrict__ wide,
                   LargeQueue lq, DevSummary *sum, int tile, unsigned long long *counter) {
     extern __shared__ __align__(16) unsigned char smem[];
-    constexpr int G = FAST_G;
-    constexpr int GPB = FAST_BLOCK / G;
-    __shared__ MeshView sview[GPB];
+    constexpr int GPB = FAST_BLOCK / 32;
+    __shared__ MeshView sview[2 * GPB];
     if (blockIdx.x == 0 && threadIdx.x == 0) sum->general_count = 0;  // k_rows_order's queue, per chunk
-    Grp<G> g;
-    CavWS &ws = reinterpret_cast<CavWS *>(smem)[threadIdx.x / G];
+    const Grp<16> g;  // one of the warp's two rows
+    CavWS &ws = reinterpret_cast<CavWS *>(smem)[threadIdx.x / 16];
+    const int half = g.base / 16;
     int cur = -1;
-    const int64_t gid = tile <= 0 ? (int64_t)blockIdx.x * GPB + threadIdx.x / G : 0;
+    const int64_t gid = (int64_t)blockIdx.x * GPB + threadIdx.x / 32;
     const int64_t ng = (int64_t)gridDim.x * GPB;
-    int64_t s = gid, s1 = tile <= 0 ? nrows : 0;
+    // a call that gives no warp a second row: one row a warp
+    const int unit = tile <= 0 && nrows <= ng ? 1 : 2;
+    int64_t s = tile <= 0 ? unit * gid : 0, s1 = tile <= 0 ? nrows : 0;
     for (;;) {
         if (s >= s1) {
             if (tile <= 0) break;
             unsigned long long t = 0;
-            if (g.lane == 0) t = atomicAdd(counter, 1ull);
-            t = __shfl_sync(g.mask, t, 0, G);
-            tile_range(t, tile, nrows, ng * tile, s, s1);
+            if ((threadIdx.x & 31) == 0) t = atomicAdd(counter, 1ull);
+            t = __shfl_sync(0xffffffffu, t, 0);
+            tile_range(t, tile, nrows, ng * tile, s, s1, 2);
             if (s >= nrows) break;
         }
-        const int64_t i = order[s];
-        const int t = located[i];
-        RowHead h{0, t, RS_OK, 0};
-        if (t == -1) {
-            h.state = RS_OUTSIDE;
-        } else if (t == -3) {
-            h.state = RS_QUEUED;
-            if (g.lane == 0) lq.list[atomicAdd(&sum->large_count, 1)] = (int)i;
-        } else if (t < 0) {
-            h.state = RS_WALK;
-        } else {
-            const double *cen;
-            const MeshView &M = rows.get(i, cur, &sview[threadIdx.x / G], g, cen);
-            const dv3 q = load_query(Q, i, cen);
-            const int rc = cavity_record<G, CavWS, PM>(M, q, ws, g, t, h, ents + s * REC_CAV);
-            if (rc != REC_DONE) {
+        const int64_t my = s + half;
+        const bool row = half < unit && my < s1;
+        int64_t i = 0;
+        RowHead h{0, -1, RS_OK, 0};
+        bool go = false;
+        if (row) {
+            i = order[my];
+            const int t = located[i];
+            h.start = t;
+            go = t >= 0;
+            if (t == -1)
+                h.state = RS_OUTSIDE;
+            else if (t == -3)
                 h.state = RS_QUEUED;
-                if (g.lane == 0) {
-                    if (rc == REC_WIDE)
-                        wide[atomicAdd(&sum->wide_count, 1)] = (int)i;
-                    else
-                        lq.list[atomicAdd(&sum->large_count, 1)] = (int)i;
-                }
-            }
+            else if (t < 0)
+                h.state = RS_WALK;
         }
-        if (g.lane == 0) heads[s] = h;
-        g.sync();
-        s += tile <= 0 ? ng : 1;
+        const double *cen = nullptr;
+        const MeshView &M = rows.get(i, cur, &sview[threadIdx.x / 16], g, cen);
+        const dv3 q = load_query(Q, i, cen);
+        const int rc = flood_pair<CavWS, PM>(M, q, ws, max(h.start, 0), go, h, ents + (row ? my : s) * REC_CAV);
+        if (rc != REC_DONE) h.state = RS_QUEUED;
+        if (row && g.lane == 0) {
+            if (rc == REC_WIDE)
+                wide[atomicAdd(&sum->wide_count, 1)] = (int)i;
+            else if (rc == REC_LARGE || h.start == -3)
+                lq.list[atomicAdd(&sum->large_count, 1)] = (int)i;
+            heads[my] = h;
+        }
+        __syncwarp();
+        s += tile <= 0 ? unit * ng : 2;
     }
 }
 
@@ -2372,7 +2380,7 @@ void launch_split(const Launch &lc, const Rows &rows, const QT *Q, int64_t M, co
         RowHead *h = keep ? heads + c0 : heads;
         RowEntry *e = keep ? ents + c0 * REC_CAV : ents;
         prof_span(SPAN_CAVITY, false, st);
-        launch_rows(k_rows_cavity<QT, Rows, COCC, PM>, lc, n, GPB * sizeof(CavWS),
+        launch_rows(k_rows_cavity<QT, Rows, COCC, PM>, lc, n, 2 * GPB * sizeof(CavWS),
                     &R.sum->work[WORK_CAVITY], false, st, rows, Q, R.order + c0, n, (const int *)located, h, e, wide, LargeQueue{R.large},
                     R.sum);
         prof_span(SPAN_CAVITY, true, st);

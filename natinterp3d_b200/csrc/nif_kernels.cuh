@@ -537,30 +537,23 @@ struct Workspace {
     alignas(16) int4 wave[G_];   // neighbours of the flood wave's cavity tets
 };
 
-// Workspaces of the split row (k_rows_cavity, then k_rows_volume): the same
-// member names as Workspace, each holding only what its phase uses.
-template <int HS_, int CAV_, int G_, class SlotT, class CavT>
-struct CavWorkspace {
-    static constexpr int HS = HS_;
+// Workspace of the split row's cavity phase (flood_pair): one a row, two rows a
+// warp.
+template <int HS_, int CAV_>
+struct alignas(16) CavWorkspace {
+    static constexpr int HS = HS_;             // tested-tet hash slots (power of two)
     static constexpr int QCAP = HS_ * 3 / 4;
     static constexpr int CAV = CAV_;
-    static constexpr int STACK = 4 * CAV_ + 1;
-    static constexpr int G = G_;
-    using slot_t = SlotT;
-    using cav_t = CavT;
-    union U {
-        struct {
-            int hkey[HS_];
-            CavT hval[HS_];
-            SlotT queue[HS_ * 3 / 4];
-        } a;
-        struct {
-            CavT stack[4 * CAV_ + 1];
-        } r;
-    } u;
+    static_assert(HS_ <= 256 && CAV_ <= 127, "slots and cavity indices are bytes");
+    int hkey[HS_];
+    int8_t hval[HS_];       // cavity index of a tested tet, -1 outside
+    int4 wave[16];          // neighbours of the wave's cavity tets
     int cav_tet[CAV_];
-    alignas(4) CavT cav_nbr[4 * CAV_];
-    alignas(16) int4 wave[G_];  // neighbours of the wave's cavity tets
+    uint8_t queue[HS_ * 3 / 4];
+    union {
+        uint8_t nsl[4 * CAV_];                // hash slot of neighbour f of cavity tet c
+        alignas(4) int8_t cav_nbr[4 * CAV_];  // then its cavity index, -1 outside
+    };
 };
 
 // Workspace of the split row's volume phase (split_row): room for BF boundary
@@ -897,9 +890,8 @@ __device__ int locate(const MeshView &M, const dv3 q, const Grp<G> &g, int *scra
 // the cavity index of the o-th visited, ws.pos its inverse and ws.cav_nbr
 // [4c + f] the cavity index of neighbour f of cavity tet c (-1 outside).  On
 // overflow / an uncertain test (PM_FILTER) r.status is set; an empty cavity
-// (0) leaves the order unset.  REPLAY = false stops after the flood and the
-// neighbour table (the split row path replays the order in k_rows_order).
-template <int G, class W, int PM, bool REPLAY = true>
+// (0) leaves the order unset.
+template <int G, class W, int PM>
 __device__ int flood_replay(const MeshView &M, const dv3 q, W &ws, const Grp<G> &g, const int start,
                             RowInfo &r, const bool on_face, double *xs) {
     using cav_t = typename W::cav_t;
@@ -1051,68 +1043,64 @@ __device__ int flood_replay(const MeshView &M, const dv3 q, W &ws, const Grp<G> 
     // cavity-local neighbour table: cav_nbr[4c+f] = cavity index of s[f] or -1
     // (every neighbour slot recorded by the flood has been tested by now)
     for (int k = g.lane; k < 4 * ncav; k += G) ws.cav_nbr[k] = ws.u.a.hval[nsl[k]];
-    if constexpr (!REPLAY) {
-        g.sync();
-    } else {
-        for (int c = g.lane; c < ncav; c += G) ws.pos[c] = (cav_t)-1;
-        g.sync();
+    for (int c = g.lane; c < ncav; c += G) ws.pos[c] = (cav_t)-1;
+    g.sync();
 
-        // cavity index 0 is the located tet, the flood's start
-        int start_c = 0;
-        if constexpr (PM == PM_RESOLVE) {
-            if (on_face && M.pmode == PRED_EXACT) start_c = canonical_start(M, ws, g, xs, q, ncav);
-        }
+    // cavity index 0 is the located tet, the flood's start
+    int start_c = 0;
+    if constexpr (PM == PM_RESOLVE) {
+        if (on_face && M.pmode == PRED_EXACT) start_c = canonical_start(M, ws, g, xs, q, ncav);
+    }
 
-        // replay natinterp3d's LIFO flood on the cavity (its non-cavity tets are
-        // leaves and do not change the order in which cavity tets are reached)
-        if (g.lane == 0) {
-            cav_t *stack = ws.u.r.stack;
-            int sp = 0, nord = 0;
-            stack[sp++] = (cav_t)start_c;
-            if constexpr (W::CAV <= 128) {
-                // visited set in two 64-bit registers
-                uint64_t v0 = 0, v1 = 0;
-                while (sp > 0) {
-                    const int c = stack[--sp];
-                    const uint64_t bit = 1ull << (c & 63);
-                    if ((c < 64 ? v0 : v1) & bit) continue;
-                    if (c < 64) v0 |= bit; else v1 |= bit;
-                    int n0, n1, n2, n3;
-                    if constexpr (sizeof(cav_t) == 1) {
-                        // the four signed 8-bit entries of tet c in one 32-bit load
-                        const int w = *reinterpret_cast<const int *>(&ws.cav_nbr[4 * c]);
-                        n0 = (int8_t)(w & 0xff);
-                        n1 = (int8_t)((w >> 8) & 0xff);
-                        n2 = (int8_t)((w >> 16) & 0xff);
-                        n3 = (int8_t)((unsigned)w >> 24);
-                    } else {
-                        n0 = ws.cav_nbr[4 * c], n1 = ws.cav_nbr[4 * c + 1];
-                        n2 = ws.cav_nbr[4 * c + 2], n3 = ws.cav_nbr[4 * c + 3];
-                    }
-                    ws.pos[c] = (cav_t)nord;
-                    ws.order[nord++] = (cav_t)c;
-                    const int nb[4] = {n0, n1, n2, n3};
-    #pragma unroll
-                    for (int f = 0; f < 4; f++) {
-                        const int nc = nb[f];
-                        if (nc >= 0 && !(((nc < 64 ? v0 : v1) >> (nc & 63)) & 1ull)) stack[sp++] = (cav_t)nc;
-                    }
+    // replay natinterp3d's LIFO flood on the cavity (its non-cavity tets are
+    // leaves and do not change the order in which cavity tets are reached)
+    if (g.lane == 0) {
+        cav_t *stack = ws.u.r.stack;
+        int sp = 0, nord = 0;
+        stack[sp++] = (cav_t)start_c;
+        if constexpr (W::CAV <= 128) {
+            // visited set in two 64-bit registers
+            uint64_t v0 = 0, v1 = 0;
+            while (sp > 0) {
+                const int c = stack[--sp];
+                const uint64_t bit = 1ull << (c & 63);
+                if ((c < 64 ? v0 : v1) & bit) continue;
+                if (c < 64) v0 |= bit; else v1 |= bit;
+                int n0, n1, n2, n3;
+                if constexpr (sizeof(cav_t) == 1) {
+                    // the four signed 8-bit entries of tet c in one 32-bit load
+                    const int w = *reinterpret_cast<const int *>(&ws.cav_nbr[4 * c]);
+                    n0 = (int8_t)(w & 0xff);
+                    n1 = (int8_t)((w >> 8) & 0xff);
+                    n2 = (int8_t)((w >> 16) & 0xff);
+                    n3 = (int8_t)((unsigned)w >> 24);
+                } else {
+                    n0 = ws.cav_nbr[4 * c], n1 = ws.cav_nbr[4 * c + 1];
+                    n2 = ws.cav_nbr[4 * c + 2], n3 = ws.cav_nbr[4 * c + 3];
                 }
-            } else {
-                while (sp > 0) {
-                    const int c = stack[--sp];
-                    if (ws.pos[c] >= 0) continue;
-                    ws.pos[c] = (cav_t)nord;
-                    ws.order[nord++] = (cav_t)c;
-                    for (int f = 0; f < 4; f++) {
-                        const int nc = ws.cav_nbr[4 * c + f];
-                        if (nc >= 0 && ws.pos[nc] < 0) stack[sp++] = (cav_t)nc;
-                    }
+                ws.pos[c] = (cav_t)nord;
+                ws.order[nord++] = (cav_t)c;
+                const int nb[4] = {n0, n1, n2, n3};
+    #pragma unroll
+                for (int f = 0; f < 4; f++) {
+                    const int nc = nb[f];
+                    if (nc >= 0 && !(((nc < 64 ? v0 : v1) >> (nc & 63)) & 1ull)) stack[sp++] = (cav_t)nc;
+                }
+            }
+        } else {
+            while (sp > 0) {
+                const int c = stack[--sp];
+                if (ws.pos[c] >= 0) continue;
+                ws.pos[c] = (cav_t)nord;
+                ws.order[nord++] = (cav_t)c;
+                for (int f = 0; f < 4; f++) {
+                    const int nc = ws.cav_nbr[4 * c + f];
+                    if (nc >= 0 && ws.pos[nc] < 0) stack[sp++] = (cav_t)nc;
                 }
             }
         }
-        g.sync();
     }
+    g.sync();
 
     return ncav;
 }
@@ -1417,41 +1405,158 @@ __device__ RowInfo sibson_row(const MeshView &M, const dv3 q, W &ws, const Grp<G
     return row_volumes<G, W, FULL>(M, q, ws, g, ncav, r, face, tet_fp, tet_tv);
 }
 
-// The split row, part 1: cavity and visiting order of q around its located
-// tet, written as a record (head, entries[REC_CAV]).  Returns REC_DONE, or
-// REC_WIDE where the cavity fits the shared-memory capacities but not the
-// record (the caller queues the row for the fused row kernel), or REC_LARGE
-// where it exceeds the shared-memory capacities (the large kernel's).
-// With PM_FILTER a test the error bound cannot certify also gives REC_LARGE
-// (the large kernel resolves it exactly).
+// The split row, part 1: the cavity of q around its located tet (flood_replay's
+// flood), written as a record (head, entries[REC_CAV]): REC_DONE, or REC_WIDE where
+// the cavity fits the shared-memory capacities but not the record (the caller
+// queues the row for the fused row kernel), or REC_LARGE where it exceeds those
+// capacities or, with PM_FILTER, where a test the error bound cannot certify
+// comes up (the large kernel's).
+//
+// A flood's waves hold some 8 tets of 32 lanes' room, so that a warp floods two
+// rows at once, one a half; both halves go through the same instructions until
+// neither has a wave left (rows that diverge by themselves, as with 16-lane
+// groups, run one after the other).  Bound by instruction issue (2.8 of 4 a
+// cycle): 2M rows, 200k keys take 2.25 ms, 3.03 ms with a warp a row.
+// `go`: this half has a row.  Called by the whole warp.
 constexpr int REC_DONE = 0, REC_WIDE = 1, REC_LARGE = 2;
-template <int G, class W, int PM = PM_PLAIN>
-__device__ int cavity_record(const MeshView &M, const dv3 q, W &ws, const Grp<G> &g, int start,
-                             RowHead &head, RowEntry *__restrict__ ent) {
+template <class W, int PM>
+__device__ __forceinline__ int flood_pair(const MeshView &M, const dv3 q, W &ws, const int start, bool go,
+                                          RowHead &head, RowEntry *__restrict__ ent) {
     static_assert(REC_CAV <= 127, "neighbour indices are signed bytes");
-    RowInfo r{ST_OK, 0, 0, false, false, 0.0, 0, 0, 0, 0, 0};
-    const int ncav = flood_replay<G, W, PM, false>(M, q, ws, g, start, r, false, nullptr);
-    if (r.status != ST_OK) return REC_LARGE;
-    if (ncav > REC_CAV) return REC_WIDE;
-    head.ncav = ncav;
-    for (int c = g.lane; c < ncav; c += G) {
-        const int tt = ws.cav_tet[c];
-        unsigned bm = 0, nb = 0;
+    constexpr unsigned FULL = 0xffffffffu;
+    constexpr int NO_TET = -2;
+    const int lane = threadIdx.x & 31, hl = lane & 15, h0 = lane & 16;  // h0: the half's first lane
+    const unsigned lt = (1u << hl) - 1u;
+    auto ballot = [&](bool p) { return (__ballot_sync(FULL, p) >> h0) & 0xffffu; };
+    const bool filt = PM != PM_PLAIN && go && M.pmode != PRED_FAST;
+
+    static_assert(offsetof(W, hval) == sizeof(ws.hkey) && (sizeof(ws.hkey) + sizeof(ws.hval)) % 256 == 0,
+                  "one run of -1s");
 #pragma unroll
-        for (int f = 0; f < 4; f++) {
-            const int nc = ws.cav_nbr[4 * c + f];
-            bm |= (nc < 0 ? 1u : 0u) << f;
-            nb |= ((unsigned)nc & 0xffu) << (8 * f);
+    for (int i = 0; i < (int)((sizeof(ws.hkey) + sizeof(ws.hval)) / 16); i += 16)
+        reinterpret_cast<int4 *>(ws.hkey)[i + hl] = make_int4(-1, -1, -1, -1);
+    __syncwarp();
+    // a missing neighbour (hull face of the super-simplex) has the slot of NO_TET
+    int none_slot = 0;
+    bool full = false;  // never: the queue's limit is below the table's
+    if (hl == 0) {
+        const int h = (int)(mix_hash(start) & (unsigned)(W::HS - 1));
+        ws.hkey[h] = start;
+        ws.queue[0] = (uint8_t)h;
+        bool fresh = false;
+        none_slot = hash_insert(ws.hkey, W::HS, NO_TET, fresh, full);
+    }
+    none_slot = __shfl_sync(FULL, none_slot, h0);
+    __syncwarp();
+    int qhead = 0, qtail = 1, ncav = 0, rc = REC_DONE;
+    // With natinterp3d's signs the located tet's neighbours join its wave (see
+    // flood_replay)
+    const bool ring = !filt;
+    {
+        bool fresh = false;
+        int sl = 0;
+        if (go && ring && hl < 4) {
+            const int nb = comp(M.tn[start], hl);
+            if (nb >= 0) sl = hash_insert(ws.hkey, W::HS, nb, fresh, full);
         }
+        const unsigned pm = ballot(fresh);
+        if (fresh) ws.queue[qtail + __popc(pm & lt)] = (uint8_t)sl;
+        qtail += __popc(pm);
+        __syncwarp();
+    }
+    for (;;) {
+        const int n = go ? min(16, qtail - qhead) : 0;
+        if (!__any_sync(FULL, n > 0)) break;
+        int slot = 0, tt = 0;
+        bool inc = false, unc = false, open = false;
+        int4 nb4 = make_int4(-1, -1, -1, -1);
+        if (hl < n) {
+            slot = ws.queue[qhead + hl];
+            tt = ws.hkey[slot];
+            nb4 = M.tn[tt];  // with the sphere: no second trip for the tets inside
+            const int side = sphere_side(M.tcc[tt], q);
+            inc = side > 0;
+            open = side == 0;
+        }
+        // tests that the cached sphere does not decide: the determinant itself
+        if (__any_sync(FULL, open)) {
+            if (open) {
+                const int4 p = M.tv[tt];
+                const dv3 a = vload(M, p.x), b = vload(M, p.y), c = vload(M, p.z), d = vload(M, p.w);
+                // insphere argument order fixed by the tet's orientation
+                // (natural_insertionfree.c:511-515); PRED_EXACT uses the exact one
+                const bool pos = (M.tinfo[tt] & ((PM != PM_PLAIN && M.pmode == PRED_EXACT) ? 4u : 1u)) != 0;
+                const dv3 ia = pos ? a : b, ib = pos ? b : a;
+                const double sv = insphere_fast(ia, ib, c, d, q);
+                inc = sv > 0;
+                if (filt) unc = insphere_uncertain(ia, ib, c, d, q, sv);
+            }
+            if (PM != PM_PLAIN && ballot(unc)) {
+                rc = REC_LARGE;
+                go = false;
+                inc = false;
+            }
+        }
+        unsigned cm = ballot(inc);
+        if (ring && qhead == 0 && !(cm & 1u)) {  // the located tet is outside: empty cavity
+            go = false;
+            cm = 0;
+            inc = false;
+        }
+        const int i = __popc(cm & lt), ci = ncav + i;
+        if (hl < n) ws.hval[slot] = (int8_t)(inc ? ci : -1);
+        if (inc && ci < W::CAV) {
+            ws.cav_tet[ci] = tt;
+            ws.wave[i] = nb4;
+            // the volume phase reads this tet's face circumcentres
+            prefetch_l2(&M.fcc[4 * (size_t)tt]);
+        }
+        const int base = ncav;
+        ncav += __popc(cm);
+        qhead += n;
+        if (ncav > W::CAV) {
+            rc = REC_LARGE;
+            go = false;
+        }
+        int items = go ? 4 * (ncav - base) : 0;
+        __syncwarp();
+        for (int k = hl; __any_sync(FULL, k < items); k += 16) {
+            bool fresh = false;
+            int sl = none_slot;
+            if (k < items) {
+                const int nb = reinterpret_cast<const int *>(ws.wave)[k];
+                if (nb >= 0) sl = hash_insert(ws.hkey, W::HS, nb, fresh, full);
+                ws.nsl[4 * base + k] = (uint8_t)sl;
+            }
+            const unsigned pm = ballot(fresh);
+            const int qi = qtail + __popc(pm & lt);
+            if (fresh && qi < W::QCAP) ws.queue[qi] = (uint8_t)sl;
+            qtail += __popc(pm);
+            if (qtail > W::QCAP) {
+                rc = REC_LARGE;
+                go = false;
+                items = 0;
+            }
+        }
+        __syncwarp();
+    }
+    if (rc == REC_DONE && ncav > REC_CAV) rc = REC_WIDE;
+    const int nrec = rc == REC_DONE ? ncav : 0;
+    // cavity-local neighbour indices (every neighbour has been tested by now)
+    for (int k = hl; k < 4 * nrec; k += 16) ws.cav_nbr[k] = ws.hval[ws.nsl[k]];
+    __syncwarp();
+    head.ncav = nrec;
+    for (int c = hl; c < nrec; c += 16) {
+        const int nb = *reinterpret_cast<const int *>(&ws.cav_nbr[4 * c]);
+        const unsigned out = (unsigned)nb & 0x80808080u;
         RowEntry e;
-        e.tet = tt;
-        e.bmask = bm;
-        e.nbr = (int)nb;
+        e.tet = ws.cav_tet[c];
+        e.bmask = (out >> 7 | out >> 14 | out >> 21 | out >> 28) & 15u;
+        e.nbr = nb;
         e.pos = 0;
         ent[c] = e;
     }
-    g.sync();
-    return REC_DONE;
+    return rc;
 }
 
 // The corner term of cavity tet t at its vertex vi (natural_insertionfree.c:
