@@ -1296,6 +1296,8 @@ struct OneMesh {
         c = cen.c;
         return M;
     }
+    // whether row i is of the mesh that get() returned last
+    __device__ __forceinline__ bool same(int64_t, int) const { return true; }
 };
 
 struct ManyMeshes {
@@ -1315,6 +1317,9 @@ struct ManyMeshes {
         }
         c = cens + 3 * p;
         return *slot;
+    }
+    __device__ __forceinline__ bool same(int64_t i, int cur) const {
+        return i >= qoff[cur] && i < qoff[cur + 1];
     }
 };
 
@@ -1402,12 +1407,14 @@ __global__ void __launch_bounds__(FAST_BLOCK, OCC) k_rows_fast(MeshView M, const
     asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
-// Point location of every row: one warp per row, rows in bucket order as
-// the row kernels take them; located[i] = the tet, -1 outside the
+// Point location of every row, rows in bucket order as the row kernels take
+// them: a warp finds the seed of one row at a time and walks eight rows at once
+// (a step is four lanes' work and three dependent reads; 2M queries, 200k keys:
+// 1.80 ms with a warp a walk, 1.55 ms); located[i] = the tet, -1 outside the
 // super-simplex, -2 a walk that hit its step limit, -3 (PM_FILTER) a walk
 // test the error bound cannot certify (the large kernel resolves the row).
 #ifndef NIF_LOC_OCC
-#define NIF_LOC_OCC 12
+#define NIF_LOC_OCC 8  // 64 registers (10 and 12 spill: 1.65 and 1.63 ms a 2M-row call for 1.55)
 #endif
 template <class QT, class Rows, int PM = PM_PLAIN>
 __global__ void __launch_bounds__(FAST_BLOCK, NIF_LOC_OCC) k_locate(const __grid_constant__ Rows rows,
@@ -1435,20 +1442,38 @@ __global__ void __launch_bounds__(FAST_BLOCK, NIF_LOC_OCC) k_locate(const __grid
             tile_range(t, tile, nrows, ng * tile, s, s1);
             if (s >= nrows) break;
         }
-        const int64_t i = order[s];
+        // the seeds of the tile's next rows (up to eight, of one mesh), a row at a
+        // time with the whole warp, then their walks together
+        const int64_t i0 = order[s];
         const double *cen;
-        const MeshView &M = rows.get(i, cur, &sview[threadIdx.x / G], g, cen);
-        const dv3 q = load_query(Q, i, cen);
-        RowInfo r{ST_OK, 0, 0, false, false, 0.0, 0, 0, 0, 0, 0};
-        bool on_face = false;
-        const int t = locate<G, PM>(M, q, g, scr, r, on_face);
-        steps += r.steps;
-        if (g.lane == 0)
-            located[i] = r.status == ST_UNCERTAIN ? -3
-                         : (r.status != ST_OK ? -2 : (r.outside ? -1 : t));
+        const MeshView &M = rows.get(i0, cur, &sview[threadIdx.x / G], g, cen);
+        int nr = 0, t = 0;
+        int64_t i = 0;
+        dv3 q{0.0, 0.0, 0.0};
+        do {
+            const int64_t ir = nr == 0 ? i0 : order[s + nr];
+            if (nr > 0 && !rows.same(ir, cur)) break;
+            const dv3 qr = load_query(Q, ir, cen);
+            int tr = grid_nearest<G>(M, qr);
+            if (tr < 0) tr = nearest_centroid<G>(M, qr, g, scr);
+            if (g.lane >> 2 == nr) {
+                i = ir;
+                q = qr;
+                t = tr;
+            }
+            nr++;
+        } while (nr < (tile <= 0 ? 1 : 8) && s + nr < s1);
+        int st;
+        t = walk_rows<PM>(M, q, t, g.lane >> 2 < nr, st);
+        if ((g.lane & 3) == 0 && g.lane >> 2 < nr) {
+            steps += st;
+            located[i] = t;
+        }
         g.sync();
-        s += tile <= 0 ? ng : 1;
+        s += tile <= 0 ? ng : nr;
     }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) steps += __shfl_xor_sync(0xffffffffu, steps, o);
     if (g.lane == 0 && steps) atomicAdd(&sum->walk_steps, steps);
 }
 

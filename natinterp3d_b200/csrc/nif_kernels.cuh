@@ -883,6 +883,57 @@ __device__ int locate(const MeshView &M, const dv3 q, const Grp<G> &g, int *scra
     }
 }
 
+// natinterp3d's walk of up to eight rows at once, four lanes a row (one face
+// test each), from the rows' seed tets t: the located tet, or -1 outside the
+// super-simplex, -2 at the step limit, -3 (PM_FILTER) at a test that the error
+// bound cannot certify and that can change the step.  `act`: the lane's row is
+// there; steps counts its steps.  Called by the whole warp, with the rows of one
+// mesh.
+template <int PM>
+__device__ __forceinline__ int walk_rows(const MeshView &M, const dv3 q, int t, bool act, int &steps) {
+    const bool filt = PM != PM_PLAIN && M.pmode != PRED_FAST;
+    const int f = threadIdx.x & 3, sh = threadIdx.x & 28;
+    steps = 0;
+    while (__any_sync(0xffffffffu, act)) {
+        int4 nbs = make_int4(-1, -1, -1, -1);
+        bool neg = false, unc = false;
+        if (act) {
+            const int4 p = M.tv[t];
+            nbs = M.tn[t];  // loaded with p: no second dependent trip per step
+            const dv3 v1 = vload(M, comp(p, face_vslot(f, 0)));
+            const dv3 v2 = vload(M, comp(p, face_vslot(f, 1)));
+            const dv3 v3 = vload(M, comp(p, face_vslot(f, 2)));
+            const double o = orient_fast(v1, v2, v3, q);
+            if (filt) unc = orient_uncertain(v1, v2, v3, q, o);
+            neg = o < 0.0 && !unc;
+        }
+        // natinterp3d tests faces 0..3 and moves through the first negative one:
+        // only uncertain tests up to that face can change the step
+        const unsigned m = (__ballot_sync(0xffffffffu, neg) >> sh) & 15u;
+        const int first = m ? __ffs(m) - 1 : 4;
+        bool open = false;
+        if constexpr (PM == PM_FILTER)
+            open = (((__ballot_sync(0xffffffffu, unc) >> sh) & 15u) & ((2u << first) - 1u)) != 0u;
+        if (act) {
+            ++steps;
+            if (open) {
+                t = -3;
+                act = false;
+            } else if (!m) {
+                act = false;
+            } else {
+                t = comp(nbs, first);
+                act = t >= 0;  // -1: outside
+                if (act && steps >= WALK_LIMIT) {
+                    t = -2;
+                    act = false;
+                }
+            }
+        }
+    }
+    return t;
+}
+
 // Steps 2 of the row: the cavity of q around tet `start` (natinterp3d's
 // findCavity, natural_insertionfree.c:486-551) by a parallel flood over the
 // tested-tet hash, then natinterp3d's LIFO visiting order replayed on it.
