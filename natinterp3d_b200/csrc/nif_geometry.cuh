@@ -120,22 +120,27 @@ NIF_GEOM_FN dv3 tri_cc(dv3 a, dv3 b, dv3 c) {
 }
 
 // circumcentre of tetrahedron (a, b, c, d); centroid when |denominator| < 1e-30
-// (tet_cc_regular: as tri_cc_regular)
-__device__ __forceinline__ dv3 tet_cc_regular(dv3 a, dv3 b, dv3 c, dv3 d, bool &flat) {
+// (tet_cc_regular: as tri_cc_regular; also the denominator, twice the
+// determinant of the edges from a, and the longest edge squared)
+__device__ __forceinline__ dv3 tet_cc_regular(dv3 a, dv3 b, dv3 c, dv3 d, bool &flat, double &den,
+                                              double &l2) {
     dv3 ba = vsub(b, a), ca = vsub(c, a), da = vsub(d, a);
     dv3 x1 = vcross(ba, ca), x2 = vcross(da, ba), x3 = vcross(ca, da);
-    dv3 m1 = vscale(x1, vdot(da, da));
-    dv3 m2 = vscale(x2, vdot(ca, ca));
-    dv3 m3 = vscale(x3, vdot(ba, ba));
+    const double lb = vdot(ba, ba), lc = vdot(ca, ca), ld = vdot(da, da);
+    l2 = fmax(lb, fmax(lc, ld));
+    dv3 m1 = vscale(x1, ld);
+    dv3 m2 = vscale(x2, lc);
+    dv3 m3 = vscale(x3, lb);
     dv3 s = vadd(m3, vadd(m1, m2));
-    double den = fmul(2.0, vdot(ba, x3));
+    den = fmul(2.0, vdot(ba, x3));
     flat = fabs(den) < 1e-30;
     return vadd(vscale(s, frcp(den)), a);
 }
 
 NIF_GEOM_FN dv3 tet_cc(dv3 a, dv3 b, dv3 c, dv3 d) {
     bool flat;
-    const dv3 r = tet_cc_regular(a, b, c, d, flat);
+    double den, l2;
+    const dv3 r = tet_cc_regular(a, b, c, d, flat, den, l2);
     if (flat)
         return dv3{fmul(fadd(fadd(fadd(a.x, b.x), c.x), d.x), 0.25),
                    fmul(fadd(fadd(fadd(a.y, b.y), c.y), d.y), 0.25),
@@ -143,20 +148,20 @@ NIF_GEOM_FN dv3 tet_cc(dv3 a, dv3 b, dv3 c, dv3 d) {
     return r;
 }
 
-// The subcell volume from the orientation sv of (pa, pb, pc) about pk, the
-// edges e1 = pa - pb, e2 = pa - pc, e3 = pb - pc, and the face circumcentres
-// (dab, dac, dbc) and the tet's (dt), relative to pk.  natinterp3d swaps pa
-// with pb and dac with dbc when sv < 0: that negates e1, exchanges e2 with e3
+// The subcell volume from the orientation of (pa, pb, pc) about pk (`swap`: it is
+// negative), the edges e1 = pa - pb, e2 = pa - pc, e3 = pb - pc, and the face circumcentres
+// (dab, dac, dbc) and the tet's (dt), relative to pk.  natinterp3d then swaps pa
+// with pb and dac with dbc: that negates e1, exchanges e2 with e3
 // and turns the cross products into (c1, -c3, -c2), so that the swapped sum is
 // the negated sum of the same nine products in the order 1, 3, 2 (a rounded
 // operation on negated operands gives the negated result).
-__device__ __forceinline__ double subcell_from(double sv, dv3 e1, dv3 e2, dv3 e3, dv3 dab, dv3 dac,
+__device__ __forceinline__ double subcell_from(bool swap, dv3 e1, dv3 e2, dv3 e3, dv3 dab, dv3 dac,
                                                dv3 dbc, dv3 dt) {
     const dv3 c1 = vcross(dab, dt), c2 = vcross(dt, dac), c3 = vcross(dbc, dt);
     const dv3 m2{fmul(e2.x, c2.x), fmul(e2.y, c2.y), fmul(e2.z, c2.z)};
     const dv3 m3{fmul(e3.x, c3.x), fmul(e3.y, c3.y), fmul(e3.z, c3.z)};
     double vol = fadd(fadd(fmul(e1.x, c1.x), fmul(e1.y, c1.y)), fmul(e1.z, c1.z));
-    if (sv < 0) {
+    if (swap) {
         vol = fadd(fadd(fadd(vol, m3.x), m3.y), m3.z);
         vol = -fadd(fadd(fadd(vol, m2.x), m2.y), m2.z);
     } else {
@@ -174,7 +179,7 @@ NIF_GEOM_FN double subcell_volume(dv3 pk, dv3 pa, dv3 pb, dv3 pc, dv3 ct, dv3 fa
                                                 dv3 fac, dv3 fbc) {
     dv3 ta = vsub(pa, pk), tb = vsub(pb, pk), tc = vsub(pc, pk);
     const double sv = vdot(ta, vcross(tb, tc));
-    return subcell_from(sv, vsub(pa, pb), vsub(pa, pc), vsub(pb, pc), vsub(fab, pk), vsub(fac, pk),
+    return subcell_from(sv < 0, vsub(pa, pb), vsub(pa, pc), vsub(pb, pc), vsub(fab, pk), vsub(fac, pk),
                         vsub(fbc, pk), vsub(ct, pk));
 }
 

@@ -617,7 +617,8 @@ struct alignas(16) VolWorkspace {
     int start[VOL_VERTS];        // first term of a neighbour: cavity, face << 16 (first: its first corner)
     int nbr_vid[VOL_VERTS];
     unsigned fid[BF_];           // ids of the face's three vertices, one byte each
-    int bff[BF_];                // fcc[] index of the face (first: visiting position << 2 | face)
+    int bff[BF_];                // fcc[] index of the face (first: visiting position << 2 | face); the
+                                 // sign bit: its corners' orientation is negative
 };
 
 // One row between k_rows_cavity, k_rows_order and k_rows_volume: a header
@@ -2044,10 +2045,21 @@ __device__ __forceinline__ void split_row_body(const MeshView &M, const dv3 q, W
         const unsigned ids = ws.fid[b];
         const dv3 pa = sload(ws.pos[ids & 0xff]), pb = sload(ws.pos[(ids >> 8) & 0xff]),
                   pc = sload(ws.pos[ids >> 16]);
-        bool flat = false;
-        const dv3 c = GENERAL ? tet_cc(q, pa, pb, pc) : tet_cc_regular(q, pa, pb, pc, flat);
-        general |= flat;
-        sstore(V.ct[b], c);
+        if (GENERAL) {
+            sstore(V.ct[b], tet_cc(q, pa, pb, pc));
+        } else {
+            // The orientation of (q, w, x) about each corner u has the exact value
+            // -det(a - q, b - q, c - q) = -den / 2.  With l the longest of the three
+            // vectors (edges are below 2 l), both computed values are within
+            // 200 eps l^3 = 2.3e-14 l^3 of it, so that beyond 1e-13 l^3 they have its
+            // sign: one orientation a face instead of one a corner (23 of a corner's
+            // 85 FP64 operations).
+            bool flat = false;
+            double den, l2;
+            sstore(V.ct[b], tet_cc_regular(q, pa, pb, pc, flat, den, l2));
+            general |= flat || !(den * den > 1e-26 * l2 * l2 * l2);
+            if (den > 0.0) ws.bff[b] |= INT_MIN;  // a negative orientation
+        }
     }
     if (!GENERAL && g.any(general)) {
         r.status = ST_GENERAL;
@@ -2062,7 +2074,8 @@ __device__ __forceinline__ void split_row_body(const MeshView &M, const dv3 q, W
             const int b = k / 3;
             constexpr unsigned NONE = (1u << W::EB) - 1u;
             const unsigned e = (unsigned)(cn >> 18) & NONE;
-            const dv3 cf = cload(&M.fcc[ws.bff[b]]);
+            const int ffi = ws.bff[b];
+            const dv3 cf = cload(&M.fcc[ffi & INT_MAX]);
             const dv3 pu = sload(ws.pos[u]), pw = sload(ws.pos[((unsigned)cn >> 6) & 63]),
                       px = sload(ws.pos[((unsigned)cn >> 12) & 63]);
             dv3 dac;
@@ -2071,9 +2084,9 @@ __device__ __forceinline__ void split_row_body(const MeshView &M, const dv3 q, W
             else
                 dac = sload(V.ec[e]);
             // subcell_volume(u, q, w, x, ct, cc(u, q, w), cc(u, q, x), cf)
-            const double sv = vdot(vsub(q, pu), vcross(vsub(pw, pu), vsub(px, pu)));
+            const bool swap = GENERAL ? vdot(vsub(q, pu), vcross(vsub(pw, pu), vsub(px, pu))) < 0 : ffi < 0;
             ws.fterm[(unsigned)(cn >> (18 + W::EB))] =
-                -subcell_from(sv, vsub(q, pw), vsub(q, px), vsub(pw, px), sload(V.ec[k]), dac, vsub(cf, pu),
+                -subcell_from(swap, vsub(q, pw), vsub(q, px), vsub(pw, px), sload(V.ec[k]), dac, vsub(cf, pu),
                               vsub(sload(V.ct[b]), pu));
         }
     }
