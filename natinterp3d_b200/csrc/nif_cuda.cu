@@ -467,10 +467,8 @@ __global__ void k_scatter(const int *__restrict__ bucket, int64_t M, int *__rest
     }
 }
 
-__global__ void k_identity(int64_t M, int *__restrict__ order) {
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < M;
-         i += (int64_t)gridDim.x * blockDim.x)
-        order[i] = (int)i;
+__global__ void k_iota(int n, int *__restrict__ out) {
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) out[i] = i;
 }
 
 // ---------------------------------------------------------------------------
@@ -1096,9 +1094,12 @@ __global__ void k_spmm(int64_t M, int D, const int32_t *__restrict__ rowptr,
 __global__ void k_row_of(int64_t M, const int32_t *__restrict__ rowptr, int32_t *__restrict__ rowof,
                          uint32_t *__restrict__ keys, const int32_t *__restrict__ cols,
                          int32_t *__restrict__ idx, const int32_t *__restrict__ rank, int64_t N) {
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < M;
-         i += (int64_t)gridDim.x * blockDim.x)
-        for (int e = rowptr[i]; e < rowptr[i + 1]; e++) {
+    // eight lanes a row, so that a warp writes four rows' runs of entries
+    for (int64_t u = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; u < 8 * M;
+         u += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t i = u >> 3;
+        const int e1 = rowptr[i + 1];
+        for (int e = rowptr[i] + (int)(u & 7); e < e1; e += 8) {
             rowof[e] = (int32_t)i;
             int k = cols[e];
             if (rank) {
@@ -1108,6 +1109,7 @@ __global__ void k_row_of(int64_t M, const int32_t *__restrict__ rowptr, int32_t 
             keys[e] = (uint32_t)k;
             idx[e] = e;
         }
+    }
 }
 
 // inverse of a processing order: inv[rank[k]] = k (entries a bad rank leaves
@@ -1120,101 +1122,117 @@ __global__ void k_rank_inverse(int64_t N, const int32_t *__restrict__ rank, int3
     }
 }
 
-// stable LSD radix sort of (key, value) pairs, 4 bits per pass
+// Stable LSD radix sort of (key, value) pairs, up to 8 bits a pass (rs_plan: as
+// few passes as the key's bits allow, of equal width).  A pass moves 16 bytes a
+// pair twice (15.5M pairs of 18 bits: three passes for the five of 4 bits that
+// packed counters allowed; with k_row_of eight lanes a row, a training step of 1M
+// rows 11.1 to 10.0 ms).
 constexpr int RS_THREADS = 256;
+constexpr int RS_WARPS = RS_THREADS / 32;
 constexpr int RS_ITEMS = 8;
 constexpr int RS_TILE = RS_THREADS * RS_ITEMS;
+constexpr int RS_BINS = 256;  // digits of a pass, at most
 
+struct RsPlan {
+    int passes, bits;
+};
+constexpr RsPlan rs_plan(int key_bits) {
+    const int passes = (key_bits + 7) / 8;
+    return RsPlan{passes, passes > 0 ? (key_bits + passes - 1) / passes : 0};
+}
+
+// hist[digit][block]; `bins` digits from bit `shift`
 __global__ void __launch_bounds__(RS_THREADS) k_rs_hist(const uint32_t *__restrict__ keys, int64_t n,
-                                                         int shift, int nblocks, int *__restrict__ hist) {
-    __shared__ int h[16];
-    if (threadIdx.x < 16) h[threadIdx.x] = 0;
+                                                        int shift, int bins, int nblocks,
+                                                        int *__restrict__ hist) {
+    __shared__ int h[RS_BINS];
+    h[threadIdx.x] = 0;
     __syncthreads();
     const int64_t base = (int64_t)blockIdx.x * RS_TILE;
     for (int j = 0; j < RS_ITEMS; j++) {
         const int64_t i = base + j * RS_THREADS + threadIdx.x;
-        if (i < n) atomicAdd(&h[(keys[i] >> shift) & 15u], 1);
+        if (i < n) atomicAdd(&h[(keys[i] >> shift) & (unsigned)(bins - 1)], 1);
     }
     __syncthreads();
-    if (threadIdx.x < 16) hist[(int64_t)threadIdx.x * nblocks + blockIdx.x] = h[threadIdx.x];
+    if ((int)threadIdx.x < bins) hist[(int64_t)threadIdx.x * nblocks + blockIdx.x] = h[threadIdx.x];
 }
 
-__device__ __forceinline__ unsigned long long pick4(unsigned long long c0, unsigned long long c1,
-                                                    unsigned long long c2, unsigned long long c3,
-                                                    int d) {
-    const unsigned long long c = (d < 4) ? c0 : (d < 8 ? c1 : (d < 12 ? c2 : c3));
-    return (c >> (16 * (d & 3))) & 0xffffull;
-}
-
-// Thread t of a block owns the tile's items 8t..8t+7 in order; an item's
-// destination is the block's start for its digit (scanned histogram) plus
-// the digit's count in earlier threads plus its rank inside its own thread,
-// so equal keys keep their input order.  Counts are packed 16 bits per digit.
+// Warp w of a block owns the tile's pairs 256 w .. 256 w + 255, 32 at a time; a
+// pair's rank among its digit's is the count in earlier warps, in the warp's
+// earlier rounds and in lower lanes (match), so equal keys keep their input
+// order.  The tile is put in digit order in shared memory first, so that a
+// digit's pairs are one run of writes; they start at the scanned histogram's
+// off[digit][block].
 __global__ void __launch_bounds__(RS_THREADS) k_rs_scatter(
-    const uint32_t *__restrict__ kin, const int32_t *__restrict__ vin, int64_t n, int shift,
+    const uint32_t *__restrict__ kin, const int32_t *__restrict__ vin, int64_t n, int shift, int bins,
     int nblocks, const int *__restrict__ off, uint32_t *__restrict__ kout, int32_t *__restrict__ vout) {
     __shared__ uint32_t sk[RS_TILE];
     __shared__ int32_t sv[RS_TILE];
-    __shared__ unsigned long long wsum[RS_THREADS / 32][4];
+    __shared__ int cnt[RS_WARPS][RS_BINS];
+    __shared__ int first[RS_BINS];  // place of a digit's first pair in the tile
+    __shared__ int wsum[RS_WARPS];
     const int64_t base = (int64_t)blockIdx.x * RS_TILE;
-    for (int j = 0; j < RS_ITEMS; j++) {
-        const int idx = j * RS_THREADS + threadIdx.x;
-        if (base + idx < n) {
-            sk[idx] = kin[base + idx];
-            sv[idx] = vin[base + idx];
-        }
-    }
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int m = (int)min((int64_t)RS_TILE, n - base);
+#pragma unroll
+    for (int w = 0; w < RS_WARPS; w++) cnt[w][threadIdx.x] = 0;
     __syncthreads();
     uint32_t mk[RS_ITEMS];
     int32_t mv[RS_ITEMS];
-    int dg[RS_ITEMS], rk[RS_ITEMS];
-    unsigned long long c0 = 0, c1 = 0, c2 = 0, c3 = 0;
+    int rk[RS_ITEMS];
 #pragma unroll
     for (int j = 0; j < RS_ITEMS; j++) {
-        const int idx = threadIdx.x * RS_ITEMS + j;
-        dg[j] = -1;
-        rk[j] = 0;
-        mk[j] = 0;
-        mv[j] = 0;
-        if (base + idx < n) {
-            mk[j] = sk[idx];
-            mv[j] = sv[idx];
-            const int d = (int)((mk[j] >> shift) & 15u);
-            dg[j] = d;
-            rk[j] = (int)pick4(c0, c1, c2, c3, d);
-            const unsigned long long inc = 1ull << (16 * (d & 3));
-            if (d < 4) c0 += inc; else if (d < 8) c1 += inc; else if (d < 12) c2 += inc; else c3 += inc;
-        }
+        const int i = warp * 32 * RS_ITEMS + j * 32 + lane;
+        mk[j] = i < m ? kin[base + i] : 0u;
+        mv[j] = i < m ? vin[base + i] : 0;
     }
-    // exclusive scan of the packed counts over the block's threads
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    unsigned long long s0 = c0, s1 = c1, s2 = c2, s3 = c3;
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const unsigned long long t0 = __shfl_up_sync(0xffffffffu, s0, o);
-        const unsigned long long t1 = __shfl_up_sync(0xffffffffu, s1, o);
-        const unsigned long long t2 = __shfl_up_sync(0xffffffffu, s2, o);
-        const unsigned long long t3 = __shfl_up_sync(0xffffffffu, s3, o);
-        if (lane >= o) {
-            s0 += t0; s1 += t1; s2 += t2; s3 += t3;
-        }
-    }
-    if (lane == 31) {
-        wsum[warp][0] = s0; wsum[warp][1] = s1; wsum[warp][2] = s2; wsum[warp][3] = s3;
+    for (int j = 0; j < RS_ITEMS; j++) {
+        const bool live = warp * 32 * RS_ITEMS + j * 32 + lane < m;
+        const int d = live ? (int)((mk[j] >> shift) & (unsigned)(bins - 1)) : -1;
+        const unsigned peers = __match_any_sync(0xffffffffu, d);
+        const int before = live ? cnt[warp][d] : 0;
+        __syncwarp();
+        if (live && lane == __ffs(peers) - 1) cnt[warp][d] = before + __popc(peers);
+        __syncwarp();
+        rk[j] = before + __popc(peers & ((1u << lane) - 1u));
     }
     __syncthreads();
-    unsigned long long e0 = s0 - c0, e1 = s1 - c1, e2 = s2 - c2, e3 = s3 - c3;
-    for (int w = 0; w < warp; w++) {
-        e0 += wsum[w][0]; e1 += wsum[w][1]; e2 += wsum[w][2]; e3 += wsum[w][3];
+    // digit t: its warps' counts to starts, then the digits' starts in the tile
+    int total = 0;
+#pragma unroll
+    for (int w = 0; w < RS_WARPS; w++) {
+        const int c = cnt[w][threadIdx.x];
+        cnt[w][threadIdx.x] = total;
+        total += c;
     }
+    int incl = total;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int t = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += t;
+    }
+    if (lane == 31) wsum[warp] = incl;
+    __syncthreads();
+    for (int w = 0; w < warp; w++) incl += wsum[w];
+    first[threadIdx.x] = incl - total;
+    __syncthreads();
 #pragma unroll
     for (int j = 0; j < RS_ITEMS; j++) {
-        const int d = dg[j];
-        if (d < 0) continue;
-        const int64_t pos = (int64_t)off[(int64_t)d * nblocks + blockIdx.x] +
-                            (int64_t)pick4(e0, e1, e2, e3, d) + rk[j];
-        kout[pos] = mk[j];
-        vout[pos] = mv[j];
+        if (warp * 32 * RS_ITEMS + j * 32 + lane < m) {
+            const int d = (int)((mk[j] >> shift) & (unsigned)(bins - 1));
+            const int at = first[d] + cnt[warp][d] + rk[j];
+            sk[at] = mk[j];
+            sv[at] = mv[j];
+        }
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < m; i += RS_THREADS) {
+        const uint32_t k = sk[i];
+        const int d = (int)((k >> shift) & (unsigned)(bins - 1));
+        const int64_t pos = (int64_t)off[(int64_t)d * nblocks + blockIdx.x] + (i - first[d]);
+        kout[pos] = k;
+        vout[pos] = sv[i];
     }
 }
 
@@ -1890,6 +1908,7 @@ struct nif_dmesh {
     size_t bytes;
     int64_t orient_unc, orient_flip;  // tets with an uncertain / flipped orientation flag
     int oct_nodes, oct_levels;        // centroid octree: nodes, node levels
+    const int *iota;                  // order of a call of up to IDENTITY_ROWS rows
     nif_tuning tune{OCC_DEFAULT, 0, MESH_TILE_DEFAULT, 0};
 };
 
@@ -1955,9 +1974,9 @@ OctScratch carve_oct_scratch(Carve &c, int nt) {
     S.key_b = c.take<uint32_t>(nt);
     S.idx_a = c.take<int32_t>(nt);
     S.idx_b = c.take<int32_t>(nt);
-    S.hist = c.take<int>(16 * S.nblocks);
-    S.off = c.take<int>(16 * S.nblocks);
-    S.bsum = c.take<int>((16 * S.nblocks + nt + SCAN_TILE - 1) / SCAN_TILE + 1);
+    S.hist = c.take<int>(RS_BINS * S.nblocks);
+    S.off = c.take<int>(RS_BINS * S.nblocks);
+    S.bsum = c.take<int>((RS_BINS * S.nblocks + nt + SCAN_TILE - 1) / SCAN_TILE + 1);
     S.tot = c.take<int>(2);
     S.code = c.take<unsigned long long>(nt);
     S.node_of = c.take<int>(nt);
@@ -1981,7 +2000,14 @@ size_t fcc_slots(int nt) {
     return need > 4 * (size_t)nt ? need : 4 * (size_t)nt;
 }
 
+// Calls of at most this many rows take them as they come: every warp then has
+// one row, so that their order decides nothing, and the bucketing's six
+// launches are left out (with the work counters cleared together, 64 rows took 15
+// launches and take 10).
+constexpr int64_t IDENTITY_ROWS = 4096;
+
 struct MeshLayout {
+    int *iota;                   // 0, 1, ... IDENTITY_ROWS - 1: such a call's order
     d4 *vtx;
     int4 *tv, *tn;
     uint32_t *tinfo;
@@ -2006,6 +2032,7 @@ constexpr int CORNER_TETS_MAX = NIF_CORNER_TETS_MAX;
 
 MeshLayout carve_mesh(Carve &c, int nv, int nt) {
     MeshLayout L;
+    L.iota = c.take<int>(IDENTITY_ROWS);
     L.vtx = c.take<d4>(nv);
     L.tv = c.take<int4>(nt);
     L.tn = c.take<int4>(nt);
@@ -2055,6 +2082,11 @@ struct QueryLayout {
     int *refill;            // fast-kernel rows longer than ROW_STAGE
     DevSummary *fill_sum;   // counters of the fill pass's recomputed rows
 };
+
+// the rows' order after run_bucketing
+inline const int *row_order(const nif_dmesh *m, const QueryLayout &L, int64_t M) {
+    return M <= IDENTITY_ROWS ? m->iota : L.order;
+}
 
 constexpr int bucket_bits(int64_t M) {
     int b = 1;
@@ -2224,13 +2256,8 @@ inline void prof_span(int kind, bool end, cudaStream_t st) {
     if (end) g_prof.skind[r][n++] = kind;
 }
 
-// Calls of at most this many rows take them as they come: every warp then has
-// one row, so that their order decides nothing, and the five launches of the
-// bucketing are one (with the launches' counters cleared together, 64 rows take
-// 10 launches for 15).
-constexpr int64_t IDENTITY_ROWS = 4096;
-
-// bucket the queries (writes L.order); positions fit int32 because M < 2^31
+// bucket the queries (writes L.order, which calls of up to IDENTITY_ROWS rows do
+// not read); positions fit int32 because M < 2^31
 template <class QT>
 void run_bucketing(const nif_dmesh *m, const QT *Q, int64_t M, const Centroid &cen,
                    const QueryLayout &L, cudaStream_t st) {
@@ -2238,7 +2265,6 @@ void run_bucketing(const nif_dmesh *m, const QT *Q, int64_t M, const Centroid &c
     const int64_t nbk = (int64_t)1 << (3 * bits);
     prof_mark(0, st);
     if (M <= IDENTITY_ROWS) {
-        k_identity<<<blocks_for(M, 256), 256, 0, st>>>(M, L.order);
         prof_mark(1, st);
         return;
     }
@@ -2264,8 +2290,8 @@ struct RowSet {
     bool beside;         // start beside the launch before (as launch_rows)
 };
 
-inline RowSet all_rows(const QueryLayout &L) {
-    return RowSet{L.order, nullptr, L.large_list, L.sum, nullptr, L.located, false};
+inline RowSet all_rows(const nif_dmesh *m, const QueryLayout &L, int64_t M) {
+    return RowSet{row_order(m, L, M), nullptr, L.large_list, L.sum, nullptr, L.located, false};
 }
 
 // queries per work item of the tiled schedule: at most `tile`, smaller for a
@@ -2401,12 +2427,13 @@ void launch_split(const Launch &lc, const Rows &rows, const QT *Q, int64_t M, co
     prof_span(SPAN_LOCATE, true, st);
     for (int64_t c0 = 0; c0 < M; c0 += REC_CHUNK) {
         const int64_t n = min((int64_t)REC_CHUNK, M - c0);
+        const int *order = R.order + c0;
         // one chunk's records, or (keep) every row's at its own position
         RowHead *h = keep ? heads + c0 : heads;
         RowEntry *e = keep ? ents + c0 * REC_CAV : ents;
         prof_span(SPAN_CAVITY, false, st);
         launch_rows(k_rows_cavity<QT, Rows, COCC, PM>, lc, n, 2 * GPB * sizeof(CavWS),
-                    &R.sum->work[WORK_CAVITY], false, st, rows, Q, R.order + c0, n, (const int *)located, h, e, wide, LargeQueue{R.large},
+                    &R.sum->work[WORK_CAVITY], false, st, rows, Q, order, n, (const int *)located, h, e, wide, LargeQueue{R.large},
                     R.sum);
         prof_span(SPAN_CAVITY, true, st);
         prof_span(SPAN_ORDER, false, st);
@@ -2423,13 +2450,13 @@ void launch_split(const Launch &lc, const Rows &rows, const QT *Q, int64_t M, co
         prof_span(SPAN_ORDER, true, st);
         // the rows already known to be for the general kernel, the last chunk's
         // wide rows and the volumes, beside one another
-        launch_general(lc, rows, Q, n, R.order + c0, h, e, gen, false, sink, R.large, R.sum, st);
+        launch_general(lc, rows, Q, n, order, h, e, gen, false, sink, R.large, R.sum, st);
         if (c0 + n == M) launch_wide();
         prof_span(SPAN_VOLUME, false, st);
         launch_rows(k_rows_volume<QT, Rows, Sink, VOCC>, lc, n, GPB * sizeof(VolWS),
-                    &R.sum->work[WORK_VOLUME], true, st, rows, Q, R.order + c0, n, (const RowHead *)h, (const RowEntry *)e, gen + gen_room,
+                    &R.sum->work[WORK_VOLUME], true, st, rows, Q, order, n, (const RowHead *)h, (const RowEntry *)e, gen + gen_room,
                     false, sink, LargeQueue{R.large}, R.sum);
-        launch_general(lc, rows, Q, n, R.order + c0, h, e, gen + gen_room, true, sink, R.large, R.sum, st);
+        launch_general(lc, rows, Q, n, order, h, e, gen + gen_room, true, sink, R.large, R.sum, st);
         prof_span(SPAN_VOLUME, true, st);
     }
 }
@@ -2476,13 +2503,13 @@ void run_rows(const nif_dmesh *m, const QT *Q, int64_t M, const Centroid &cen, c
               const Sink &sink, cudaStream_t st, int large_groups = LARGE_GROUPS,
               const RecordLayout *rec = nullptr) {
     if (m->view.pmode == PRED_FAST && rec)
-        launch_fast<QT, Sink, PM_PLAIN>(m, Q, M, cen, all_rows(L), sink, st, rec->heads, rec->ents,
+        launch_fast<QT, Sink, PM_PLAIN>(m, Q, M, cen, all_rows(m, L, M), sink, st, rec->heads, rec->ents,
                                         L.wide, L.gen, true);
     else if (m->view.pmode == PRED_FAST)
-        launch_fast<QT, Sink, PM_PLAIN>(m, Q, M, cen, all_rows(L), sink, st, L.heads, L.ents, L.wide,
+        launch_fast<QT, Sink, PM_PLAIN>(m, Q, M, cen, all_rows(m, L, M), sink, st, L.heads, L.ents, L.wide,
                                         L.gen);
     else
-        launch_fast<QT, Sink, PM_FILTER>(m, Q, M, cen, all_rows(L), sink, st, L.heads, L.ents, L.wide,
+        launch_fast<QT, Sink, PM_FILTER>(m, Q, M, cen, all_rows(m, L, M), sink, st, L.heads, L.ents, L.wide,
                                         L.gen);
     prof_mark(2, st);
     k_rows_large<QT, Sink><<<large_groups, 32, 0, st>>>(m->view, Q, cen, LargeQueue{L.large_list},
@@ -2591,6 +2618,7 @@ NIF_EXPORT int nif_dmesh_create(const double *d_vxyz, const int32_t *d_tet_v,
         delete h;
         return NIF_ERR_CUDA;
     }
+    h->iota = L.iota;
     MeshView &V = h->view;
     V.vtx = L.vtx;
     V.tv = L.tv;
@@ -2613,6 +2641,7 @@ NIF_EXPORT int nif_dmesh_create(const double *d_vxyz, const int32_t *d_tet_v,
     int rc = NIF_OK;
     do {
         if (cudaMemsetAsync(L.flag, 0, 4 * sizeof(int), st) != cudaSuccess) { rc = NIF_ERR_CUDA; break; }
+        k_iota<<<blocks_for(IDENTITY_ROWS, 256), 256, 0, st>>>((int)IDENTITY_ROWS, L.iota);
         k_prep_vertices<<<blocks_for(n_vertices, 256), 256, 0, st>>>(d_vxyz, n_vertices, L.vtx);
         k_prep_tets<<<blocks_for(n_tets, 256), 256, 0, st>>>(d_tet_v, d_tet_n, n_vertices, n_tets,
                                                              L.tv, L.tn, L.flag);
@@ -2703,12 +2732,14 @@ NIF_EXPORT int nif_dmesh_create(const double *d_vxyz, const int32_t *d_tet_v,
             int32_t *vin = T.idx_a, *vout = T.idx_b;
             for (int word = 0; word < 2; word++) {
                 if (word == 1) k_gather_key<<<nb, 256, 0, st>>>(T.chi, vin, n_tets, kin);
-                for (int pass = 0; pass < 8; pass++) {
-                    k_rs_hist<<<(unsigned)T.nblocks, RS_THREADS, 0, st>>>(kin, n_tets, 4 * pass,
+                constexpr RsPlan rs = rs_plan(32);
+                for (int pass = 0; pass < rs.passes; pass++) {
+                    const int shift = rs.bits * pass, bins = 1 << rs.bits;
+                    k_rs_hist<<<(unsigned)T.nblocks, RS_THREADS, 0, st>>>(kin, n_tets, shift, bins,
                                                                            (int)T.nblocks, T.hist);
-                    launch_scan<int>(T.hist, 16 * T.nblocks, T.bsum, T.tot, T.off, st);
+                    launch_scan<int>(T.hist, bins * T.nblocks, T.bsum, T.tot, T.off, st);
                     k_rs_scatter<<<(unsigned)T.nblocks, RS_THREADS, 0, st>>>(
-                        kin, vin, n_tets, 4 * pass, (int)T.nblocks, T.off, kout, vout);
+                        kin, vin, n_tets, shift, bins, (int)T.nblocks, T.off, kout, vout);
                     std::swap(kin, kout);
                     std::swap(vin, vout);
                 }
@@ -3258,7 +3289,7 @@ struct CscLayout {
 CscLayout carve_csc(Carve &c, int64_t nnz, int64_t N) {
     CscLayout L{};
     const int64_t nb = (nnz + RS_TILE - 1) / RS_TILE;
-    const int64_t nh = 16 * (nb > 0 ? nb : 1);
+    const int64_t nh = RS_BINS * (nb > 0 ? nb : 1);
     L.rowof = c.take<int32_t>(nnz > 0 ? nnz : 1);
     L.idx_a = c.take<int32_t>(nnz > 0 ? nnz : 1);
     L.idx_b = c.take<int32_t>(nnz > 0 ? nnz : 1);
@@ -3320,7 +3351,7 @@ int spmm_t_impl(int64_t M, int64_t N, int64_t nnz, const int32_t *d_rowptr, cons
     Carve c{reinterpret_cast<unsigned char *>(d_ws), 0, ws_bytes, true};
     CscLayout L = carve_csc(c, nnz, N);
     if (M > 0)
-        k_row_of<<<blocks_for(M, 256), 256, 0, st>>>(M, d_rowptr, L.rowof, L.key_a, d_cols, L.idx_a,
+        k_row_of<<<blocks_for(8 * M, 256), 256, 0, st>>>(M, d_rowptr, L.rowof, L.key_a, d_cols, L.idx_a,
                                                       d_key_rank, N);
     const int32_t *inv = nullptr;
     if (d_key_rank && N > 0) {
@@ -3328,18 +3359,18 @@ int spmm_t_impl(int64_t M, int64_t N, int64_t nnz, const int32_t *d_rowptr, cons
         k_rank_inverse<<<blocks_for(N, 256), 256, 0, st>>>(N, d_key_rank, L.inv);
         inv = L.inv;
     }
-    // stable sort by column over as many 4-bit digits as the column count needs
+    // stable sort by column over as many bits as the column count needs
     int bits = 0;
     while (bits < 32 && ((int64_t)1 << bits) < N) bits++;
-    const int passes = (bits + 3) / 4;
+    const RsPlan rs = rs_plan(bits);
     uint32_t *kin = L.key_a, *kout = L.key_b;
     int32_t *vin = L.idx_a, *vout = L.idx_b;
     const int64_t nblocks = (nnz + RS_TILE - 1) / RS_TILE;
-    for (int pass = 0; pass < passes && nnz > 0; pass++) {
-        const int shift = 4 * pass;
-        k_rs_hist<<<(unsigned)nblocks, RS_THREADS, 0, st>>>(kin, nnz, shift, (int)nblocks, L.hist);
-        launch_scan<int>(L.hist, 16 * nblocks, L.bsum, L.total, L.off, st);
-        k_rs_scatter<<<(unsigned)nblocks, RS_THREADS, 0, st>>>(kin, vin, nnz, shift, (int)nblocks,
+    for (int pass = 0; pass < rs.passes && nnz > 0; pass++) {
+        const int shift = rs.bits * pass, bins = 1 << rs.bits;
+        k_rs_hist<<<(unsigned)nblocks, RS_THREADS, 0, st>>>(kin, nnz, shift, bins, (int)nblocks, L.hist);
+        launch_scan<int>(L.hist, bins * nblocks, L.bsum, L.total, L.off, st);
+        k_rs_scatter<<<(unsigned)nblocks, RS_THREADS, 0, st>>>(kin, vin, nnz, shift, bins, (int)nblocks,
                                                                 L.off, kout, vout);
         uint32_t *tk = kin; kin = kout; kout = tk;
         int32_t *tv = vin; vin = vout; vout = tv;
@@ -3409,15 +3440,16 @@ void grad_records_typed(const nif_dmesh *m, const void *q, int64_t M, const Cent
     for (int64_t c0 = 0; c0 < M; c0 += REC_CHUNK) {
         const int64_t n = min((int64_t)REC_CHUNK, M - c0);
         const bool last = c0 + n == M;
+        const int *order = row_order(m, L, M) + c0;
         if (last) {
             const RowSet W{L.wide, &L.sum->wide_count, R.requeue, R.sum, nullptr, nullptr, false};
             launch_fast_loc<QT, Sink, PM_PLAIN>(m, Q, M, cen, W, sink, st);
         }
         launch_rows(k_rows_volume<QT, OneMesh, Sink, Sink::VOL_BLOCKS>, lc, n, GPB * sizeof(VolWS),
-                    &R.sum->work[WORK_VOLUME], last, st, rows, Q, L.order + c0, n,
+                    &R.sum->work[WORK_VOLUME], last, st, rows, Q, order, n,
                     (const RowHead *)(R.heads + c0), (const RowEntry *)(R.ents + c0 * REC_CAV), gen_end, true,
                     sink, LargeQueue{R.requeue}, R.sum);
-        launch_general(lc, rows, Q, n, L.order + c0, R.heads + c0, R.ents + c0 * REC_CAV, gen_end, true, sink,
+        launch_general(lc, rows, Q, n, order, R.heads + c0, R.ents + c0 * REC_CAV, gen_end, true, sink,
                        R.requeue, R.sum, st);
         if (!last)  // the next chunk's counter and queue
             cudaMemsetAsync(&R.sum->work[WORK_VOLUME], 0, sizeof(unsigned long long) + 2 * sizeof(int), st);

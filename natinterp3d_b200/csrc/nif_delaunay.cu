@@ -309,6 +309,12 @@ __global__ void k_check_inside(Dev D) {
 // ---------------------------------------------------------------------------
 // one insertion round
 
+// A round's kernels are launched ahead of their predecessors' end (launch_next):
+// each starts with the wait for it.
+__device__ __forceinline__ void after_previous() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 // A build that is finished or has failed: the rest of the rounds the host has
 // enqueued do nothing.
 __device__ __forceinline__ bool over(const Dev &D) {
@@ -317,6 +323,7 @@ __device__ __forceinline__ bool over(const Dev &D) {
 
 // (also clears the round's counters: their last readers are done)
 __global__ void k_nominate(Dev D, int round) {
+    after_previous();
     if (over(D)) return;
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         if (round > 1 && D.st->nwin == 0) set_err(D.st, ERR_CAPACITY);  // no way on
@@ -332,6 +339,7 @@ __global__ void k_nominate(Dev D, int round) {
 }
 
 __global__ void k_collect(Dev D, int round) {
+    after_previous();
     if (over(D)) return;
     for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < D.n; p += gridDim.x * blockDim.x) {
         const int t = D.ptet[p];
@@ -383,6 +391,7 @@ __device__ int h_find(const CavWS &w, int t) {
 
 // The cavity of every nominee and its claims.  One warp per nominee.
 __global__ void __launch_bounds__(THREADS) k_cavity(Dev D, int round) {
+    after_previous();
     __shared__ CavWS wsv[WARPS];
     CavWS &w = wsv[threadIdx.x >> 5];
     const int lane = threadIdx.x & 31;
@@ -576,6 +585,7 @@ struct InsWS {
 // and two winners' tets are disjoint, so that a nominee can be checked while
 // another is inserted.)
 __global__ void __launch_bounds__(THREADS) k_insert(Dev D, int round) {
+    after_previous();
     extern __shared__ __align__(16) unsigned char smem[];
     InsWS &w = reinterpret_cast<InsWS *>(smem)[threadIdx.x >> 5];
     const int lane = threadIdx.x & 31;
@@ -667,6 +677,7 @@ __global__ void __launch_bounds__(THREADS) k_insert(Dev D, int round) {
 }
 
 __global__ void k_reloc_collect(Dev D, int round) {
+    after_previous();
     if (over(D)) return;
     for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < D.n; p += gridDim.x * blockDim.x) {
         const int t = D.ptet[p];
@@ -679,6 +690,7 @@ __global__ void k_reloc_collect(Dev D, int round) {
 // star), so that a key takes one step where a walk through the star took several
 // in a row.  Exact signs; a key on a common face takes the first.
 __global__ void __launch_bounds__(THREADS) k_relocate(Dev D) {
+    after_previous();
     const int lane = threadIdx.x & 31;
     const int warps = (gridDim.x * blockDim.x) >> 5;
     if (over(D)) return;
@@ -901,6 +913,23 @@ Layout carve(Carve &c, int n, int cap) {
     return L;
 }
 
+// a launch whose set-up overlaps the end of the launch before it; the kernel
+// waits for that itself (after_previous)
+template <class... Params, class... Args>
+void launch_next(void (*kern)(Params...), int blocks, int threads, size_t smem, cudaStream_t st, Args... args) {
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)blocks);
+    cfg.blockDim = dim3((unsigned)threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, kern, args...);
+}
+
 int rc_of(cudaError_t e) { return e == cudaSuccess ? NIF_OK : NIF_ERR_CUDA; }
 
 }  // namespace dt
@@ -976,12 +1005,12 @@ NIF_EXPORT int nif_delaunay_build(const double *d_keys, int n, void *d_ws, size_
         }
         for (int k = 0; k < ROUND_BATCH; k++) {
             ++round;
-            k_nominate<<<pblocks, 256, 0, st>>>(D, round);
-            k_collect<<<pblocks, 256, 0, st>>>(D, round);
-            k_cavity<<<wblocks, THREADS, 0, st>>>(D, round);
-            k_insert<<<wblocks, THREADS, ins_smem, st>>>(D, round);
-            k_reloc_collect<<<pblocks, 256, 0, st>>>(D, round);
-            k_relocate<<<wblocks, THREADS, 0, st>>>(D);
+            launch_next(k_nominate, pblocks, 256, 0, st, D, round);
+            launch_next(k_collect, pblocks, 256, 0, st, D, round);
+            launch_next(k_cavity, wblocks, THREADS, 0, st, D, round);
+            launch_next(k_insert, wblocks, THREADS, ins_smem, st, D, round);
+            launch_next(k_reloc_collect, pblocks, 256, 0, st, D, round);
+            launch_next(k_relocate, wblocks, THREADS, 0, st, D);
         }
         DT_CHECK(cudaGetLastError());
         DT_CHECK(cudaMemcpyAsync(&h, D.st, sizeof(State), cudaMemcpyDeviceToHost, st));
