@@ -1376,6 +1376,7 @@ template <class QT, class Sink, int PM, int OCC>
 __global__ void __launch_bounds__(FAST_BLOCK, OCC) k_rows_fast(MeshView M, const QT *__restrict__ Q,
                                                           Centroid cen, const int *__restrict__ order,
                                                           int64_t nrows, const int *nrows_dev,
+                                                          const int *__restrict__ located,
                                                           Sink sink, LargeQueue lq,
                                                           DevSummary *sum, int tile,
                                                           unsigned long long *counter) {
@@ -1403,7 +1404,8 @@ __global__ void __launch_bounds__(FAST_BLOCK, OCC) k_rows_fast(MeshView M, const
         }
         const int64_t i = order[s];
         const dv3 q = load_query(Q, i, cen.c);
-        const RowInfo r = sibson_row<G, FastWS, Sink::FULL, PM>(M, q, ws, g);
+        const RowInfo r = sibson_row<G, FastWS, Sink::FULL, PM>(M, q, ws, g, nullptr,
+                                                               located ? located[i] : -1);
         steps += r.steps;
         if (r.status == ST_CAPACITY || r.status == ST_UNCERTAIN) {
             if (g.lane == 0) {
@@ -2000,11 +2002,11 @@ size_t fcc_slots(int nt) {
     return need > 4 * (size_t)nt ? need : 4 * (size_t)nt;
 }
 
-// Calls of at most this many rows take them as they come: every warp then has
-// one row, so that their order decides nothing, and the bucketing's six
-// launches are left out (with the work counters cleared together, 64 rows took 15
-// launches and take 10).
-constexpr int64_t IDENTITY_ROWS = 4096;
+// Calls of at most this many rows take them as they come: a warp has a few rows
+// at most, so that their order decides little, and the bucketing's six launches
+// are left out (5,003 rows on 50k keys 237 to 214 us a call, 14,003 rows 284 to
+// 261 us).
+constexpr int64_t IDENTITY_ROWS = 16384;
 
 struct MeshLayout {
     int *iota;                   // 0, 1, ... IDENTITY_ROWS - 1: such a call's order
@@ -2286,7 +2288,7 @@ struct RowSet {
     int *large;
     DevSummary *sum;
     unsigned long long *counter;  // to clear before the launch; null: sum->work, clear already
-    const int *located;  // k_locate's tets of these rows, or null (the row kernel locates)
+    const int *located;  // k_locate's tets by row, or null (the row kernel locates)
     bool beside;         // start beside the launch before (as launch_rows)
 };
 
@@ -2341,7 +2343,8 @@ void launch_fast_occ(const nif_dmesh *m, const QT *Q, int64_t M, const Centroid 
     if (blocks > cap) blocks = cap;
     if (blocks < 1) blocks = 1;
     if (tile > 0 && R.counter) cudaMemsetAsync(R.counter, 0, sizeof(unsigned long long), st);
-    launch_beside(kern, (unsigned)blocks, smem, R.beside, st, m->view, Q, cen, R.order, M, R.nrows_dev, sink,
+    launch_beside(kern, (unsigned)blocks, smem, R.beside, st, m->view, Q, cen, R.order, M, R.nrows_dev,
+                  R.nrows_dev ? R.located : nullptr, sink,
                   LargeQueue{R.large}, R.sum, tile, R.counter ? R.counter : &R.sum->work[WORK_FUSED]);
 }
 
@@ -2476,7 +2479,7 @@ void launch_fast(const nif_dmesh *m, const QT *Q, int64_t M, const Centroid &cen
             // rows whose cavity exceeds a record: the fused row kernel (which
             // queues what exceeds its own capacities for the large kernel)
             auto launch_wide = [&]() {
-                const RowSet W{wide, &R.sum->wide_count, R.large, R.sum, nullptr, nullptr, true};
+                const RowSet W{wide, &R.sum->wide_count, R.large, R.sum, nullptr, R.located, true};
                 prof_span(SPAN_FUSED, false, st);
                 launch_fast_loc<QT, Sink, PM>(m, Q, M, cen, W, sink, st);
                 prof_span(SPAN_FUSED, true, st);
@@ -3442,7 +3445,7 @@ void grad_records_typed(const nif_dmesh *m, const void *q, int64_t M, const Cent
         const bool last = c0 + n == M;
         const int *order = row_order(m, L, M) + c0;
         if (last) {
-            const RowSet W{L.wide, &L.sum->wide_count, R.requeue, R.sum, nullptr, nullptr, false};
+            const RowSet W{L.wide, &L.sum->wide_count, R.requeue, R.sum, nullptr, L.located, false};
             launch_fast_loc<QT, Sink, PM_PLAIN>(m, Q, M, cen, W, sink, st);
         }
         launch_rows(k_rows_volume<QT, OneMesh, Sink, Sink::VOL_BLOCKS>, lc, n, GPB * sizeof(VolWS),
@@ -3634,7 +3637,8 @@ template <class QT, class Sink, int PM, int OCC>
 __global__ void __launch_bounds__(FAST_BLOCK, OCC)
     k_rows_batch(const MeshView *__restrict__ views, const int64_t *__restrict__ qoff, int P,
                  const QT *__restrict__ Q, const double *__restrict__ cens,
-                 const int *__restrict__ order, int64_t nrows, const int *nrows_dev, Sink sink,
+                 const int *__restrict__ order, int64_t nrows, const int *nrows_dev,
+                 const int *__restrict__ located, Sink sink,
                  LargeQueue lq, DevSummary *sum, unsigned long long *counter, int tile) {
     extern __shared__ __align__(16) unsigned char smem[];
     asm volatile("griddepcontrol.launch_dependents;");  // k_rows_volume beside the few wide rows
@@ -3666,7 +3670,7 @@ __global__ void __launch_bounds__(FAST_BLOCK, OCC)
                 cur = p;
             }
             const dv3 q = load_query(Q, i, cens + 3 * p);
-            const RowInfo r = sibson_row<G, FastWS, Sink::FULL, PM>(M, q, ws, g);
+            const RowInfo r = sibson_row<G, FastWS, Sink::FULL, PM>(M, q, ws, g, nullptr, located[i]);
             steps += r.steps;
             if (r.status == ST_CAPACITY || r.status == ST_UNCERTAIN) {
                 if (g.lane == 0) {
@@ -3792,7 +3796,8 @@ void launch_batch_rows_occ(const nif_dbatch *b, const QT *Q, int64_t M, const in
     if (blocks > want) blocks = want;
     if (blocks < 1) blocks = 1;
     launch_beside(kern, (unsigned)blocks, smem, true, st, (const MeshView *)b->d_views, qoff, b->P, Q, cens,
-                  order, M, nrows_dev, sink, LargeQueue{L.large_list}, L.sum, &L.sum->work[WORK_FUSED], tile);
+                  order, M, nrows_dev, (const int *)L.located, sink, LargeQueue{L.large_list}, L.sum,
+                  &L.sum->work[WORK_FUSED], tile);
 }
 
 // the fused batch row kernel over positions [0, M) of `order` (bounded by

@@ -1428,14 +1428,16 @@ __device__ RowInfo row_volumes(const MeshView &M, const dv3 q, W &ws, const Grp<
 // predicate variant (PM_*); PM_RESOLVE needs xs, NIF_EXACT_SCRATCH doubles of
 // global scratch owned by this group.  (The split kernels, k_rows_cavity and
 // k_rows_volume, run the same steps on located rows.)
+// `located`: the row's located tet, or -1 to find it here.
 template <int G, class W, bool FULL = true, int PM = PM_PLAIN>
 __device__ RowInfo sibson_row(const MeshView &M, const dv3 q, W &ws, const Grp<G> &g,
-                              double *xs = nullptr) {
+                              double *xs = nullptr, int located = -1) {
     RowInfo r{ST_OK, 0, 0, false, false, 0.0, 0, 0, 0, 0, 0};
     bool on_face = false;  // PRED_EXACT: a face test of the located tet is exactly zero
 
     // ---- 1. point location -------------------------------------------------
-    const int start = locate<G, PM>(M, q, g, reinterpret_cast<int *>(ws.acc), r, on_face, xs);
+    const int start = located >= 0 ? located
+                                   : locate<G, PM>(M, q, g, reinterpret_cast<int *>(ws.acc), r, on_face, xs);
     if (r.status != ST_OK || r.outside) return r;
 
     // ---- 2. cavity and natinterp3d's visiting order ---------------------------
