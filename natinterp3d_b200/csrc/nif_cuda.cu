@@ -1575,14 +1575,23 @@ __global__ void __launch_bounds__(FAST_BLOCK, OCC)
 // there, and the lanes write the positions back entry by entry.  Rows without
 // a cavity record are left alone.  A warp's replays diverge from one another: a
 // call with fewer rows than 32 for each resident warp spreads them (5,000 rows:
-// 31 us with 32 rows a warp, 17 us with 4).
-constexpr int ORD_WARPS = 2;
-constexpr int ORD_RESIDENT = 16;  // warps a SM holds
+// 31 us with 32 rows a warp, 17 us with 4).  Bound by the shared-memory latency
+// of the replays, so by the warps that fit: 11 KB each with the stack no deeper
+// than a record's faces ask for and its limit kept by one minimum a pop, blocks
+// of one warp (2M rows: 0.89 ms with 16 warps of 14 KB a SM in blocks of two,
+// 0.79 with 11 KB, 0.70 in blocks of one, 0.68 with the minimum in place of a
+// test a push).
+constexpr int ORD_WARPS = 1;
+constexpr int ORD_RESIDENT = 16;  // warps a SM (18 fit; spread over 20 a SM, 5,000 rows take 21 us)
+// A tet is pushed once for each face it shares with a tet visited before it: at
+// most half the record's faces, and the start.  (Neighbour entries that are not
+// mutual could ask for more; the stack then stays at its limit.)
+constexpr int ORD_STACK = 2 * REC_CAV + 1;
 constexpr int ORD_PAD = REC_CAV + 1;  // row stride of the shared tables (banks)
 struct OrderWS {
     int nbr[32][ORD_PAD];
-    int8_t stack[32][4 * REC_CAV + 1];
-    int8_t pos[32][REC_CAV];
+    int8_t stack[32][ORD_STACK + 4];  // one tet's pushes more than the limit
+    int8_t pos[32][REC_CAV + 1];
     int start[33];
 };
 
@@ -1669,6 +1678,7 @@ __global__ void __launch_bounds__(32 * ORD_WARPS) k_rows_order(int64_t nrows, in
                     const int n = (int8_t)((wd >> (8 * f)) & 0xffu);
                     if (n >= 0 && !((vis >> n) & 1ull)) stack[sp++] = (int8_t)n;
                 }
+                sp = min(sp, ORD_STACK);
             }
             if (nbf > VolWS::BF) {
                 heads[s].state = RS_GENERAL;
@@ -2441,12 +2451,12 @@ void launch_split(const Launch &lc, const Rows &rows, const QT *Q, int64_t M, co
         prof_span(SPAN_CAVITY, true, st);
         prof_span(SPAN_ORDER, false, st);
         {
-            // one row a warp while the rows fit the resident warps (14 KB each), up to 32
+            // one row a warp while the rows fit the resident warps (11 KB each), up to 32
             int per = 1;
             while (per < 32 && n > (int64_t)per * ORD_RESIDENT * lc.num_sms) per *= 2;
             const int64_t groups = (n + per - 1) / per;
             int64_t ob = (groups + ORD_WARPS - 1) / ORD_WARPS;
-            if (ob > (int64_t)lc.num_sms * 32) ob = (int64_t)lc.num_sms * 32;
+            if (ob > (int64_t)lc.num_sms * 256) ob = (int64_t)lc.num_sms * 256;
             k_rows_order<<<(unsigned)ob, 32 * ORD_WARPS, ORD_WARPS * sizeof(OrderWS), st>>>(
                 n, per, h, e, gen, R.sum);
         }
