@@ -132,7 +132,10 @@ typedef struct nif_dmesh nif_dmesh;
  * nearest tet centroid, which natinterp3d finds in a k-d tree built by its
  * constructor, delaunay.c:141-159).  (natinterp3d keeps the mesh as pointer-linked
  * structs, delaunay.h:44-70, and re-packs it on first query,
- * natural_insertionfree.c:397-450.) */
+ * natural_insertionfree.c:397-450.)  Meshes of up to 2^26 tets also hold the
+ * terms of their tets' corners in every stolen volume, 512 bytes a tet: a
+ * buffer of 512 * n_tets bytes less is accepted too, its queries compute them
+ * (about 1.3 times as long). */
 int nif_dmesh_bytes(int n_vertices, int n_tets, size_t *bytes);
 
 /* Uploads a mesh: derives the resident arrays in d_buf from the packed
@@ -177,8 +180,9 @@ int nif_dmesh_set_predicates(nif_dmesh *m, int mode);
  * whose query loop is OpenMP `schedule(dynamic, 64)` over Morton-sorted
  * queries, natural_insertionfree.c:856, 866-887.)
  *   blocks_per_sm  resident 4-warp blocks per SM of the shared-memory row
- *                  kernel, one warp per query: 6 (80 registers a thread) or
- *                  8 (64 registers, more spills, more warps hiding latency)
+ *                  kernels, one warp per query: 6 (80 registers a thread) or
+ *                  8 (64 registers, more spills, more warps hiding latency;
+ *                  the volume kernel then takes 7 with 72 registers)
  *   bucket_shift   Morton bucket resolution of the query ordering, in bits per
  *                  axis relative to the size-based default: -2 .. 1
  *   tile           queries a warp takes per work item: 0 = a static grid
@@ -244,10 +248,10 @@ int nif_weights_count(const nif_dmesh *m, const void *d_queries, int query_dtype
 /* Sibson weights, step 2 of 2: writes the CSR arrays d_vals (vals_dtype,
  * nnz) and d_cols (int32, nnz) for the d_rowptr of step 1.  Takes the same
  * queries, dtype, M, centroid and workspace as nif_weights_count (the queries
- * must be unchanged in between).  Rows of up to 24 entries were staged by
+ * must be unchanged in between).  Rows of up to 32 entries were staged by
  * step 1 and are copied; longer rows, and rows the large-capacity kernel
  * handled, are recomputed straight into their slices, so the workspace holds
- * no more than 24 entries a row and no row is limited by a staging arena.
+ * no more than 32 entries a row and no row is limited by a staging arena.
  * Columns of a row appear in natinterp3d's first-seen order.  If
  * d_row_totals is not NULL it receives each row's normaliser (the sum of its
  * stolen volumes, 0 for empty rows; float64 [M]), which nif_query_grad takes

@@ -1732,15 +1732,45 @@ __device__ __forceinline__ bool finish_row(int64_t i, RowInfo &r, RowLanes<IDS> 
     }
 }
 
+// The corner terms of a chunk's record entries, for meshes without the corner
+// table: a warp a row, a lane a corner, written beside the entries for
+// k_rows_volume.  Bound by the gathers of its circumcentres: 1.5 ms a 1M-row
+// chunk, so that a 2M-row call takes 14.7 ms where one with the table takes
+// 11.5 and one that computed the terms in the row kernels 23.2.
+template <class Rows>
+__global__ void __launch_bounds__(FAST_BLOCK)
+    k_rows_terms(const __grid_constant__ Rows rows, const int *__restrict__ order, int64_t nrows,
+                 const RowHead *__restrict__ heads, const RowEntry *__restrict__ ents, d4 *__restrict__ terms) {
+    constexpr int G = FAST_G;
+    constexpr int GPB = FAST_BLOCK / G;
+    __shared__ MeshView sview[GPB];
+    Grp<G> g;
+    int cur = -1;
+    for (int64_t s = (int64_t)blockIdx.x * GPB + threadIdx.x / G; s < nrows; s += (int64_t)gridDim.x * GPB) {
+        const RowHead h = heads[s];
+        if (h.state != RS_OK && h.state != RS_GENERAL) continue;
+        const int n = 4 * min(h.ncav, REC_CAV);
+        const double *cen;
+        const MeshView &M = rows.get(order[s], cur, &sview[threadIdx.x / G], g, cen);
+        if (M.corner) continue;
+        double *const out = reinterpret_cast<double *>(terms + s * REC_CAV);
+        for (int k = g.lane; k < n; k += G) {
+            const RowEntry x = ents[s * REC_CAV + k / 4];
+            out[k] = corner_term(M, x.tet, ((unsigned)x.pos >> 8) & 15u, k & 3);
+        }
+    }
+}
+
 // Rows that split_row_body gives up on (ST_GENERAL) are queued for
 // k_rows_general, by position, from the end of `gen` (gen_end); with `late` so
 // are those that k_rows_order found too large and queued from its start.
-template <class QT, class Rows, class Sink, int OCC>
+template <class QT, class Rows, class Sink, int OCC, bool TERMS>
 __global__ void __launch_bounds__(FAST_BLOCK, OCC)
     k_rows_volume(const __grid_constant__ Rows rows, const QT *__restrict__ Q,
                   const int *__restrict__ order, int64_t nrows, const RowHead *__restrict__ heads,
-                  const RowEntry *__restrict__ ents, int *__restrict__ gen_end, bool late, Sink sink,
-                  LargeQueue lq, DevSummary *sum, int tile, unsigned long long *counter) {
+                  const RowEntry *__restrict__ ents, const d4 *__restrict__ terms,
+                  int *__restrict__ gen_end, bool late, Sink sink, LargeQueue lq, DevSummary *sum, int tile,
+                  unsigned long long *counter) {
     extern __shared__ __align__(16) unsigned char smem[];
     constexpr int G = FAST_G;
     constexpr int GPB = FAST_BLOCK / G;
@@ -1771,7 +1801,8 @@ __global__ void __launch_bounds__(FAST_BLOCK, OCC)
             RowInfo r{ST_OK, 0, 0, h.state == RS_OUTSIDE, false, 0.0, 0, 0, 0, 0, 0};
             RowLanes<1> L;
             if (h.state == RS_OK)
-                split_row_body<G, VolWS, Sink::FULL, false>(M, q, ws, g, h, ents + s * REC_CAV, r, L);
+                split_row_body<G, VolWS, Sink::FULL, false, TERMS>(M, q, ws, g, h, ents + s * REC_CAV,
+                                                                   terms + (TERMS ? s * REC_CAV : 0), r, L);
             if (h.state == RS_WALK) r.status = ST_WALK;
             if (!finish_row(i, r, L, M, q, ws, g, sink, lq, sum) && g.lane == 0)
                 gen_end[-1 - atomicAdd(&sum->late_count, 1)] = (int)s;
@@ -1787,12 +1818,12 @@ __global__ void __launch_bounds__(FAST_BLOCK, OCC)
 // k_rows_volume (`late` = false), those k_rows_volume finds after it: a kernel of
 // its own, because the two bodies together outgrow the instruction cache (with
 // both in one kernel the volume pass took 11.1 ms a 2M-row call, 8.0 ms apart).
-template <class QT, class Rows, class Sink>
+template <class QT, class Rows, class Sink, bool TERMS>
 __global__ void __launch_bounds__(FAST_BLOCK, GEN_OCC)
     k_rows_general(const __grid_constant__ Rows rows, const QT *__restrict__ Q,
                    const int *__restrict__ order, const RowHead *__restrict__ heads,
-                   const RowEntry *__restrict__ ents, const int *__restrict__ gen, bool late, Sink sink,
-                   LargeQueue lq, DevSummary *sum) {
+                   const RowEntry *__restrict__ ents, const d4 *__restrict__ terms,
+                   const int *__restrict__ gen, bool late, Sink sink, LargeQueue lq, DevSummary *sum) {
     extern __shared__ __align__(16) unsigned char smem[];
     asm volatile("griddepcontrol.launch_dependents;");
     constexpr int G = FAST_G;
@@ -1810,7 +1841,8 @@ __global__ void __launch_bounds__(FAST_BLOCK, GEN_OCC)
         const dv3 q = load_query(Q, i, cen);
         RowInfo r{ST_OK, 0, 0, false, false, 0.0, 0, 0, 0, 0, 0};
         RowLanes<2> L;
-        split_row_body<G, GenWS, Sink::FULL, true>(M, q, ws, g, heads[s], ents + s * REC_CAV, r, L);
+        split_row_body<G, GenWS, Sink::FULL, true, TERMS>(M, q, ws, g, heads[s], ents + s * REC_CAV,
+                                                          terms + (TERMS ? s * REC_CAV : 0), r, L);
         finish_row(i, r, L, M, q, ws, g, sink, lq, sum);
         g.sync();
     }
@@ -2024,7 +2056,7 @@ struct MeshLayout {
     int4 *tv, *tn;
     uint32_t *tinfo;
     d4 *tcc, *fcc;
-    d4 *corner;                  // corner terms, null beyond CORNER_TETS_MAX
+    d4 *corner;                  // corner terms, or null
     d4 *cs;                      // sorted centroids
     float4 *onode;               // octree node records, two float4 each
     unsigned long long *omask;   // octree child digits
@@ -2036,13 +2068,15 @@ struct MeshLayout {
 
 // Largest mesh that holds its corner terms: 512 bytes a tet, 34 GB here (about
 // 10M keys), next to 270 bytes a tet for the rest.  Larger meshes, which are to
-// leave room for others' data, compute them per row.
+// leave room for others' data, and those whose caller has no room for the table,
+// compute them per row (k_rows_terms: a 2M-row call takes 14.7 ms, with the
+// table 11.5).
 #ifndef NIF_CORNER_TETS_MAX
 #define NIF_CORNER_TETS_MAX (1 << 26)
 #endif
 constexpr int CORNER_TETS_MAX = NIF_CORNER_TETS_MAX;
 
-MeshLayout carve_mesh(Carve &c, int nv, int nt) {
+MeshLayout carve_mesh(Carve &c, int nv, int nt, bool corner) {
     MeshLayout L;
     L.iota = c.take<int>(IDENTITY_ROWS);
     L.vtx = c.take<d4>(nv);
@@ -2051,7 +2085,7 @@ MeshLayout carve_mesh(Carve &c, int nv, int nt) {
     L.tinfo = c.take<uint32_t>(nt);
     L.tcc = c.take<d4>(nt);
     L.fcc = c.take<d4>(fcc_slots(nt));
-    L.corner = nt <= CORNER_TETS_MAX ? c.take<d4>(16 * (size_t)nt) : nullptr;
+    L.corner = corner ? c.take<d4>(16 * (size_t)nt) : nullptr;
     L.cs = c.take<d4>(nt);
     L.onode = c.take<float4>(2 * (size_t)oct_node_cap(nt));
     L.omask = c.take<unsigned long long>(oct_node_cap(nt));
@@ -2082,6 +2116,7 @@ struct QueryLayout {
     int *located;           // k_locate's tet per row (null: the row kernel locates)
     RowHead *heads;         // split-row records of one chunk of rows
     RowEntry *ents;
+    d4 *terms;              // their corner terms, on a mesh without the table
     int *wide;              // split rows whose cavity exceeds a record
     int *gen;               // one chunk's rows for k_rows_general
     // weights mode only
@@ -2108,7 +2143,7 @@ constexpr int bucket_bits(int64_t M) {
 
 // The layout does not depend on the mesh's tuning: bcount has room for one
 // bucket bit per axis more than the default, and run_bucketing clamps to it.
-QueryLayout carve_query(Carve &c, int64_t M, int mode) {
+QueryLayout carve_query(Carve &c, const nif_dmesh *m, int64_t M, int mode) {
     QueryLayout L{};
     const int bits = min(10, bucket_bits(M) + 1);
     const int64_t nbk = (int64_t)1 << (3 * bits);
@@ -2131,6 +2166,7 @@ QueryLayout carve_query(Carve &c, int64_t M, int mode) {
         L.ents = c.take<RowEntry>(ch * REC_CAV);
         L.wide = c.take<int>(M > 0 ? M : 1);
         L.gen = c.take<int>(ch);
+        if (!m->view.corner) L.terms = c.take<d4>(ch * REC_CAV);
     }
     if (mode == NIF_MODE_WEIGHTS) {
         const int64_t m1 = M > 0 ? M : 1;
@@ -2191,21 +2227,29 @@ int set_smem(Kern k, size_t bytes) {
 // memory, on the current device.  The first call per (kernel, device) sets
 // the kernel's shared-memory limit there and queries the occupancy; the
 // answer is cached, and concurrent first calls from several host threads are
-// serialised.
+// serialised.  Kernels of one signature (template arguments that no parameter
+// shows) share an instance of this function, so the cache tells them apart.
 template <class Kern>
 int resident_blocks(Kern k, int threads, size_t smem) {
-    constexpr int DEVS = 64;
+    constexpr int DEVS = 64, KERNS = 8;
     static std::mutex mu;
-    static int cache[DEVS] = {};
+    static Kern known[KERNS] = {};
+    static int cache[KERNS][DEVS] = {};
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) dev = -1;
     std::lock_guard<std::mutex> lock(mu);
-    if (dev >= 0 && dev < DEVS && cache[dev] > 0) return cache[dev];
+    int slot = 0;
+    while (slot < KERNS && known[slot] && known[slot] != k) slot++;
+    const bool cached = slot < KERNS && dev >= 0 && dev < DEVS;
+    if (cached && cache[slot][dev] > 0) return cache[slot][dev];
     if (smem > 48 * 1024) set_smem(k, smem);
     int n = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k, threads, smem) != cudaSuccess || n < 1)
         n = 1;
-    if (dev >= 0 && dev < DEVS) cache[dev] = n;
+    if (cached) {
+        known[slot] = k;
+        cache[slot][dev] = n;
+    }
     return n;
 }
 
@@ -2405,17 +2449,17 @@ constexpr int sink_occ() {
 }
 
 // k_rows_general over the rows queued from the start of `gen`, or before it (late)
-template <class QT, class Rows, class Sink>
+template <bool TERMS, class QT, class Rows, class Sink>
 void launch_general(const Launch &lc, const Rows &rows, const QT *Q, int64_t n, const int *order,
-                    const RowHead *h, const RowEntry *e, const int *gen, bool late, const Sink &sink,
-                    int *large, DevSummary *sum, cudaStream_t st) {
+                    const RowHead *h, const RowEntry *e, const d4 *terms, const int *gen, bool late,
+                    const Sink &sink, int *large, DevSummary *sum, cudaStream_t st) {
     constexpr int GPB = FAST_BLOCK / FAST_G;
-    auto kern = k_rows_general<QT, Rows, Sink>;
+    auto kern = k_rows_general<QT, Rows, Sink, TERMS>;
     const size_t smem = GPB * sizeof(GenWS);
     const int64_t cap = (int64_t)resident_blocks(kern, FAST_BLOCK, smem) * lc.num_sms;
     const int64_t blocks = min((n + GPB - 1) / GPB, cap);
-    kern<<<(unsigned)blocks, FAST_BLOCK, smem, st>>>(rows, Q, order, h, e, gen, late, sink, LargeQueue{large},
-                                                    sum);
+    kern<<<(unsigned)blocks, FAST_BLOCK, smem, st>>>(rows, Q, order, h, e, terms, gen, late, sink,
+                                                    LargeQueue{large}, sum);
 }
 
 // The split row over positions [0, M) of R.order, whose rows `rows` maps to
@@ -2427,8 +2471,8 @@ void launch_general(const Launch &lc, const Rows &rows, const QT *Q, int64_t n, 
 // rows: a 43 us volume launch and 61 us of wide rows end after 81 us).
 template <class QT, class Rows, class Sink, int OCC, int PM = PM_PLAIN, class Wide>
 void launch_split(const Launch &lc, const Rows &rows, const QT *Q, int64_t M, const RowSet &R,
-                  RowHead *heads, RowEntry *ents, int *wide, int *gen, const Sink &sink, cudaStream_t st,
-                  const Wide &launch_wide, bool keep = false) {
+                  RowHead *heads, RowEntry *ents, d4 *terms, int *wide, int *gen, const Sink &sink,
+                  cudaStream_t st, const Wide &launch_wide, bool keep = false) {
     constexpr int GPB = FAST_BLOCK / FAST_G;
     constexpr int COCC = NIF_CAV_OCC > 0 ? NIF_CAV_OCC : OCC;
     constexpr int VOCC = sink_occ<Sink, (NIF_VOL_OCC > 0 ? NIF_VOL_OCC : (OCC == OCC_HI ? 7 : OCC))>();
@@ -2463,13 +2507,30 @@ void launch_split(const Launch &lc, const Rows &rows, const QT *Q, int64_t M, co
         prof_span(SPAN_ORDER, true, st);
         // the rows already known to be for the general kernel, the last chunk's
         // wide rows and the volumes, beside one another
-        launch_general(lc, rows, Q, n, order, h, e, gen, false, sink, R.large, R.sum, st);
-        if (c0 + n == M) launch_wide();
-        prof_span(SPAN_VOLUME, false, st);
-        launch_rows(k_rows_volume<QT, Rows, Sink, VOCC>, lc, n, GPB * sizeof(VolWS),
-                    &R.sum->work[WORK_VOLUME], true, st, rows, Q, order, n, (const RowHead *)h, (const RowEntry *)e, gen + gen_room,
-                    false, sink, LargeQueue{R.large}, R.sum);
-        launch_general(lc, rows, Q, n, order, h, e, gen + gen_room, true, sink, R.large, R.sum, st);
+        auto volumes = [&](auto with_terms) {
+            constexpr bool TERMS = decltype(with_terms)::value;
+            launch_general<TERMS>(lc, rows, Q, n, order, h, e, terms, gen, false, sink, R.large, R.sum, st);
+            if (c0 + n == M) launch_wide();
+            prof_span(SPAN_VOLUME, false, st);
+            launch_rows(k_rows_volume<QT, Rows, Sink, VOCC, TERMS>, lc, n, GPB * sizeof(VolWS),
+                        &R.sum->work[WORK_VOLUME], true, st, rows, Q, order, n, (const RowHead *)h,
+                        (const RowEntry *)e, (const d4 *)terms, gen + gen_room, false, sink, LargeQueue{R.large},
+                        R.sum);
+            launch_general<TERMS>(lc, rows, Q, n, order, h, e, terms, gen + gen_room, true, sink, R.large, R.sum,
+                                  st);
+        };
+        if constexpr (Sink::FULL) {
+            if (terms) {
+                constexpr int TERM_BLOCKS = 16;  // a SM: enough to balance the rows' lengths
+                const int64_t tb = min((n + GPB - 1) / GPB, (int64_t)TERM_BLOCKS * lc.num_sms);
+                k_rows_terms<Rows><<<(unsigned)tb, FAST_BLOCK, 0, st>>>(rows, order, n, h, e, terms);
+                volumes(std::true_type());
+            } else {
+                volumes(std::false_type());
+            }
+        } else {
+            volumes(std::false_type());
+        }
         prof_span(SPAN_VOLUME, true, st);
     }
 }
@@ -2481,7 +2542,8 @@ void launch_split(const Launch &lc, const Rows &rows, const QT *Q, int64_t M, co
 template <class QT, class Sink, int PM>
 void launch_fast(const nif_dmesh *m, const QT *Q, int64_t M, const Centroid &cen,
                  const RowSet &R, const Sink &sink, cudaStream_t st, RowHead *heads = nullptr,
-                 RowEntry *ents = nullptr, int *wide = nullptr, int *gen = nullptr, bool keep = false) {
+                 RowEntry *ents = nullptr, d4 *terms = nullptr, int *wide = nullptr, int *gen = nullptr,
+                 bool keep = false) {
     if constexpr (PM == PM_PLAIN || PM == PM_FILTER) {
         if (R.located && heads && !R.nrows_dev) {
             const Launch lc{m->tune.tile, m->num_sms};
@@ -2495,10 +2557,10 @@ void launch_fast(const nif_dmesh *m, const QT *Q, int64_t M, const Centroid &cen
                 prof_span(SPAN_FUSED, true, st);
             };
             if (m->tune.blocks_per_sm == OCC_LO)
-                launch_split<QT, OneMesh, Sink, OCC_LO, PM>(lc, rows, Q, M, R, heads, ents, wide, gen,
+                launch_split<QT, OneMesh, Sink, OCC_LO, PM>(lc, rows, Q, M, R, heads, ents, terms, wide, gen,
                                                             sink, st, launch_wide, keep);
             else
-                launch_split<QT, OneMesh, Sink, OCC_HI, PM>(lc, rows, Q, M, R, heads, ents, wide, gen,
+                launch_split<QT, OneMesh, Sink, OCC_HI, PM>(lc, rows, Q, M, R, heads, ents, terms, wide, gen,
                                                             sink, st, launch_wide, keep);
             return;
         }
@@ -2517,13 +2579,13 @@ void run_rows(const nif_dmesh *m, const QT *Q, int64_t M, const Centroid &cen, c
               const RecordLayout *rec = nullptr) {
     if (m->view.pmode == PRED_FAST && rec)
         launch_fast<QT, Sink, PM_PLAIN>(m, Q, M, cen, all_rows(m, L, M), sink, st, rec->heads, rec->ents,
-                                        L.wide, L.gen, true);
+                                        L.terms, L.wide, L.gen, true);
     else if (m->view.pmode == PRED_FAST)
-        launch_fast<QT, Sink, PM_PLAIN>(m, Q, M, cen, all_rows(m, L, M), sink, st, L.heads, L.ents, L.wide,
-                                        L.gen);
+        launch_fast<QT, Sink, PM_PLAIN>(m, Q, M, cen, all_rows(m, L, M), sink, st, L.heads, L.ents, L.terms,
+                                        L.wide, L.gen);
     else
-        launch_fast<QT, Sink, PM_FILTER>(m, Q, M, cen, all_rows(m, L, M), sink, st, L.heads, L.ents, L.wide,
-                                        L.gen);
+        launch_fast<QT, Sink, PM_FILTER>(m, Q, M, cen, all_rows(m, L, M), sink, st, L.heads, L.ents, L.terms,
+                                        L.wide, L.gen);
     prof_mark(2, st);
     k_rows_large<QT, Sink><<<large_groups, 32, 0, st>>>(m->view, Q, cen, LargeQueue{L.large_list},
                                                         sink, L.large_ws, L.exact, L.sum);
@@ -2600,7 +2662,7 @@ constexpr int MAX_TETS = INT_MAX / 4;
 NIF_EXPORT int nif_dmesh_bytes(int n_vertices, int n_tets, size_t *bytes) {
     if (!bytes || n_vertices < 5 || n_tets < 1 || n_tets > MAX_TETS) return NIF_ERR_ARG;
     Carve c{nullptr, 0, (size_t)-1, true};
-    carve_mesh(c, n_vertices, n_tets);
+    carve_mesh(c, n_vertices, n_tets, n_tets <= CORNER_TETS_MAX);
     *bytes = align_up(c.off, 256);
     return NIF_OK;
 }
@@ -2616,10 +2678,15 @@ NIF_EXPORT int nif_dmesh_create(const double *d_vxyz, const int32_t *d_tet_v,
     if (reinterpret_cast<uintptr_t>(d_buf) % 256 != 0) return NIF_ERR_ARG;
     size_t need = 0;
     nif_dmesh_bytes(n_vertices, n_tets, &need);
+    bool corner = n_tets <= CORNER_TETS_MAX;
+    if (corner && buf_bytes < need) {  // no room for the corner terms
+        need -= 16 * sizeof(d4) * (size_t)n_tets;
+        corner = false;
+    }
     if (buf_bytes < need) return NIF_ERR_WORKSPACE;
     cudaStream_t st = S(stream);
     Carve c{reinterpret_cast<unsigned char *>(d_buf), 0, buf_bytes, true};
-    MeshLayout L = carve_mesh(c, n_vertices, n_tets);
+    MeshLayout L = carve_mesh(c, n_vertices, n_tets, corner);
 
     nif_dmesh *h = new (std::nothrow) nif_dmesh();
     if (!h) return NIF_ERR_NOMEM;
@@ -2891,7 +2958,7 @@ NIF_EXPORT int nif_query_workspace_bytes(const nif_dmesh *m, int64_t M, int mode
     if (!m || !bytes || M < 0 || (mode != NIF_MODE_WEIGHTS && mode != NIF_MODE_INTERP))
         return NIF_ERR_ARG;
     Carve c{nullptr, 0, (size_t)-1, true};
-    carve_query(c, M, mode);
+    carve_query(c, m, M, mode);
     *bytes = align_up(c.off, 256);
     return NIF_OK;
 }
@@ -2916,7 +2983,7 @@ int weights_count(const nif_dmesh *m, const void *d_queries, int query_dtype, in
     if (ws_bytes < need) return NIF_ERR_WORKSPACE;
     cudaStream_t st = S(stream);
     Carve c{reinterpret_cast<unsigned char *>(d_ws), 0, ws_bytes, true};
-    QueryLayout L = carve_query(c, M, NIF_MODE_WEIGHTS);
+    QueryLayout L = carve_query(c, m, M, NIF_MODE_WEIGHTS);
     Centroid cen{{centroid[0], centroid[1], centroid[2]}};
     NIF_CUDA(cudaMemsetAsync(L.sum, 0, sizeof(DevSummary), st));
     if (M > 0) {
@@ -2999,7 +3066,7 @@ NIF_EXPORT int nif_weights_fill(const nif_dmesh *m, const void *d_queries, int q
     if (!d_vals || !d_cols) return NIF_ERR_ARG;
     cudaStream_t st = S(stream);
     Carve c{reinterpret_cast<unsigned char *>(const_cast<void *>(d_ws)), 0, ws_bytes, true};
-    QueryLayout L = carve_query(c, M, NIF_MODE_WEIGHTS);
+    QueryLayout L = carve_query(c, m, M, NIF_MODE_WEIGHTS);
     Centroid cen{{centroid[0], centroid[1], centroid[2]}};
     if (d_row_totals)
         NIF_CUDA(cudaMemcpyAsync(d_row_totals, L.rtot, sizeof(double) * M, cudaMemcpyDeviceToDevice, st));
@@ -3037,7 +3104,7 @@ NIF_EXPORT int nif_interpolate(const nif_dmesh *m, const void *d_queries, int qu
     if (ws_bytes < need) return NIF_ERR_WORKSPACE;
     cudaStream_t st = S(stream);
     Carve c{reinterpret_cast<unsigned char *>(d_ws), 0, ws_bytes, true};
-    QueryLayout L = carve_query(c, M, NIF_MODE_INTERP);
+    QueryLayout L = carve_query(c, m, M, NIF_MODE_INTERP);
     Centroid cen{{centroid[0], centroid[1], centroid[2]}};
     NIF_CUDA(cudaMemsetAsync(L.sum, 0, sizeof(DevSummary), st));
     if (M > 0) {
@@ -3458,11 +3525,12 @@ void grad_records_typed(const nif_dmesh *m, const void *q, int64_t M, const Cent
             const RowSet W{L.wide, &L.sum->wide_count, R.requeue, R.sum, nullptr, L.located, false};
             launch_fast_loc<QT, Sink, PM_PLAIN>(m, Q, M, cen, W, sink, st);
         }
-        launch_rows(k_rows_volume<QT, OneMesh, Sink, Sink::VOL_BLOCKS>, lc, n, GPB * sizeof(VolWS),
+        launch_rows(k_rows_volume<QT, OneMesh, Sink, Sink::VOL_BLOCKS, false>, lc, n, GPB * sizeof(VolWS),
                     &R.sum->work[WORK_VOLUME], last, st, rows, Q, order, n,
-                    (const RowHead *)(R.heads + c0), (const RowEntry *)(R.ents + c0 * REC_CAV), gen_end, true,
+                    (const RowHead *)(R.heads + c0), (const RowEntry *)(R.ents + c0 * REC_CAV),
+                    (const d4 *)nullptr, gen_end, true,
                     sink, LargeQueue{R.requeue}, R.sum);
-        launch_general(lc, rows, Q, n, order, R.heads + c0, R.ents + c0 * REC_CAV, gen_end, true, sink,
+        launch_general<false>(lc, rows, Q, n, order, R.heads + c0, R.ents + c0 * REC_CAV, nullptr, gen_end, true, sink,
                        R.requeue, R.sum, st);
         if (!last)  // the next chunk's counter and queue
             cudaMemsetAsync(&R.sum->work[WORK_VOLUME], 0, sizeof(unsigned long long) + 2 * sizeof(int), st);
@@ -3494,7 +3562,7 @@ NIF_EXPORT int nif_query_grad_records(const nif_dmesh *m, const void *d_queries,
     if (records_bytes < rneed) return NIF_ERR_WORKSPACE;
     cudaStream_t st = S(stream);
     Carve c{reinterpret_cast<unsigned char *>(const_cast<void *>(d_ws)), 0, ws_bytes, true};
-    const QueryLayout L = carve_query(c, M, NIF_MODE_WEIGHTS);
+    const QueryLayout L = carve_query(c, m, M, NIF_MODE_WEIGHTS);
     Carve cr{static_cast<unsigned char *>(d_records), 0, records_bytes, true};
     const RecordLayout R = carve_records(cr, M);
     Centroid cen{{centroid[0], centroid[1], centroid[2]}};
@@ -3537,7 +3605,7 @@ NIF_EXPORT int nif_query_grad(const nif_dmesh *m, const void *d_queries, int que
     if (ws_bytes < need) return NIF_ERR_WORKSPACE;
     cudaStream_t st = S(stream);
     Carve c{reinterpret_cast<unsigned char *>(d_ws), 0, ws_bytes, true};
-    QueryLayout L = carve_query(c, M, NIF_MODE_INTERP);
+    QueryLayout L = carve_query(c, m, M, NIF_MODE_INTERP);
     Centroid cen{{centroid[0], centroid[1], centroid[2]}};
     NIF_CUDA(cudaMemsetAsync(L.sum, 0, sizeof(DevSummary), st));
     if (M > 0) {
@@ -3749,6 +3817,7 @@ struct nif_dbatch {
     int device;
     int num_sms;
     bool filtered;      // some mesh uses a non-default predicate mode
+    bool untabled;      // some mesh has no corner table
     MeshView *d_views;  // [P] in the caller's buffer
     nif_tuning tune{OCC_DEFAULT, 0, BATCH_TILE_DEFAULT, 0};
 };
@@ -3766,9 +3835,10 @@ struct BatchLayout {
     int *located, *wide, *gen;
     RowHead *heads;
     RowEntry *ents;
+    d4 *terms;  // with `terms`: one chunk's corner terms
 };
 
-BatchLayout carve_batch(Carve &c, int P, int64_t M) {
+BatchLayout carve_batch(Carve &c, int P, int64_t M, bool terms) {
     BatchLayout L{};
     const int64_t nbk = 8 * (int64_t)P + M / 2 + 1;
     L.sum = c.take<DevSummary>(1);
@@ -3789,6 +3859,7 @@ BatchLayout carve_batch(Carve &c, int P, int64_t M) {
     L.heads = c.take<RowHead>(ch);
     L.ents = c.take<RowEntry>(ch * REC_CAV);
     L.gen = c.take<int>(ch);
+    L.terms = terms ? c.take<d4>(ch * REC_CAV) : nullptr;
     return L;
 }
 
@@ -3847,7 +3918,7 @@ void batch_typed(const nif_dbatch *b, const void *q, int64_t M, const int64_t *q
     auto split = [&](auto pm, auto occ) {
         constexpr int PM = decltype(pm)::value, OCC = decltype(occ)::value;
         launch_split<QT, ManyMeshes, Sink, OCC, PM>(
-            lc, rows, Q, M, R, L.heads, L.ents, L.wide, L.gen, sink, st,
+            lc, rows, Q, M, R, L.heads, L.ents, L.terms, L.wide, L.gen, sink, st,
             [&]() { launch_batch_rows<QT, Sink, PM>(b, Q, M, qoff, cens, sink, L, st, L.wide, &L.sum->wide_count); });
     };
     auto by_occ = [&](auto pm) {
@@ -3895,7 +3966,7 @@ NIF_EXPORT int nif_batch_create(int n_problems, nif_dmesh *const *meshes, void *
     MeshView *host = static_cast<MeshView *>(malloc(sizeof(MeshView) * (size_t)n_problems));
     if (!host) return NIF_ERR_NOMEM;
     int dev = -1;
-    bool filtered = false;
+    bool filtered = false, untabled = false;
     for (int p = 0; p < n_problems; p++) {
         if (!meshes[p] || (p > 0 && meshes[p]->device != dev)) {
             free(host);
@@ -3904,6 +3975,7 @@ NIF_EXPORT int nif_batch_create(int n_problems, nif_dmesh *const *meshes, void *
         dev = meshes[p]->device;
         host[p] = meshes[p]->view;  // predicate modes as of now
         filtered = filtered || host[p].pmode != PRED_FAST;
+        untabled = untabled || !host[p].corner;
     }
     cudaStream_t st = S(stream);
     if (cudaMemcpyAsync(d_buf, host, sizeof(MeshView) * (size_t)n_problems, cudaMemcpyHostToDevice, st) !=
@@ -3919,6 +3991,7 @@ NIF_EXPORT int nif_batch_create(int n_problems, nif_dmesh *const *meshes, void *
     b->device = dev;
     b->num_sms = meshes[0]->num_sms;
     b->filtered = filtered;
+    b->untabled = untabled;
     b->d_views = static_cast<MeshView *>(d_buf);
     *out = b;
     return NIF_OK;
@@ -3929,7 +4002,7 @@ NIF_EXPORT void nif_batch_destroy(nif_dbatch *b) { delete b; }
 NIF_EXPORT int nif_batch_workspace_bytes(const nif_dbatch *b, int64_t total_queries, size_t *bytes) {
     if (!b || !bytes || total_queries < 0 || total_queries > (int64_t)INT32_MAX) return NIF_ERR_ARG;
     Carve c{nullptr, 0, (size_t)-1, true};
-    carve_batch(c, b->P, total_queries);
+    carve_batch(c, b->P, total_queries, b->untabled);
     *bytes = align_up(c.off, 256);
     return NIF_OK;
 }
@@ -3952,7 +4025,7 @@ NIF_EXPORT int nif_batch_interpolate(const nif_dbatch *b, const void *d_queries,
     if (ws_bytes < need) return NIF_ERR_WORKSPACE;
     cudaStream_t st = S(stream);
     Carve c{reinterpret_cast<unsigned char *>(d_ws), 0, ws_bytes, true};
-    BatchLayout L = carve_batch(c, b->P, total_queries);
+    BatchLayout L = carve_batch(c, b->P, total_queries, b->untabled);
     if (total_queries == 0) return cuda_rc(cudaMemsetAsync(L.sum, 0, sizeof(DevSummary), st));
     const int64_t M = total_queries;
     if (query_dtype == NIF_F64 && values_dtype == NIF_F64)
@@ -3977,7 +4050,7 @@ NIF_EXPORT int nif_batch_summary(const nif_dbatch *b, int64_t total_queries, con
     if (nif_batch_workspace_bytes(b, total_queries, &need) != NIF_OK || ws_bytes < need)
         return NIF_ERR_WORKSPACE;
     Carve c{reinterpret_cast<unsigned char *>(const_cast<void *>(d_ws)), 0, ws_bytes, true};
-    BatchLayout L = carve_batch(c, b->P, total_queries);
+    BatchLayout L = carve_batch(c, b->P, total_queries, b->untabled);
     DevSummary d;
     cudaStream_t st = S(stream);
     NIF_CUDA(cudaMemcpyAsync(&d, L.sum, sizeof(d), cudaMemcpyDeviceToHost, st));
@@ -4004,6 +4077,6 @@ NIF_EXPORT int nif_query_summary(const nif_dmesh *m, int64_t M, int mode, const 
     if (rc != NIF_OK) return rc;
     if (ws_bytes < need) return NIF_ERR_WORKSPACE;
     Carve c{reinterpret_cast<unsigned char *>(const_cast<void *>(d_ws)), 0, ws_bytes, true};
-    QueryLayout L = carve_query(c, M, mode);
+    QueryLayout L = carve_query(c, m, M, mode);
     return read_summary(L, S(stream), summary, nullptr);
 }

@@ -1621,7 +1621,8 @@ __device__ __forceinline__ int flood_pair(const MeshView &M, const dv3 q, W &ws,
 // nothing but the mesh and the mask, so that meshes of up to CORNER_TETS_MAX
 // tets hold all of them (MeshView::corner, four a tet and mask: a cavity tet
 // is one 32-byte sector to a row instead of four vertices, five circumcentres
-// and some 110 FP64 operations a corner).
+// and some 110 FP64 operations a corner).  For larger meshes k_rows_terms writes
+// them beside the records of a chunk.
 __device__ __forceinline__ double corner_term(const MeshView &M, int t, unsigned mask, int vi) {
     const int4 p = M.tv[t];
     const int4 n = M.tn[t];
@@ -1637,14 +1638,6 @@ __device__ __forceinline__ double corner_term(const MeshView &M, int t, unsigned
     const int o0 = vi == 0 ? 1 : 0, o1 = vi <= 1 ? 2 : 1, o2 = vi <= 2 ? 3 : 2;
     return subcell_volume(vload(M, comp(p, vi)), vload(M, comp(p, o0)), vload(M, comp(p, o1)),
                           vload(M, comp(p, o2)), cload(&M.tcc[t]), face(o2), face(o1), face(o0));
-}
-
-// all four, out of line, for the rows of a mesh without the table
-__device__ __noinline__ d4 corner_terms_direct(const MeshView &M, int t, unsigned mask) {
-    double v[4];
-#pragma unroll 1
-    for (int i = 0; i < 4; i++) v[i] = corner_term(M, t, mask, i);
-    return d4{v[0], v[1], v[2], v[3]};
 }
 
 // the ids of a face's three vertices, one byte each, from its tet's ids
@@ -1717,10 +1710,12 @@ struct RowLanes {
     }
 };
 
-template <int G, class W, bool FULL, bool GENERAL, int IDS>
+// TERMS: the row's corner terms are at ent_terms, by entry, on meshes without the table.
+template <int G, class W, bool FULL, bool GENERAL, bool TERMS, int IDS>
 __device__ __forceinline__ void split_row_body(const MeshView &M, const dv3 q, W &ws, const Grp<G> &g,
                                                const RowHead &head, const RowEntry *__restrict__ ent,
-                                               RowInfo &r, RowLanes<IDS> &out) {
+                                               const d4 *__restrict__ ent_terms, RowInfo &r,
+                                               RowLanes<IDS> &out) {
     static_assert(G == 32, "one warp a row");
     constexpr int FW = W::FW;
     static_assert(GENERAL || FW == 1, "a face set is one word of the common rows");
@@ -1741,10 +1736,6 @@ __device__ __forceinline__ void split_row_body(const MeshView &M, const dv3 q, W
         out.vid[0] = v;
         if (co) out.col[0] = __popc(cm & g.lt());
         out.a[0] = r.nnb > 0 ? fdiv(1.0, (double)r.nnb) : 0.0;
-        return;
-    }
-    if (FULL && !GENERAL && !M.corner) {
-        r.status = ST_GENERAL;
         return;
     }
     auto &C = ws.u.c;
@@ -1774,7 +1765,12 @@ __device__ __forceinline__ void split_row_body(const MeshView &M, const dv3 q, W
         const int4 p = M.tv[x.tet];
         if (FULL && e < 32) {
             first_o = o;
-            if (!GENERAL) terms = M.corner[16 * (size_t)x.tet + (((unsigned)x.pos >> 8) & 15u)];
+            if (!GENERAL) {
+                if (TERMS && !M.corner)
+                    terms = ent_terms[e];
+                else
+                    terms = M.corner[16 * (size_t)x.tet + (((unsigned)x.pos >> 8) & 15u)];
+            }
         }
         unsigned slots = 0;
         // most vertices get the slot of their hash or the one beside it, all four
@@ -1967,8 +1963,8 @@ __device__ __forceinline__ void split_row_body(const MeshView &M, const dv3 q, W
         if (GENERAL || e >= 32) {
             const int t = C.tet[o];
             const unsigned m = C.mask[o] >> 4;
-            if (GENERAL && !M.corner)
-                terms = corner_terms_direct(M, t, m);
+            if (TERMS && !M.corner)
+                terms = ent_terms[e];
             else
                 terms = M.corner[16 * (size_t)t + m];
         }

@@ -115,7 +115,14 @@ class DeviceMesh:
         N.check(self._lib.nif_dmesh_bytes(self.n_vertices, self.n_tets, ctypes.byref(nbytes)),
                 'nif_dmesh_bytes')
         with torch.cuda.device(self.device):
-            self._buf = torch.empty(int(nbytes.value), dtype=torch.uint8, device=self.device)
+            try:
+                self._buf = torch.empty(int(nbytes.value), dtype=torch.uint8, device=self.device)
+            except torch.cuda.OutOfMemoryError:
+                # without the corner terms (nif_dmesh_bytes)
+                if nbytes.value < 512 * self.n_tets:
+                    raise
+                nbytes.value -= 512 * self.n_tets
+                self._buf = torch.empty(int(nbytes.value), dtype=torch.uint8, device=self.device)
             if on_device:
                 d_v = vxyz.to(self.device, torch.float64).contiguous()
                 d_tv = tet_v.to(self.device, torch.int32).contiguous()
