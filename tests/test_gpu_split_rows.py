@@ -79,3 +79,19 @@ def test_interpolation_equals_weights_times_values(cuda_device, kind, D):
     W32 = W32.astype(np.float32)
     W32.sort_indices()
     assert np.array_equal(it.interpolate(q32, v32), W32 @ v32)
+
+
+@pytest.mark.parametrize('M', [1, 63, 4096, 16384, 16385, 16400])
+def test_row_order_does_not_matter(cuda_device, M):
+    """Calls of up to 16,384 rows run as they come, larger ones by bucket: the
+    same rows have the same bits in one call and in two."""
+    rng = np.random.default_rng(72)
+    it = ni.Interpolator(rng.uniform(0, 1, (3000, 3)), constructor='gpu')
+    q = rng.uniform(-0.02, 1.02, (M, 3))
+    v = rng.standard_normal((3000, 2))
+    whole = it.interpolate(q, v)
+    cut = M // 3
+    parts = [it.interpolate(p, v) for p in (q[:cut], q[cut:]) if len(p)]
+    assert np.array_equal(whole.view(np.uint8), np.concatenate(parts).view(np.uint8))
+    W = it.get_weights(q)
+    assert np.array_equal(W @ v, whole)
