@@ -39,14 +39,14 @@ WORKLOAD = ('plain interpolate at scale: {keys:,} keys U[0,1]^3 float64, {querie
 
 # DRAM bytes (read + write) per row of one launch, from the ncu captures in
 # profiles/ (TRAFFIC_SOURCE)
-TRAFFIC_PER_ROW = {'k_rows_volume': (796.55e6 + 52.46e6) / 1_000_000}
+TRAFFIC_PER_ROW = {'k_rows_volume': (1045.9e6 + 46.7e6) / 1_000_000}
 TRAFFIC_SOURCE = ('one 1,000,000-row k_rows_volume launch of the 1M-key / 10M-query workload '
                   '(dram__bytes_read.sum + dram__bytes_write.sum, 1 pass; '
                   'profiles/k_rows_volume_200k_keys_2M_queries.md)')
 
 # FP64 operations per unit of work, counted as natinterp3d's C evaluates them
 # (each add, subtract, multiply and divide is one flop; no fused multiply-add)
-FLOPS = {'orient': 23, 'insphere': 77, 'tet_cc': 79, 'tri_cc': 56, 'subcell': 89}
+FLOPS = {'orient': 23, 'sphere': 9, 'tet_cc': 79, 'tri_cc': 56, 'subcell_from': 63}
 
 
 def parse():
@@ -165,20 +165,20 @@ class ClockSampler:
 def flops_per_query(stats, gpu_walk_steps, n):
     """Algorithmic FP64 flops per query of the row path, by kernel.
 
-    The kernels read tet and face circumcentres from the per-mesh cache, so
-    per query they evaluate: 4 orientation tests per walk step (k_locate),
-    the insphere tests (k_rows_cavity), and in k_rows_volume one virtual-tet
-    circumcentre per boundary face, two fresh triangle circumcentres and one
-    subcell volume per new term, one subcell volume per old term, one
+    The kernels read tet circumspheres, face circumcentres and the cavity
+    tets' corner terms from the mesh, so per query they evaluate: 4
+    orientation tests per walk step (k_locate), a sphere test per tested tet
+    (k_rows_cavity), and in k_rows_volume one virtual-tet circumcentre per
+    boundary face, one fresh triangle circumcentre and one subcell volume per
+    new term (an edge's other direction is the neighbouring face's), one
     addition per term, and the normalisation.  Returns {'locate', 'cavity',
     'volume', 'total'} per query."""
     q = stats['queries']
     terms = stats['old_terms'] + stats['new_terms']
     locate = 4 * FLOPS['orient'] * gpu_walk_steps / n * q
-    cavity = FLOPS['insphere'] * stats['insphere']
+    cavity = FLOPS['sphere'] * stats['insphere']
     volume = (FLOPS['tet_cc'] * stats['boundary']
-              + 2 * FLOPS['tri_cc'] * stats['new_terms']
-              + FLOPS['subcell'] * terms
+              + (FLOPS['tri_cc'] + FLOPS['subcell_from']) * stats['new_terms']
               + terms + 3 * stats['neighbours'] + 4 * q)
     out = {'locate': locate / q, 'cavity': cavity / q, 'volume': volume / q}
     out['total'] = sum(out.values())
@@ -191,7 +191,7 @@ def plain_config(args, world):
                                         seed=args.seed),
             'keys': args.keys, 'queries_per_gpu': args.queries, 'D': args.dim,
             'parallelism': 'replicated mesh, queries sharded' if world > 1 else 'single GPU',
-            'l2': 'inputs larger than L2 (10M queries = 240 MB; the resident mesh about 1.6 GB)'}
+            'l2': 'inputs larger than L2 (10M queries = 240 MB; the resident mesh about 5.3 GB)'}
 
 
 def run_reference(args, rank, world):
@@ -759,7 +759,8 @@ def main():
         fused, separate = ctypes.c_double(), ctypes.c_double()
         lib.nif_measure_fp64_peak(ctypes.byref(fused), ctypes.byref(separate))
         # the dominant kernel, k_rows_volume: its launches take every row but
-        # the few the fused kernel takes (cavities wider than a record)
+        # the few the fused kernel takes (cavities wider than a record) and the
+        # two in a hundred of k_rows_general
         vol_rows = M - int(summ['rows_wide'])
         vol_ms, vol_launches = kms[2], kn[2]
         achieved = (fpq['volume'] * vol_rows / (vol_ms * 1e-3) / 1e12) if vol_ms > 0 else None
@@ -771,8 +772,9 @@ def main():
         for i, part in enumerate(['locate', 'cavity', 'volume']):
             kernels[names[i]]['flops_per_query'] = fpq[part]
         # bucketing (k_bucket, three scan kernels, k_scatter), the row kernels
-        # the profiler bracketed, and the large-row kernel
-        launches_per_step = int(round(5 + sum(kn) + 1))
+        # the profiler bracketed, two k_rows_general a volume launch, and the
+        # large-row kernel
+        launches_per_step = int(round(5 + sum(kn) + 2 * kn[2] + 1))
         cpu = None if args.no_cpu_baseline else cpu_baseline(interp, queries, values)
         line = {
             'metric': METRIC, 'value': value, 'unit': 'queries/s', 'n_gpus': world,

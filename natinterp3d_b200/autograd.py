@@ -6,8 +6,8 @@ and back-propagates into both arguments:
 * d/dvalues = W^T @ grad_out, a deterministic transpose product (CSC built by
   a stable sort on the GPU, no floating-point atomics);
 * d/dqueries from the analytic derivative of the Sibson coordinates with
-  respect to the query position (the GPU kernel differentiates the
-  virtual-tet volumes, the only terms that move with the query).  The
+  respect to the query position (each neighbour's volume changes with the
+  query by the motion of the facet between their cells).  The
   forward keeps every row's cavity record (788 bytes a row) so that the
   backward starts from it; beyond RECORDS_MAX_BYTES of records, or on meshes
   with other than the default fast predicates, the backward locates and

@@ -77,8 +77,8 @@ constexpr int REC_CHUNK = NIF_REC_CHUNK;
 // The cavity kernel takes 8 (64 registers; 10 blocks spill: 2.57 ms a 2M-row call
 // for 2.25).  The volume kernel takes 6 or, for the
 // setting of 8, 7: with 72 registers a thread it barely spills, and a warp's
-// workspace holds 42 boundary faces (2M queries, 200k keys: 7.1 ms at 7
-// blocks, 7.4 ms at 6, 10.1 ms at 8 with 64 registers and 34 faces).
+// workspace holds 42 boundary faces (2M queries, 200k keys, when 7 blocks took
+// 7.1 ms, now 6.1: 7.4 ms at 6, 10.1 ms at 8 with 64 registers and 34 faces).
 #ifndef NIF_CAV_OCC
 #define NIF_CAV_OCC 8
 #endif
@@ -201,7 +201,7 @@ __global__ void k_prep_geometry(MeshView M, uint32_t *__restrict__ tinfo, d4 *__
 }
 
 // every corner term of every tet, one thread a (tet, mask): 32 bytes each,
-// 512 a tet in one piece
+// 512 a tet in one piece (bound by those stores: 3.5 GB at 1M keys)
 __global__ void k_prep_corner(MeshView M, d4 *__restrict__ corner) {
     const int64_t n = 16 * (int64_t)M.nt;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
@@ -845,7 +845,7 @@ struct GradSink {
     // to the next vertex and the other face of that edge, is one triangle of
     // u's facet: about 40 operations instead of the 3,000 of the dual numbers,
     // so that the pass is bound by the same row setup as the weights (1M rows,
-    // 200k keys, 16 columns: 10.1 ms with dual numbers, 2.6 ms).
+    // 200k keys, 16 columns: 10.1 ms with dual numbers, 2.4 ms).
     // Returns false where that does not hold: faces that do not close or that
     // differ in orientation, or tets and triangles near natinterp3d's
     // degeneracy thresholds; k_rows_general takes those rows, with the dual

@@ -459,8 +459,9 @@ __device__ int grid_nearest(const MeshView &M, const dv3 q) {
 // error bound, because prep_sphere gives only those tets a radius for which
 //   6V |d2 - w| > 2 E  for |d2 - w| > SPHERE_REL w and d2 < SPHERE_FAR w,
 // d2 = |q - c|^2, E the static error bound of inspherefast; the others have
-// w = NaN, which decides nothing.  Ten FP64 operations on one 32-byte record
-// for some 80 on four vertices behind the tet's vertex record.
+// w = NaN, which decides nothing.  Nine FP64 operations on one 32-byte record
+// for some 80 on four vertices behind the tet's vertex record (the cavity pass
+// of 2M rows on 200k keys: 4.55 to 3.3 ms).
 constexpr double SPHERE_REL = 1e-6, SPHERE_FAR = 1e4;
 __device__ __forceinline__ int sphere_side(const d4 &c, const dv3 &q) {
     const double x = q.x - c.x, y = q.y - c.y, z = q.z - c.z;
@@ -1658,9 +1659,12 @@ __device__ __forceinline__ void sstore(double (&p)[3], const dv3 &v) {
 // sibson_row returns it (steps 3-5, or the coincident-vertex row).  With
 // FULL = false it stops at the neighbours and the boundary faces.
 //
-// Bound by instruction issue, and by instruction fetch where the code
-// outgrows the instruction cache: loops are not unrolled, and what a row
-// shares is computed once.
+// Bound by the shared-memory pipe (81 % of its wavefronts) and instruction issue
+// (70 %, 2,580 warp instructions a row), and by instruction fetch where the code
+// outgrows the instruction cache: loops are not unrolled (unrolled 12.2 ms a
+// 2M-row call on 200k keys, rolled 8.4), and what a row shares is computed once.
+// With what follows such a call's rows take 6.1 ms; 11.7 ms with a tet's terms
+// evaluated per row, both of an edge's circumcentres per face and a lane a face.
 //  - vertices get their id once per cavity tet (one hash pass over the tets'
 //    vertices), and their positions are staged by id;
 //  - cavity terms come from the mesh's corner table;

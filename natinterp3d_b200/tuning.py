@@ -5,7 +5,8 @@ and :func:`tune` checks that on its sample before keeping a winner.  For one
 mesh (``Interpolator``) the candidates are
 
   blocks_per_sm  6 or 8      resident 4-warp blocks per SM of the
-                             one-warp-per-query row kernel (80 or 64
+                             one-warp-per-query row kernels (the volume
+                             kernel takes 7 for the setting of 8: 80 or 72
                              registers a thread)
   tile           0, 8, 32    static grid stride, or tiles of 8 / 32
                              consecutive bucket-ordered queries a warp pulls
@@ -17,10 +18,11 @@ and for a batch (``BatchInterpolator``) blocks_per_sm 6 or 8 times tiles of
 16, 32, 64 or 128 queries.  Each candidate runs once untimed, then ``reps``
 times between CUDA events on the current stream; the smallest time wins.
 
-Lanes per query stay at one warp.  Groups of 16 or 8 lanes (two or four
-queries per warp) diverge between their queries' control flow and ran
-0.62x and 0.32x as fast as one warp per query on the 1M-key / 10M-query
-interpolation workload, so they are not candidates.  The shared-memory
+Lanes per query are fixed by kernel: 16 for the cavity search, one for the
+visiting order, one warp for the volumes.  Groups of 16 or 8 lanes for a
+whole row (two or four queries per warp) diverge between their queries'
+control flow and ran 0.62x and 0.32x as fast as one warp per query on the
+1M-key / 10M-query interpolation workload, so they are not candidates.  The shared-memory
 capacities of the fast kernel (tested-tet hash 256, cavity 96, boundary
 faces 128, neighbours 64) are fixed: at 8 blocks per SM registers, not
 shared memory, limit residency, and rows beyond them go to the large-row
