@@ -5,6 +5,8 @@ library's own sm_100a kernels.  All tensors passed to the library are
 contiguous CUDA tensors on the mesh's device.
 """
 import ctypes
+import threading
+import weakref
 
 import numpy as np
 import torch
@@ -13,6 +15,38 @@ from . import _native as N
 
 _DT = {torch.float64: N.NIF_F64, torch.float32: N.NIF_F32}
 _NP_DT = {np.dtype(np.float64): N.NIF_F64, np.dtype(np.float32): N.NIF_F32}
+
+
+# The corner terms of a mesh (nif_dmesh_bytes) save a query about a quarter of its
+# time and take 512 bytes a tet, nearly twice the rest of the mesh.  What a program
+# allocates after its meshes is to fit as it does without them: the tables of a
+# process take at most a quarter of the memory that is free or theirs on a device, so
+# that three quarters stay for the rest, and leave 4 GB of it (the workspaces and
+# results of two pipelined chunks).
+CORNER_BYTES = 512
+_TABLE_SHARE = 4
+_TABLE_LEAVES = 4 << 30
+_tables_mu = threading.Lock()
+_tables = weakref.WeakSet()  # meshes that hold a table
+
+
+def _table_fits(table, room, held):
+    """Whether a table of `table` bytes may be taken where `room` bytes are free
+    besides the rest of its mesh and `held` bytes are other meshes' tables."""
+    return table <= room - _TABLE_LEAVES and (held + table) * _TABLE_SHARE <= room + held
+
+
+def _room(device):
+    """Bytes that can still be allocated on `device`."""
+    free, total = torch.cuda.mem_get_info(device)
+    try:
+        stats = torch.cuda.memory_stats_as_nested_dict(device)
+        used = stats['allocated_bytes']['all']['current']
+        cached = stats['reserved_bytes']['all']['current'] - used
+        limit = int(total * torch.cuda.get_per_process_memory_fraction(device))
+    except (RuntimeError, KeyError):  # an allocator that keeps no such counts
+        return free
+    return min(free + cached, limit - used)
 
 
 def _stream_ptr(device):
@@ -114,27 +148,32 @@ class DeviceMesh:
         nbytes = ctypes.c_size_t()
         N.check(self._lib.nif_dmesh_bytes(self.n_vertices, self.n_tets, ctypes.byref(nbytes)),
                 'nif_dmesh_bytes')
+        full = int(nbytes.value)
+        # (the largest meshes have no table in it)
+        lean = full - CORNER_BYTES * self.n_tets if full > CORNER_BYTES * self.n_tets else full
         with torch.cuda.device(self.device):
-            try:
-                self._buf = torch.empty(int(nbytes.value), dtype=torch.uint8, device=self.device)
-            except torch.cuda.OutOfMemoryError:
-                # without the corner terms (nif_dmesh_bytes)
-                if nbytes.value < 512 * self.n_tets:
-                    raise
-                nbytes.value -= 512 * self.n_tets
-                self._buf = torch.empty(int(nbytes.value), dtype=torch.uint8, device=self.device)
-            if on_device:
-                d_v = vxyz.to(self.device, torch.float64).contiguous()
-                d_tv = tet_v.to(self.device, torch.int32).contiguous()
-                d_tn = tet_n.to(self.device, torch.int32).contiguous()
-            else:
-                d_v = torch.from_numpy(vxyz).to(self.device)
-                d_tv = torch.from_numpy(tet_v).to(self.device)
-                d_tn = torch.from_numpy(tet_n).to(self.device)
+            table = full > lean
+            while True:
+                try:
+                    table = self._allocate(full, lean, table)
+                    if on_device:
+                        d_v = vxyz.to(self.device, torch.float64).contiguous()
+                        d_tv = tet_v.to(self.device, torch.int32).contiguous()
+                        d_tn = tet_n.to(self.device, torch.int32).contiguous()
+                    else:
+                        d_v = torch.from_numpy(vxyz).to(self.device)
+                        d_tv = torch.from_numpy(tet_v).to(self.device)
+                        d_tn = torch.from_numpy(tet_n).to(self.device)
+                    break
+                except torch.cuda.OutOfMemoryError:
+                    if not table:
+                        raise
+                    table = False  # again, without it
+                    self._buf = d_v = d_tv = d_tn = None
             self._vertices = d_v   # keys' coordinates (the transpose product's key order)
             self._h = ctypes.c_void_p()
             N.check(self._lib.nif_dmesh_create(_vp(d_v), _vp(d_tv), _vp(d_tn), self.n_vertices,
-                                               self.n_tets, _vp(self._buf), nbytes.value,
+                                               self.n_tets, _vp(self._buf), self._buf.numel(),
                                                _stream_ptr(self.device), ctypes.byref(self._h)),
                     'nif_dmesh_create')
         info = (ctypes.c_int64 * 8)()
@@ -146,6 +185,19 @@ class DeviceMesh:
         self.orientation_stats = {'uncertain': int(info[5]), 'flipped': int(info[6])}
         self.predicates = 'fast'
         self.last_summary = None
+
+    def _allocate(self, full, lean, table):
+        """The resident buffer, with the table of corner terms if `table` and
+        there is room for it; returns whether it has the table."""
+        with _tables_mu:  # a table is decided on by what is free
+            if table:
+                held = sum(m.table_bytes for m in _tables if m.device == self.device)
+                uploads = 24 * self.n_vertices + 32 * self.n_tets
+                table = _table_fits(full - lean, _room(self.device) - lean - uploads, held)
+            self.table_bytes = full - lean if table else 0
+            (_tables.add if table else _tables.discard)(self)
+            self._buf = torch.empty(full if table else lean, dtype=torch.uint8, device=self.device)
+        return table
 
     def set_predicates(self, mode):
         """'fast' (natinterp3d's signs, the default), 'audit' (the same
