@@ -184,7 +184,8 @@ int nif_dmesh_set_predicates(nif_dmesh *m, int mode);
  *                  8 (64 registers, more spills, more warps hiding latency;
  *                  the volume kernel then takes 7 with 72 registers)
  *   bucket_shift   Morton bucket resolution of the query ordering, in bits per
- *                  axis relative to the size-based default: -2 .. 1
+ *                  axis relative to the size-based default: -2 .. 1 (no effect
+ *                  on calls of up to 16,384 rows, which are taken as they come)
  *   tile           queries a warp takes per work item: 0 = a static grid
  *                  stride (one query per step), 1 .. 1024 = tiles of
  *                  consecutive bucket-ordered queries pulled from a device

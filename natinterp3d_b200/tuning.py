@@ -13,6 +13,8 @@ mesh (``Interpolator``) the candidates are
                              from a device counter
   bucket_shift   -1, 0, 1    Morton bucket resolution of the query order,
                              in bits per axis relative to the size default
+                             (0 alone for calls of up to 16,384 queries,
+                             which are taken as they come)
 
 and for a batch (``BatchInterpolator``) blocks_per_sm 6 or 8 times tiles of
 16, 32, 64 or 128 queries.  Each candidate runs once untimed, then ``reps``
@@ -31,7 +33,7 @@ kernel whatever their size.
 Results are cached per (GPU name, mode, key count, query count, dtypes,
 value columns, predicate mode) in a JSON file (``NATINTERP3D_B200_TUNING``,
 default ``~/.cache/natinterp3d_b200/tuning.json``); counts are rounded to
-powers of two.
+powers of two, query counts on one side of 16,384 kept apart from the other.
 """
 import itertools
 import json
@@ -47,6 +49,9 @@ MESH_CANDIDATES = [{'blocks_per_sm': b, 'tile': t, 'bucket_shift': s}
                    for b, t, s in itertools.product((8, 6), (8, 0, 32), (0, -1, 1))]
 BATCH_CANDIDATES = [{'blocks_per_sm': b, 'tile': t, 'bucket_shift': 0}
                     for b, t in itertools.product((8, 6), (64, 16, 32, 128))]
+
+# calls of at most this many rows of one mesh are not bucketed (nif_tuning.bucket_shift)
+IDENTITY_ROWS = 16384
 
 
 def cache_path():
@@ -79,6 +84,21 @@ def _store_cache(key, entry):
 
 def _p2(n):
     return 0 if n <= 0 else int(round(math.log2(n)))
+
+
+def _query_class(M):
+    """Query count of a cache key.  Around IDENTITY_ROWS the rounding alone would
+    put calls that the bucket resolution matters to with calls that it does not."""
+    p = _p2(M)
+    return 'q2^%d' % p if p != _p2(IDENTITY_ROWS) else 'q%s%d' % ('<=' if M <= IDENTITY_ROWS else '>',
+                                                                  IDENTITY_ROWS)
+
+
+def _mesh_candidates(M):
+    """The candidates that differ on a sample of M queries."""
+    if M > IDENTITY_ROWS:
+        return MESH_CANDIDATES
+    return [c for c in MESH_CANDIDATES if c['bucket_shift'] == 0]
 
 
 def _time(fn, reps):
@@ -156,15 +176,15 @@ def tune(interp, query_points, values=None, mode='interpolate', max_queries=2_00
         run = lambda: interp.get_weights_device(q)  # noqa: E731
         vdesc = '-'
     key = '|'.join([torch.cuda.get_device_name(dm.device), mode, 'k2^%d' % _p2(interp.n_keys),
-                    'q2^%d' % _p2(M_full), str(q.dtype).replace('torch.', ''), vdesc,
+                    _query_class(M_full), str(q.dtype).replace('torch.', ''), vdesc,
                     interp.predicates])
     if use_cache and candidates is None:
         hit = _load_cache().get(key)
-        if hit is not None:
+        if hit is not None and (M_full > IDENTITY_ROWS or hit['tuning'].get('bucket_shift', 0) == 0):
             interp.set_tuning(hit['tuning'])
             return {'tuning': hit['tuning'], 'times_ms': hit.get('times_ms', []), 'cached': True}
     with torch.cuda.device(dm.device):
-        best, report = _search(candidates or MESH_CANDIDATES, interp.set_tuning, run, reps)
+        best, report = _search(candidates or _mesh_candidates(int(q.shape[0])), interp.set_tuning, run, reps)
     entry = {'tuning': best, 'times_ms': [(c, round(t, 3)) for c, t in report],
              'sample_queries': int(q.shape[0])}
     if use_cache and candidates is None:
