@@ -14,7 +14,9 @@
     CUDA runtime.
 
 Both are built in-tree so that a prebuilt copy travels with the source tree;
-where the natinterp3d sources are absent the prebuilt constructor is used.
+where the natinterp3d sources are absent the prebuilt constructor is used.  With
+neither, the CUDA library is built alone: meshes then come from the GPU
+constructor or from saved files, and the host constructor raises.
 """
 import os
 import subprocess
@@ -81,6 +83,11 @@ def _stale(target, sources):
     return any(os.path.getmtime(s) > t for s in sources if os.path.exists(s))
 
 
+def have_mesh_lib():
+    """Whether natinterp3d's constructor is built here or can be."""
+    return os.path.exists(MESH_SO) or _has_sources(ref_source_dir())
+
+
 def build_mesh_lib(force=False):
     ref_src = ref_source_dir()
     src = os.path.join(CSRC, 'mesh_export.c')
@@ -116,11 +123,18 @@ def build_cuda_lib(force=False, extra_flags=()):
 
 
 def build(force=False):
-    build_mesh_lib(force)
+    """Both libraries; returns whether the constructor is among them (the CUDA
+    library does not need natinterp3d's sources)."""
     build_cuda_lib(force)
+    if not have_mesh_lib():
+        print('natinterp3d constructor sources not found at %r: %s not built'
+              % (ref_source_dir(), MESH_SO), file=sys.stderr)
+        return False
+    build_mesh_lib(force)
+    return True
 
 
 if __name__ == '__main__':
-    build(force='--force' in sys.argv)
-    print(MESH_SO)
+    if build(force='--force' in sys.argv):
+        print(MESH_SO)
     print(CUDA_SO)
