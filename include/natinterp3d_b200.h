@@ -135,7 +135,7 @@ typedef struct nif_dmesh nif_dmesh;
  * natural_insertionfree.c:397-450.)  Meshes of up to 2^26 tets also hold the
  * terms of their tets' corners in every stolen volume, 512 bytes a tet: a
  * buffer of 512 * n_tets bytes less is accepted too, its queries compute them
- * (about 1.3 times as long). */
+ * (about 1.3 times as long, in a workspace of about the same size). */
 int nif_dmesh_bytes(int n_vertices, int n_tets, size_t *bytes);
 
 /* Uploads a mesh: derives the resident arrays in d_buf from the packed

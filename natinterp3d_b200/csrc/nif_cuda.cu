@@ -73,6 +73,17 @@ constexpr int GEN_OCC = 3;
 #define NIF_REC_CHUNK (1 << 20)
 #endif
 constexpr int REC_CHUNK = NIF_REC_CHUNK;
+// Rows of a call's chunks.  Where the corner terms of a chunk stand beside its
+// records (meshes without the corner table), a row takes 1,536 bytes more than its
+// 784: chunks of a third of the rows then need no more memory than a mesh with the
+// table does.  Calls of fewer than three times TERMS_CHUNK_MIN rows (100 MB of
+// terms) are cut less, for their launches.
+constexpr int TERMS_CHUNK_MIN = 1 << 16;
+inline int64_t record_chunk(int64_t M, bool terms) {
+    const int64_t rows = M < REC_CHUNK ? (M > 0 ? M : 1) : REC_CHUNK;
+    const int64_t cuts = terms ? min((int64_t)3, (rows + TERMS_CHUNK_MIN - 1) / TERMS_CHUNK_MIN) : 1;
+    return (rows + cuts - 1) / cuts;
+}
 // resident blocks per SM of the split kernels (0: the mesh's blocks_per_sm).
 // The cavity kernel takes 8 (64 registers; 10 blocks spill: 2.57 ms a 2M-row call
 // for 2.25).  The volume kernel takes 6 or, for the
@@ -2161,7 +2172,7 @@ QueryLayout carve_query(Carve &c, const nif_dmesh *m, int64_t M, int mode) {
     L.exact = c.take<double>((size_t)LARGE_GROUPS * NIF_EXACT_SCRATCH);
     L.located = c.take<int>(M > 0 ? M : 1);
     {
-        const int64_t ch = M < REC_CHUNK ? (M > 0 ? M : 1) : REC_CHUNK;
+        const int64_t ch = record_chunk(M, !m->view.corner);
         L.heads = c.take<RowHead>(ch);
         L.ents = c.take<RowEntry>(ch * REC_CAV);
         L.wide = c.take<int>(M > 0 ? M : 1);
@@ -2463,7 +2474,7 @@ void launch_general(const Launch &lc, const Rows &rows, const QT *Q, int64_t n, 
 }
 
 // The split row over positions [0, M) of R.order, whose rows `rows` maps to
-// their meshes: k_locate over all rows, then per chunk of REC_CHUNK rows the
+// their meshes: k_locate over all rows, then per chunk (record_chunk) of rows the
 // cavity records and the volumes.  Rows whose cavity exceeds a record are
 // left in `wide` (count in R.sum->wide_count) for the fused kernel, which
 // launch_wide launches once all cavities are known: the last chunk's volumes run
@@ -2477,13 +2488,13 @@ void launch_split(const Launch &lc, const Rows &rows, const QT *Q, int64_t M, co
     constexpr int COCC = NIF_CAV_OCC > 0 ? NIF_CAV_OCC : OCC;
     constexpr int VOCC = sink_occ<Sink, (NIF_VOL_OCC > 0 ? NIF_VOL_OCC : (OCC == OCC_HI ? 7 : OCC))>();
     int *located = const_cast<int *>(R.located);
-    const int64_t gen_room = min(M, (int64_t)REC_CHUNK);
+    const int64_t chunk = record_chunk(M, terms != nullptr);
     prof_span(SPAN_LOCATE, false, st);
     launch_rows(k_locate<QT, Rows, PM>, lc, M, 0, &R.sum->work[WORK_LOCATE], false, st, rows, Q, R.order, M, located,
                 R.sum);
     prof_span(SPAN_LOCATE, true, st);
-    for (int64_t c0 = 0; c0 < M; c0 += REC_CHUNK) {
-        const int64_t n = min((int64_t)REC_CHUNK, M - c0);
+    for (int64_t c0 = 0; c0 < M; c0 += chunk) {
+        const int64_t n = min(chunk, M - c0);
         const int *order = R.order + c0;
         // one chunk's records, or (keep) every row's at its own position
         RowHead *h = keep ? heads + c0 : heads;
@@ -2514,9 +2525,9 @@ void launch_split(const Launch &lc, const Rows &rows, const QT *Q, int64_t M, co
             prof_span(SPAN_VOLUME, false, st);
             launch_rows(k_rows_volume<QT, Rows, Sink, VOCC, TERMS>, lc, n, GPB * sizeof(VolWS),
                         &R.sum->work[WORK_VOLUME], true, st, rows, Q, order, n, (const RowHead *)h,
-                        (const RowEntry *)e, (const d4 *)terms, gen + gen_room, false, sink, LargeQueue{R.large},
+                        (const RowEntry *)e, (const d4 *)terms, gen + chunk, false, sink, LargeQueue{R.large},
                         R.sum);
-            launch_general<TERMS>(lc, rows, Q, n, order, h, e, terms, gen + gen_room, true, sink, R.large, R.sum,
+            launch_general<TERMS>(lc, rows, Q, n, order, h, e, terms, gen + chunk, true, sink, R.large, R.sum,
                                   st);
         };
         if constexpr (Sink::FULL) {
@@ -3516,9 +3527,10 @@ void grad_records_typed(const nif_dmesh *m, const void *q, int64_t M, const Cent
     const Launch lc{m->tune.tile, m->num_sms};
     const OneMesh rows{m->view, cen};
     cudaMemsetAsync(R.sum, 0, sizeof(DevSummary), st);
-    int *gen_end = L.gen + min(M, (int64_t)REC_CHUNK);
-    for (int64_t c0 = 0; c0 < M; c0 += REC_CHUNK) {
-        const int64_t n = min((int64_t)REC_CHUNK, M - c0);
+    const int64_t chunk = record_chunk(M, L.terms != nullptr);
+    int *gen_end = L.gen + chunk;
+    for (int64_t c0 = 0; c0 < M; c0 += chunk) {
+        const int64_t n = min(chunk, M - c0);
         const bool last = c0 + n == M;
         const int *order = row_order(m, L, M) + c0;
         if (last) {
@@ -3853,7 +3865,7 @@ BatchLayout carve_batch(Carve &c, int P, int64_t M, bool terms) {
     L.large_ws = c.take<LargeWS>(LARGE_GROUPS);
     L.exact = c.take<double>((size_t)LARGE_GROUPS * NIF_EXACT_SCRATCH);
     const int64_t m1 = M > 0 ? M : 1;
-    const int64_t ch = m1 < REC_CHUNK ? m1 : REC_CHUNK;
+    const int64_t ch = record_chunk(M, terms);
     L.located = c.take<int>(m1);
     L.wide = c.take<int>(m1);
     L.heads = c.take<RowHead>(ch);
