@@ -211,16 +211,38 @@ __global__ void k_prep_geometry(MeshView M, uint32_t *__restrict__ tinfo, d4 *__
     }
 }
 
-// every corner term of every tet, one thread a (tet, mask): 32 bytes each,
-// 512 a tet in one piece (bound by those stores: 3.5 GB at 1M keys)
-__global__ void k_prep_corner(MeshView M, d4 *__restrict__ corner) {
-    const int64_t n = 16 * (int64_t)M.nt;
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
-         i += (int64_t)gridDim.x * blockDim.x) {
-        const int t = (int)(i >> 4);
-        const unsigned m = (unsigned)i & 15u;
-        corner[i] = d4{corner_term(M, t, m, 0), corner_term(M, t, m, 1), corner_term(M, t, m, 2),
-                       corner_term(M, t, m, 3)};
+// Every corner term of every tet, one thread a corner: its eight choices, each the
+// same whether the face opposite it is a copy or not, so 16 entries.  A warp's eight
+// tets are put together in shared memory and written in one piece, 512 bytes a tet.
+// 200k keys, 1.35M tets: 316 us, with each of a tet's 64 entries evaluated by itself
+// 840; 106 are its stores.
+constexpr int CORNER_THREADS = 128;
+constexpr int CORNER_PAD = 64 + 2;  // doubles of a tet in shared memory (banks)
+__global__ void __launch_bounds__(CORNER_THREADS) k_prep_corner(MeshView M, d4 *__restrict__ corner) {
+    __shared__ __align__(16) double put[CORNER_THREADS / 32][8 * CORNER_PAD];
+    double *const s = put[threadIdx.x >> 5];
+    const int lane = threadIdx.x & 31, vi = lane & 3;
+    const int64_t warps = (int64_t)gridDim.x * (CORNER_THREADS / 32);
+    for (int64_t w = (int64_t)blockIdx.x * (CORNER_THREADS / 32) + (threadIdx.x >> 5); 8 * w < M.nt; w += warps) {
+        const int64_t t0 = 8 * w;
+        const int n = (int)min((int64_t)8, M.nt - t0);  // tets of this warp
+        if (lane >> 2 < n) {
+            double v[8];
+            corner_terms(M, (int)t0 + (lane >> 2), vi, v);
+#pragma unroll
+            for (int k = 0; k < 8; k++) {
+                const int below = k & ((1 << vi) - 1);
+                const int mask = below | (k - below) << 1;  // bit vi clear
+                double *const at = s + (lane >> 2) * CORNER_PAD + vi;
+                at[4 * mask] = v[k];
+                at[4 * (mask | 1 << vi)] = v[k];
+            }
+        }
+        __syncwarp();
+        double2 *const out = reinterpret_cast<double2 *>(corner + 16 * t0);
+        for (int k = 0; k < n; k++)
+            out[32 * k + lane] = reinterpret_cast<const double2 *>(s + k * CORNER_PAD)[lane];
+        __syncwarp();
     }
 }
 
@@ -2893,7 +2915,7 @@ NIF_EXPORT int nif_dmesh_create(const double *d_vxyz, const int32_t *d_tet_v,
         }
         k_prep_geometry<<<blocks_for(n_tets, 128), 128, 0, st>>>(V, L.tinfo, L.tcc, L.fcc, L.flag);
         if (L.corner)
-            k_prep_corner<<<blocks_for(16 * (int64_t)n_tets, 128), 128, 0, st>>>(V, L.corner);
+            k_prep_corner<<<blocks_for(4 * (int64_t)n_tets, CORNER_THREADS), CORNER_THREADS, 0, st>>>(V, L.corner);
         int flag[4];
         if (cudaMemcpyAsync(flag, L.flag, sizeof(flag), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
             cudaStreamSynchronize(st) != cudaSuccess) {

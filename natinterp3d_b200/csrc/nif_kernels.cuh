@@ -1641,6 +1641,57 @@ __device__ __forceinline__ double corner_term(const MeshView &M, int t, unsigned
                           vload(M, comp(p, o2)), cload(&M.tcc[t]), face(o2), face(o1), face(o0));
 }
 
+// The same for all eight choices of copies of the three faces through p[vi] (bit
+// 0, 1, 2 of the index: the lowest, middle and highest of them takes the
+// neighbour's).  A face's copy enters one of the term's three cross products, so
+// that the eight share six of them; each is summed in corner_term's order.
+__device__ __forceinline__ void corner_terms(const MeshView &M, int t, int vi, double (&out)[8]) {
+    const int4 p = M.tv[t];
+    const int4 n = M.tn[t];
+    const uint32_t info = M.tinfo[t];
+    const int o0 = vi == 0 ? 1 : 0, o1 = vi <= 1 ? 2 : 1, o2 = vi <= 2 ? 3 : 2;
+    const dv3 pk = vload(M, comp(p, vi));
+    const dv3 pa = vload(M, comp(p, o0)), pb = vload(M, comp(p, o1)), pc = vload(M, comp(p, o2));
+    const dv3 dt = vsub(cload(&M.tcc[t]), pk);
+    const bool swap = vdot(vsub(pa, pk), vcross(vsub(pb, pk), vsub(pc, pk))) < 0;
+    auto copy = [&](int i, int taken) {
+        const int j = 3 - i;
+        const int nb = comp(n, j);
+        const int k = taken && nb >= 0 ? 4 * nb + (3 - (int)((info >> (8 + 2 * j)) & 3u)) : 4 * t + i;
+        return vsub(cload(&M.fcc[k]), pk);
+    };
+    auto products = [](dv3 e, dv3 c) { return dv3{fmul(e.x, c.x), fmul(e.y, c.y), fmul(e.z, c.z)}; };
+    const dv3 e1 = vsub(pa, pb), e2 = vsub(pa, pc), e3 = vsub(pb, pc);
+    double first[2];   // of the face opposite o2
+    dv3 next[2], last[2];
+#pragma unroll
+    for (int c = 0; c < 2; c++) {
+        const dv3 m1 = products(e1, vcross(copy(o2, c), dt));
+        const dv3 m2 = products(e2, vcross(dt, copy(o1, c)));
+        const dv3 m3 = products(e3, vcross(copy(o0, c), dt));
+        first[c] = fadd(fadd(m1.x, m1.y), m1.z);
+        next[c] = swap ? m3 : m2;
+        last[c] = swap ? m2 : m3;
+    }
+    double sum[2][2][2];
+#pragma unroll
+    for (int a = 0; a < 2; a++)
+#pragma unroll
+        for (int b = 0; b < 2; b++) {
+            const double ab = fadd(fadd(fadd(first[a], next[b].x), next[b].y), next[b].z);
+#pragma unroll
+            for (int c = 0; c < 2; c++) {
+                const double v = fadd(fadd(fadd(ab, last[c].x), last[c].y), last[c].z);
+                sum[a][b][c] = div12(swap ? -v : v);
+            }
+        }
+#pragma unroll
+    for (int k = 0; k < 8; k++) {
+        const int h = k >> 2, m = (k >> 1) & 1, l = k & 1;
+        out[k] = swap ? sum[h][l][m] : sum[h][m][l];
+    }
+}
+
 // the ids of a face's three vertices, one byte each, from its tet's ids
 __device__ __forceinline__ unsigned face_ids(unsigned lid, int f) {
     // byte selectors of getFaceVerticies3's slots: (0, 1, 2), (3, 1, 0), (0, 2, 3), (3, 2, 1)
