@@ -164,7 +164,8 @@ __global__ void k_prep_tets(const int32_t *__restrict__ tet_v, const int32_t *__
 }
 
 // orientation flags, mirror slots, tet and face circumcentres.  flag[0]: bad
-// mesh, flag[1]: tets whose orientation sign the filter cannot certify.
+// mesh, flag[1]: tets whose orientation sign the filter cannot certify, flag[3]:
+// some tet is flat_sized.
 __global__ void k_prep_geometry(MeshView M, uint32_t *__restrict__ tinfo, d4 *__restrict__ tcc,
                                 d4 *__restrict__ fcc, int *__restrict__ bad) {
     for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < M.nt; t += gridDim.x * blockDim.x) {
@@ -197,7 +198,9 @@ __global__ void k_prep_geometry(MeshView M, uint32_t *__restrict__ tinfo, d4 *__
         }
         tinfo[t] = info;
         const dv3 c = tet_cc(P0, P1, P2, P3);
-        tcc[t] = d4{c.x, c.y, c.z, prep_sphere(c, P0, P1, P2, P3, o, unc)};
+        const double w = prep_sphere(c, P0, P1, P2, P3, o, unc);
+        tcc[t] = d4{c.x, c.y, c.z, w};
+        if (flat_sized(w, P0, P1)) bad[3] = 1;
         // face opposite p[i], remaining vertices in ascending slot order
         // (natural_insertionfree.c:649-652)
         const dv3 f0 = tri_cc(P1, P2, P3);
@@ -1591,6 +1594,8 @@ __global__ void __launch_bounds__(FAST_BLOCK, OCC)
                 wide[atomicAdd(&sum->wide_count, 1)] = (int)i;
             else if (rc == REC_LARGE || h.start == -3)
                 lq.list[atomicAdd(&sum->large_count, 1)] = (int)i;
+            else if (M.small && h.ncav > 0 && flat_sized(M, h.start))
+                h.state = RS_FLAT;
             heads[my] = h;
         }
         __syncwarp();
@@ -1645,9 +1650,11 @@ __global__ void __launch_bounds__(32 * ORD_WARPS) k_rows_order(int64_t nrows, in
         const int64_t s0 = gi * per;
         const int64_t s = s0 + lane;
         int nc = 0;
+        bool flat = false;
         if (lane < per && s < nrows) {
             const RowHead h = heads[s];
-            if (h.state == RS_OK && h.ncav > 0 && h.ncav <= REC_CAV) nc = h.ncav;
+            flat = h.state == RS_FLAT;
+            if ((flat || h.state == RS_OK) && h.ncav > 0 && h.ncav <= REC_CAV) nc = h.ncav;
         }
         // entry offsets of the 32 rows in one flattened index space
         int incl = nc;
@@ -1713,7 +1720,7 @@ __global__ void __launch_bounds__(32 * ORD_WARPS) k_rows_order(int64_t nrows, in
                 }
                 sp = min(sp, ORD_STACK);
             }
-            if (nbf > VolWS::BF) {
+            if (flat || nbf > VolWS::BF) {
                 heads[s].state = RS_GENERAL;
                 gen[atomicAdd(&sum->general_count, 1)] = (int)s;
             }
@@ -2924,6 +2931,7 @@ NIF_EXPORT int nif_dmesh_create(const double *d_vxyz, const int32_t *d_tet_v,
         }
         if (flag[0]) { rc = NIF_ERR_INTERNAL; break; }
         h->orient_unc = flag[1];
+        V.small = flag[3];
         if (flag[1] > 0) {
             // rare: near-flat tets; resolve their exact orientation flags
             k_prep_exact_orient<<<blocks_for(n_tets, 32, 4 * 148), 32, 0, st>>>(V, L.tinfo, L.flag);

