@@ -194,6 +194,14 @@ def plain_config(args, world):
             'l2': 'inputs larger than L2 (10M queries = 240 MB; the resident mesh about 5.3 GB)'}
 
 
+def make_interpolator(keys, **kw):
+    """natinterp3d's own constructor, or, where its library is not there and cannot
+    be built, the GPU constructor (the same set of tets)."""
+    import natinterp3d_b200 as ni
+    from natinterp3d_b200 import _build
+    return ni.Interpolator(keys, constructor='host' if _build.have_mesh_lib() else 'gpu', **kw)
+
+
 def run_reference(args, rank, world):
     """natinterp3d's own CPU implementation (oracle/_ref: its C sources built with
     its own flags) with all host threads.  Each step is get_weights + scipy
@@ -384,12 +392,11 @@ def leg_get_weights_small(local_rank, steps, warmup, cpu=True):
     """get_weights at the small configuration: 10,000 keys U[0,1]^3, 100,000
     queries U[0.05,0.95]^3, seed 0 (float64)."""
     import torch
-    import natinterp3d_b200 as ni
     dev = torch.device('cuda', local_rank)
     rng = np.random.default_rng(0)
     keys = rng.uniform(0.0, 1.0, (10_000, 3))
     queries = rng.uniform(0.05, 0.95, (100_000, 3))
-    interp = ni.Interpolator(keys, device=dev, keep_host_mesh=cpu)
+    interp = make_interpolator(keys, device=dev, keep_host_mesh=cpu)
     return _weights_leg(interp, queries, steps, warmup, cpu, 100_000,
                         'get_weights: 10,000 keys U[0,1]^3, 100,000 queries U[0.05,0.95]^3, '
                         'float64, seed 0')
@@ -435,18 +442,23 @@ def leg_gpu_construction(keys, interp, host_build_s, local_rank):
         times.append(time.perf_counter() - t0)
         last = tv
     t = min(times)
-    host_tv = interp.mesh_arrays[1]
-    same = (tet_set_digest(last.cpu().numpy()) == tet_set_digest(host_tv)
-            and np.array_equal(vxyz.cpu().numpy().view(np.uint8),
-                               interp.mesh_arrays[0].view(np.uint8)))
+    same = speedup = None
+    if interp.construction['constructor'] == 'host':
+        host_tv = interp.mesh_arrays[1]
+        same = bool(tet_set_digest(last.cpu().numpy()) == tet_set_digest(host_tv)
+                    and np.array_equal(vxyz.cpu().numpy().view(np.uint8),
+                                       interp.mesh_arrays[0].view(np.uint8)))
+        speedup = host_build_s / t
+    else:
+        host_build_s = None
     return {'value': keys.shape[0] / t, 'unit': 'keys/s', 'gpu_s': t,
-            'host_constructor_s': host_build_s, 'speedup_vs_host': host_build_s / t,
+            'host_constructor_s': host_build_s, 'speedup_vs_host': speedup,
             'tets': int(info['n_tets']), 'rounds': int(info['rounds']),
             'max_cavity': int(info['max_cavity']),
             'exact_evaluations': int(info['exact_evaluations']),
             'checks': {k: int(info[k]) for k in ('bad_orientation', 'bad_adjacency',
                                                   'non_delaunay_faces', 'cospherical_faces')},
-            'same_tets_and_vertices_as_natinterp3d': bool(same),
+            'same_tets_and_vertices_as_natinterp3d': same,
             'config': {'workload': 'Delaunay tetrahedralization of the plain workload\'s keys '
                                    '(+ natinterp3d\'s super-simplex), wall clock with the result '
                                    'on the device'}}
@@ -457,7 +469,6 @@ def leg_fwdbwd(args, rank, local_rank, steps, warmup, cpu=True):
     values (200k keys U[0,1]^3, 1M queries U[0.1,0.9]^3 float64 with grad,
     values D=16 float32 with grad, seed 3)."""
     import torch
-    import natinterp3d_b200 as ni
     from natinterp3d_b200 import autograd as nag
     keys_n, q_n, dim = 200_000, 1_000_000, 16
     torch.cuda.set_device(local_rank)
@@ -465,7 +476,7 @@ def leg_fwdbwd(args, rank, local_rank, steps, warmup, cpu=True):
     rng = np.random.default_rng([3, rank])
     keys = rng.uniform(0, 1, (keys_n, 3))
     t0 = time.perf_counter()
-    interp = ni.Interpolator(keys, device=dev, keep_host_mesh=cpu)
+    interp = make_interpolator(keys, device=dev, keep_host_mesh=cpu)
     build_s = time.perf_counter() - t0
     qn = rng.uniform(0.1, 0.9, (q_n, 3))
     vn = rng.standard_normal((keys_n, dim)).astype(np.float32)
@@ -653,7 +664,6 @@ def main():
         return
 
     import torch
-    import natinterp3d_b200 as ni
     from natinterp3d_b200 import _native
     from oracle import oracle
 
@@ -668,8 +678,8 @@ def main():
 
     keys, queries, values = make_data(args, rank)
     t0 = time.perf_counter()
-    interp = ni.Interpolator(keys, device=dev, keep_host_mesh=(rank == 0 and not args.no_cpu_baseline),
-                             predicates=args.predicates)
+    interp = make_interpolator(keys, device=dev, keep_host_mesh=(rank == 0 and not args.no_cpu_baseline),
+                               predicates=args.predicates)
     build_s = time.perf_counter() - t0
     t0 = time.perf_counter()
     dm = interp.device_mesh
@@ -783,6 +793,7 @@ def main():
             'data': 'synthetic: seeded uniform keys and queries, N(0,1) float32 values',
             'config': plain_config(args, world),
             'setup': {
+                'constructor': interp.construction['constructor'],
                 'mesh_build_s': round(build_s, 2), 'mesh_upload_s': round(upload_s, 3),
                 'tets': dm.n_tets, 'resident_mesh_mb': round(dm.nbytes / 1e6, 1),
                 'octree': dm.octree_stats,
@@ -840,8 +851,12 @@ def main():
                                          max(args.warmup, 3), cpu_on)
             legs['gpu_construction_1M_keys'] = leg_gpu_construction(keys, interp, build_s,
                                                                     local_rank)
-            legs['batched'] = leg_batched(args, rank, local_rank, max(args.steps, 3),
-                                          max(args.warmup, 3), cpu_on)
+            from natinterp3d_b200 import _build
+            legs['batched'] = (
+                leg_batched(args, rank, local_rank, max(args.steps, 3), max(args.warmup, 3), cpu_on)
+                if _build.have_mesh_lib() else
+                {'unavailable': "BatchInterpolator builds its meshes with natinterp3d's constructor, "
+                                'whose library is not built'})
             line['legs'] = legs
         print(json.dumps(line))
     if dist is not None:
