@@ -44,8 +44,10 @@ TRAFFIC_SOURCE = ('one 1,000,000-row k_rows_volume launch of the 1M-key / 10M-qu
                   '(dram__bytes_read.sum + dram__bytes_write.sum, 1 pass; '
                   'profiles/k_rows_volume_200k_keys_2M_queries.md)')
 
-# FP64 operations per unit of work, counted as natinterp3d's C evaluates them
-# (each add, subtract, multiply and divide is one flop; no fused multiply-add)
+# FP64 operations per unit of work (each add, subtract, multiply and divide is one
+# flop; no fused multiply-add): orientations and circumcentres as natinterp3d's C
+# evaluates them, a test against a cached sphere and a subcell volume from its face
+# circumcentres as the kernels do
 FLOPS = {'orient': 23, 'sphere': 9, 'tet_cc': 79, 'tri_cc': 56, 'subcell_from': 63}
 
 
@@ -768,14 +770,15 @@ def main():
         fpq = flops_per_query(stats, summ['walk_steps'], M)
         fused, separate = ctypes.c_double(), ctypes.c_double()
         lib.nif_measure_fp64_peak(ctypes.byref(fused), ctypes.byref(separate))
-        # the dominant kernel, k_rows_volume: its launches take every row but
-        # the few the fused kernel takes (cavities wider than a record) and the
-        # two in a hundred of k_rows_general
+        # the dominant kernel, k_rows_volume, with k_rows_general for the two rows
+        # in a hundred that it does not take (their times come as one): every
+        # row but the few the fused kernel takes (cavities wider than a record)
         vol_rows = M - int(summ['rows_wide'])
         vol_ms, vol_launches = kms[2], kn[2]
         achieved = (fpq['volume'] * vol_rows / (vol_ms * 1e-3) / 1e12) if vol_ms > 0 else None
         path_achieved = fpq['total'] * M / (rows_ms * 1e-3) / 1e12 if rows_ms > 0 else None
-        names = ['k_locate', 'k_rows_cavity', 'k_rows_volume', 'k_rows_fast', 'k_rows_order']
+        names = ['k_locate', 'k_rows_cavity', 'k_rows_volume + k_rows_general', 'k_rows_fast',
+                 'k_rows_order']
         kernels = {n: {'ms_per_step': kms[i], 'launches_per_step': kn[i],
                        'share_of_rows_phase': kms[i] / rows_ms if rows_ms > 0 else None}
                    for i, n in enumerate(names)}
@@ -802,7 +805,7 @@ def main():
                 'tune_s': round(tune_s, 2), 'tune_sample_ms': tune_times,
             },
             'roofline': {
-                'bound': 'fp64', 'kernel': 'k_rows_volume',
+                'bound': 'fp64', 'kernel': names[2],
                 'achieved': achieved, 'peak': separate.value, 'unit': 'TFLOP/s',
                 'frac': (achieved / separate.value) if achieved and separate.value else None,
                 'peak_fused_fma': fused.value,
@@ -813,12 +816,13 @@ def main():
                 'launch_ms': vol_ms / vol_launches if vol_launches else None,
                 # dram__bytes_read.sum + dram__bytes_write.sum of one
                 # k_rows_volume launch from an ncu capture (profiles/), per row,
-                # times this workload's rows per launch
+                # times the rows of a launch and its k_rows_general's
                 'traffic': (TRAFFIC_PER_ROW['k_rows_volume'] * vol_rows / vol_launches
                             if vol_launches else None),
                 'traffic_note': 'per launch; ncu capture of %s' % TRAFFIC_SOURCE,
                 'row_path': {
-                    'kernels': 'k_locate + k_rows_cavity + k_rows_order + k_rows_volume (+ k_rows_fast)',
+                    'kernels': 'k_locate + k_rows_cavity + k_rows_order + k_rows_volume + k_rows_general '
+                               '(+ k_rows_fast)',
                     'achieved': path_achieved, 'flops_per_query': fpq['total'],
                     'frac': (path_achieved / separate.value) if path_achieved and separate.value
                     else None,

@@ -396,7 +396,8 @@ int nif_batch_summary(const nif_dbatch *b, int64_t total_queries, const void *d_
  * nif_profile_kernels then returns, for the same calls, the device time in
  * milliseconds and the launches per call of each row kernel: {k_locate,
  * k_rows_cavity, k_rows_volume, k_rows_fast, k_rows_order} (events bracket
- * each launch, at most 48 a call). */
+ * each launch, at most 64 a call).  The time of k_rows_volume includes its two
+ * k_rows_general, which take the rows it does not. */
 int nif_profile_enable(int on);
 int nif_profile_read(double ms[4]);
 int nif_profile_kernels(double ms[5], double launches[5]);

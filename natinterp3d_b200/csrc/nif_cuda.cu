@@ -2303,9 +2303,12 @@ int resident_blocks(Kern k, int threads, size_t smem) {
 // from the others.
 constexpr int PROF_EVENTS = 5;  // start | bucketing | fast rows | large rows | finish
 constexpr int PROF_RING = 64;
-constexpr int PROF_SPANS = 48;  // kernel spans recorded per call (further launches are not)
-constexpr int PROF_KINDS = 5;   // k_locate | k_rows_cavity | k_rows_volume | k_rows_fast | k_rows_order
+constexpr int PROF_SPANS = 64;  // kernel spans recorded per call (further launches are not)
+constexpr int PROF_KINDS = 5;   // k_locate | k_rows_cavity | k_rows_volume and k_rows_general | k_rows_fast | k_rows_order
 enum { SPAN_LOCATE = 0, SPAN_CAVITY = 1, SPAN_VOLUME = 2, SPAN_FUSED = 3, SPAN_ORDER = 4 };
+// k_rows_general before k_rows_volume: its time is SPAN_VOLUME's, which holds the one
+// after it too, its launch is not counted
+constexpr int SPAN_GENERAL = PROF_KINDS;
 struct Profiler {
     bool on = false;
     bool created = false;
@@ -2549,7 +2552,9 @@ void launch_split(const Launch &lc, const Rows &rows, const QT *Q, int64_t M, co
         // wide rows and the volumes, beside one another
         auto volumes = [&](auto with_terms) {
             constexpr bool TERMS = decltype(with_terms)::value;
+            prof_span(SPAN_GENERAL, false, st);
             launch_general<TERMS>(lc, rows, Q, n, order, h, e, terms, gen, false, sink, R.large, R.sum, st);
+            prof_span(SPAN_GENERAL, true, st);
             if (c0 + n == M) launch_wide();
             prof_span(SPAN_VOLUME, false, st);
             launch_rows(k_rows_volume<QT, Rows, Sink, VOCC, TERMS>, lc, n, GPB * sizeof(VolWS),
@@ -3191,8 +3196,9 @@ NIF_EXPORT int nif_profile_read(double ms[4]) {
         for (int j = 0; j < g_prof.nspan[r]; j++) {
             float t = 0.f;
             NIF_CUDA(cudaEventElapsedTime(&t, g_prof.sev[r][j][0], g_prof.sev[r][j][1]));
-            g_prof.kms[g_prof.skind[r][j]] += t / ncalls;
-            g_prof.klaunch[g_prof.skind[r][j]] += 1.0 / ncalls;
+            const int kind = g_prof.skind[r][j];
+            g_prof.kms[kind == SPAN_GENERAL ? SPAN_VOLUME : kind] += t / ncalls;
+            if (kind != SPAN_GENERAL) g_prof.klaunch[kind] += 1.0 / ncalls;
         }
     }
     g_prof.calls = 0;
