@@ -6,6 +6,7 @@ contiguous CUDA tensors on the mesh's device.
 """
 import ctypes
 import threading
+import time
 import weakref
 
 import numpy as np
@@ -28,6 +29,8 @@ _TABLE_SHARE = 4
 _TABLE_LEAVES = 4 << 30
 _tables_mu = threading.Lock()
 _tables = weakref.WeakSet()  # meshes that hold a table
+_MEASURED_FOR = 1.0  # seconds
+_all_free = {}  # by device: when measured, memory free if this process held none, all memory
 
 
 def _table_fits(table, room, held):
@@ -36,17 +39,23 @@ def _table_fits(table, room, held):
     return table <= room - _TABLE_LEAVES and (held + table) * _TABLE_SHARE <= room + held
 
 
-def _room(device):
-    """Bytes that can still be allocated on `device`."""
-    free, total = torch.cuda.mem_get_info(device)
+def _room(device, measure=True):
+    """Bytes that can still be allocated on `device`.  Without `measure`: by a
+    measurement (0.1 ms, at times 2) of the last second, and what this process's
+    allocator has taken or given back since."""
     try:
         stats = torch.cuda.memory_stats_as_nested_dict(device)
         used = stats['allocated_bytes']['all']['current']
-        cached = stats['reserved_bytes']['all']['current'] - used
-        limit = int(total * torch.cuda.get_per_process_memory_fraction(device))
+        reserved = stats['reserved_bytes']['all']['current']
+        share = torch.cuda.get_per_process_memory_fraction(device)
     except (RuntimeError, KeyError):  # an allocator that keeps no such counts
-        return free
-    return min(free + cached, limit - used)
+        return torch.cuda.mem_get_info(device)[0]
+    now = time.monotonic()
+    if measure or device not in _all_free or now - _all_free[device][0] > _MEASURED_FOR:
+        free, total = torch.cuda.mem_get_info(device)
+        _all_free[device] = now, free + reserved, total
+    _, free, total = _all_free[device]
+    return min(free, int(total * share)) - used
 
 
 def _stream_ptr(device):
@@ -192,8 +201,10 @@ class DeviceMesh:
         with _tables_mu:  # a table is decided on by what is free
             if table:
                 held = sum(m.table_bytes for m in _tables if m.device == self.device)
-                uploads = 24 * self.n_vertices + 32 * self.n_tets
-                table = _table_fits(full - lean, _room(self.device) - lean - uploads, held)
+                rest = lean + 24 * self.n_vertices + 32 * self.n_tets  # and the uploads
+                # with half the room to spare by the last measurement, or by a new one
+                table = _table_fits(full - lean, _room(self.device, False) // 2 - rest, held) or \
+                    _table_fits(full - lean, _room(self.device) - rest, held)
             self.table_bytes = full - lean if table else 0
             (_tables.add if table else _tables.discard)(self)
             self._buf = torch.empty(full if table else lean, dtype=torch.uint8, device=self.device)

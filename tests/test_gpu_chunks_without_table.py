@@ -20,7 +20,7 @@ def meshes(cuda_device):
     c = keys.mean(axis=0)
     packed, _ = nd.gpu_delaunay(keys - c)
     with pytest.MonkeyPatch.context() as m:
-        m.setattr(nd, '_room', lambda d: 0)
+        m.setattr(nd, '_room', lambda *a: 0)
         lean = nd.DeviceMesh(*packed, device=cuda_device)
     full = nd.DeviceMesh(*packed, device=cuda_device)
     assert lean.table_bytes == 0 < full.table_bytes

@@ -17,7 +17,7 @@ def test_same_bits(cuda_device, n):
     c = keys.mean(axis=0)
     packed, _ = nd.gpu_delaunay(keys - c, cuda_device)
     with pytest.MonkeyPatch.context() as m:
-        m.setattr(nd, '_room', lambda d: 0)
+        m.setattr(nd, '_room', lambda *a: 0)
         lean = nd.DeviceMesh(*packed, device=cuda_device)
     full = nd.DeviceMesh(*packed, device=cuda_device)
     assert lean.table_bytes == 0 < full.table_bytes

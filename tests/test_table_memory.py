@@ -26,6 +26,39 @@ def test_rule():
     assert held <= 178 * GB // 4 and meshes >= 178 // 2 * 3 // 4
 
 
+def test_room_is_measured_once_and_kept_up(monkeypatch):
+    """The free memory is asked for once a second; what the process's allocator
+    takes and gives back, and its limit, are followed without."""
+    clock = [100.0]
+    monkeypatch.setattr(nd.time, 'monotonic', lambda: clock[0])
+    now = {'free': 90 * GB, 'reserved': 10 * GB, 'used': 4 * GB, 'share': 1.0, 'asked': 0}
+
+    def info(device):
+        now['asked'] += 1
+        return now['free'], 100 * GB
+    monkeypatch.setattr(torch.cuda, 'mem_get_info', info)
+    monkeypatch.setattr(torch.cuda, 'get_per_process_memory_fraction', lambda d: now['share'])
+    monkeypatch.setattr(torch.cuda, 'memory_stats_as_nested_dict', lambda d: {
+        'allocated_bytes': {'all': {'current': now['used']}},
+        'reserved_bytes': {'all': {'current': now['reserved']}}})
+    monkeypatch.setattr(nd, '_all_free', {})
+    assert nd._room('d', False) == 96 * GB
+    now.update(free=70 * GB, reserved=30 * GB, used=28 * GB)
+    assert nd._room('d', False) == 72 * GB and now['asked'] == 1
+    now.update(free=20 * GB)  # someone else took 50 GB
+    assert nd._room('d', False) == 72 * GB and nd._room('d') == nd._room('d', False) == 22 * GB
+    now.update(share=0.4)
+    assert nd._room('d', False) == 12 * GB and now['asked'] == 2
+    now.update(free=30 * GB, share=1.0)
+    clock[0] += 1.5
+    assert nd._room('d', False) == 32 * GB and now['asked'] == 3
+
+    def none(device):
+        raise RuntimeError
+    monkeypatch.setattr(torch.cuda, 'memory_stats_as_nested_dict', none)
+    assert nd._room('d', False) == 30 * GB
+
+
 @pytest.fixture(scope='module')
 def mesh(cuda_device):
     keys = np.random.default_rng(91).uniform(0, 1, (60_000, 3))
