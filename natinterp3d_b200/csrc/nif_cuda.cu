@@ -85,9 +85,9 @@ inline int64_t record_chunk(int64_t M, bool terms) {
     return (rows + cuts - 1) / cuts;
 }
 // resident blocks per SM of the split kernels (0: the mesh's blocks_per_sm).
-// The cavity kernel takes 8 (64 registers; 10 blocks spill: 2.57 ms a 2M-row call
-// for 2.25).  The volume kernel takes 6 or, for the
-// setting of 8, 7: with 72 registers a thread it barely spills, and a warp's
+// The cavity kernel takes 8 (64 registers, 84 bytes a thread spilled, 228 in the
+// filtered modes; 10 blocks spill more: 2.57 ms a 2M-row call for 2.25).  The volume
+// kernel takes 6 or, for the setting of 8, 7: with 72 registers a thread it barely spills, and a warp's
 // workspace holds 42 boundary faces (2M queries, 200k keys, when 7 blocks took
 // 7.1 ms, now 6.1: 7.4 ms at 6, 10.1 ms at 8 with 64 registers and 34 faces).
 #ifndef NIF_CAV_OCC
@@ -1470,7 +1470,9 @@ __global__ void __launch_bounds__(FAST_BLOCK, OCC) k_rows_fast(MeshView M, const
 // super-simplex, -2 a walk that hit its step limit, -3 (PM_FILTER) a walk
 // test the error bound cannot certify (the large kernel resolves the row).
 #ifndef NIF_LOC_OCC
-#define NIF_LOC_OCC 8  // 64 registers (10 and 12 spill: 1.65 and 1.63 ms a 2M-row call for 1.55)
+// 64 registers, 20 bytes a thread spilled (128 with many meshes); 10 and 12 blocks spill
+// more: 1.65 and 1.63 ms a 2M-row call for 1.55
+#define NIF_LOC_OCC 8
 #endif
 template <class QT, class Rows, int PM = PM_PLAIN>
 __global__ void __launch_bounds__(FAST_BLOCK, NIF_LOC_OCC) k_locate(const __grid_constant__ Rows rows,
@@ -1587,15 +1589,17 @@ __global__ void __launch_bounds__(FAST_BLOCK, OCC)
         const double *cen = nullptr;
         const MeshView &M = rows.get(i, cur, &sview[threadIdx.x / 16], g, cen);
         const dv3 q = load_query(Q, i, cen);
+        if (M.small && go && flat_sized(M, h.start)) h.state = RS_FLAT;
         const int rc = flood_pair<CavWS, PM>(M, q, ws, max(h.start, 0), go, h, ents + (row ? my : s) * REC_CAV);
-        if (rc != REC_DONE) h.state = RS_QUEUED;
+        if (rc != REC_DONE)
+            h.state = RS_QUEUED;
+        else if (h.state == RS_FLAT && h.ncav == 0)
+            h.state = RS_OK;  // the coincident-vertex row
         if (row && g.lane == 0) {
             if (rc == REC_WIDE)
                 wide[atomicAdd(&sum->wide_count, 1)] = (int)i;
             else if (rc == REC_LARGE || h.start == -3)
                 lq.list[atomicAdd(&sum->large_count, 1)] = (int)i;
-            else if (M.small && h.ncav > 0 && flat_sized(M, h.start))
-                h.state = RS_FLAT;
             heads[my] = h;
         }
         __syncwarp();
