@@ -700,7 +700,11 @@ struct InterpSink {
     int D;
     static constexpr bool FULL = true;
     static constexpr bool SORTED = sizeof(WT) == 4;
-    static constexpr int STAGED_D = 8;  // columns summed from staged products
+    // Columns summed from staged products: 1M rows, 50k keys take 5,506 us with one
+    // column, 5,568 with four, 5,588 with five, 5,630 with six and 5,809 with eight
+    // where a lane a column takes 5,626 with any of them (1M keys: 6,244 / 6,309 /
+    // 6,342 / 6,400 / 6,554, and 6,412; float32 the same way).
+    static constexpr int STAGED_D = 5;
     static constexpr int LANE_D = 4;    // of these, the columns a lane reads ahead
 
     template <int G, class W>
@@ -2091,7 +2095,9 @@ size_t fcc_slots(int nt) {
 // Calls of at most this many rows take them as they come: a warp has a few rows
 // at most, so that their order decides little, and the bucketing's six launches
 // are left out (5,003 rows on 50k keys 237 to 214 us a call, 14,003 rows 284 to
-// 261 us).
+// 261 us).  The line is on the safe side: on 1M keys, queries in random order, 20,000
+// rows take 371 us by bucket and 346 as they come, 100,000 rows 941 and 938, 200,000
+// rows 1,608 and 1,645.
 constexpr int64_t IDENTITY_ROWS = 16384;
 
 struct MeshLayout {
