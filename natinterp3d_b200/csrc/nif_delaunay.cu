@@ -68,7 +68,6 @@ enum : int {
     ERR_NONE = 0,
     ERR_DEGENERATE = 1,   // an exact zero that decides the result
     ERR_CAPACITY = 2,     // tet slots or list space exhausted
-    ERR_WALK = 3,         // a relocation walk exceeded its step limit
     ERR_OUTSIDE = 4,      // a key outside the super-simplex
     ERR_INTERNAL = 5,     // an inconsistency (a negative boundary orientation)
 };
@@ -1027,7 +1026,6 @@ NIF_EXPORT int nif_delaunay_build(const double *d_keys, int n, void *d_ws, size_
     info->error = h.err;
     if (h.err == ERR_DEGENERATE || h.err == ERR_OUTSIDE) return NIF_ERR_DEGENERATE;
     if (h.err == ERR_CAPACITY) return NIF_ERR_CAPACITY;
-    if (h.err == ERR_WALK) return NIF_ERR_WALK;
     if (h.err != ERR_NONE) return NIF_ERR_INTERNAL;
     k_verify<<<wblocks, THREADS, 0, st>>>(D, L.bad);
     k_alive<<<pblocks, 256, 0, st>>>(D, L.flag);

@@ -16,8 +16,10 @@
 //               floating-point summation order of every weight
 //   3. boundary faces and natural neighbours in first-seen order (:559-584)
 //   4. signed Voronoi-subcell volumes: +cavity-tet terms (:642-676) and
-//      -virtual-tet terms (:681-719), one term per lane, folded into each
-//      neighbour's sum in natinterp3d's accumulation order
+//      -virtual-tet terms (:681-719), added to each neighbour's sum in
+//      natinterp3d's accumulation order: the split rows (split_row_body) store
+//      a neighbour's terms next to each other and one lane adds them, the fused
+//      and large rows fold a term per lane
 //   5. normalisation (:721-737)
 // Tet circumcentres and face circumcentres are read from the per-mesh cache
 // (computed with the same formulas and argument orders); a face shared by two
@@ -526,7 +528,6 @@ __device__ __forceinline__ bool flat_sized(const MeshView &M, int t) {
 // visiting order.  Index types are the narrowest that hold each capacity.
 template <int HS_, int CAV_, int BF_, int NBR_, int VH_, int G_, class SlotT, class CavT>
 struct Workspace {
-    static constexpr bool SPLIT = false;
     static constexpr int HS = HS_;        // tested-tet hash slots (power of two)
     static constexpr int QCAP = HS_ * 3 / 4;
     static constexpr int CAV = CAV_;      // cavity tets
@@ -587,7 +588,6 @@ constexpr int VOL_VERTS = 56;      // ids of a row (columns are below 63)
 constexpr int VOL_NO_ID = 255;     // a cavity vertex that is on no boundary face
 template <int CAV_, int BF_, int VH_, int G_>
 struct alignas(16) VolWorkspace {
-    static constexpr bool SPLIT = true;
     static constexpr int CAV = CAV_;
     static constexpr int BF = BF_;
     static constexpr int FW = (BF_ + 63) / 64;  // 64-bit words of a face set
