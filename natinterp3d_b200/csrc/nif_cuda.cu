@@ -885,7 +885,7 @@ struct GradSink {
     // to the next vertex and the other face of that edge, is one triangle of
     // u's facet: about 40 operations instead of the 3,000 of the dual numbers,
     // so that the pass is bound by the same row setup as the weights (1M rows,
-    // 200k keys, 16 columns: 10.1 ms with dual numbers, 2.4 ms).
+    // 200k keys, 16 columns: 11.2 ms with dual numbers, 2.6 ms).
     // Returns false where that does not hold: faces that do not close or that
     // differ in orientation, or tets and triangles near natinterp3d's
     // degeneracy thresholds; k_rows_general takes those rows, with the dual
