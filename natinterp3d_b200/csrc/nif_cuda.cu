@@ -1782,9 +1782,9 @@ __device__ __forceinline__ bool finish_row(int64_t i, RowInfo &r, RowLanes<IDS> 
 
 // The corner terms of a chunk's record entries, for meshes without the corner
 // table: a warp a row, a lane a corner, written beside the entries for
-// k_rows_volume.  Bound by the gathers of its circumcentres: 1.5 ms a 1M-row
-// chunk, so that a 2M-row call takes 14.7 ms where one with the table takes
-// 11.5 and one that computed the terms in the row kernels 23.2.
+// k_rows_volume.  Bound by the gathers of its circumcentres: 1.5 ms a 1M rows,
+// so that a 2M-row call takes 14.4 ms where one with the table takes
+// 11.0 (and took 23.2 with the terms computed in the row kernels).
 template <class Rows>
 __global__ void __launch_bounds__(FAST_BLOCK)
     k_rows_terms(const __grid_constant__ Rows rows, const int *__restrict__ order, int64_t nrows,
@@ -2119,8 +2119,8 @@ struct MeshLayout {
 // Largest mesh that holds its corner terms: 512 bytes a tet, 34 GB here (about
 // 10M keys), next to 270 bytes a tet for the rest.  Larger meshes, which are to
 // leave room for others' data, and those whose caller has no room for the table,
-// compute them per row (k_rows_terms: a 2M-row call takes 14.7 ms, with the
-// table 11.5).
+// compute them per row (k_rows_terms: a 2M-row call takes 14.4 ms, with the
+// table 11.0).
 #ifndef NIF_CORNER_TETS_MAX
 #define NIF_CORNER_TETS_MAX (1 << 26)
 #endif
